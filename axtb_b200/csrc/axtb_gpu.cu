@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -29,6 +30,7 @@
 #include "k_solvation.cuh"
 #include "params/gfn2_tables.h"
 #include "team_kernel.cuh"
+#include "trd.cuh"
 #include "chase.cuh"
 
 using std::vector;
@@ -331,6 +333,28 @@ struct AxtbBatch {
     axg::TeamPlan P{};
     axg::ChasePlan CP{};    // molecules whose band k_chase reduces (stage 2 on chip)
     int nchase = 0, chase_grid = 0;
+    // tridiagonal reductions on chip: one launch per size class and cluster size (k_trd), each on
+    // its own stream, and the whole-grid molecules one after the other (k_trd_grid)
+    struct TrdLaunch {
+        const void* fn;
+        int G, count, smem;
+        const int* list;
+        double cost;
+    };
+    struct TrdGrid {
+        const void* fn;
+        int mol, smem;
+    };
+    vector<TrdLaunch> trd;
+    vector<TrdGrid> trd_grid;
+    int grid_sms = 0;          // CTAs of k_trd_grid
+    double* d_xpub = nullptr;  // what k_trd_grid's CTAs publish to one another
+    vector<cudaStream_t> side;
+    vector<cudaEvent_t> side_ev;  // fork, then one join per side stream
+    void launch_trd();
+    void plan_trd(int big_nao, bool big_given, int band_max, const vector<int>& nao, int nsm, vector<int>& kind);
+    void place_trd(const vector<int>& kind, const vector<int>& nao, int nsm,
+                   const std::function<const int*(const vector<int>&)>& up);
     void* dmem = nullptr;
     void* hpin = nullptr;  // pinned staging
     size_t hpin_size = 0;
@@ -381,11 +405,138 @@ struct AxtbBatch {
 AxtbBatch::~AxtbBatch() {
     for (auto& e : phase_ev)
         if (e) cudaEventDestroy(e);
+    for (auto& e : side_ev) cudaEventDestroy(e);
+    for (auto& x : side) cudaStreamDestroy(x);
     if (h_act) cudaFreeHost(h_act);
     if (h_stage) cudaFreeHost(h_stage);
     if (dmem) cudaFree(dmem);
     if (hpin) cudaFreeHost(hpin);
     if (st) cudaStreamDestroy(st);
+}
+
+// Which molecules reduce to tridiagonal form on chip (trd.cuh). From TRD_MIN_NAO AOs on (below it
+// the one-CTA reduction keeps the bits that some chaotic SCFs follow: the largest molecule that
+// does so in the recorded sets has 99 AOs), one molecule per cluster as long as 16 CTAs hold it
+// (768 AOs); from big_nao on, and above 768 AOs in batches of at most 64 such molecules (one after
+// the other on the whole grid at ~2.5 us per column beats one CTA each only while there are few),
+// on the whole grid as long as the chip holds the matrix.
+constexpr int TRD_MIN_NAO = 100;
+void AxtbBatch::plan_trd(int big_nao, bool big_given, int band_max, const vector<int>& nao, int nsm, vector<int>& kind) {
+    int nc = 0, ng = 0, optin = 0, clusters = 0;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    CK(cudaDeviceGetAttribute(&clusters, cudaDevAttrClusterLaunch, device));
+    if (optin < axg::TRD_SMEM_MAX || !clusters) return;
+    const axg::TrdClass* cls = axg::trd_classes(nc);
+    const axg::TrdClass* gcl = axg::trd_grid_classes(ng);
+    int large = 0;
+    for (int n : nao) large += n > 32 * cls[nc - 1].rt && n < big_nao;
+    for (int m = 0; m < nmol; m++) {
+        int n = nao[m];
+        if (n < TRD_MIN_NAO) continue;
+        bool grid_mol = n >= big_nao || (n > 32 * cls[nc - 1].rt && !big_given && large <= 64);
+        if (!grid_mol) {
+            if (n > 32 * cls[nc - 1].rt || (n > axg::BW + 1 && n < band_max)) continue;
+            kind[m] = 1;
+            continue;
+        }
+        for (int c = 0; c < ng; c++)
+            if (n <= 256 * gcl[c].rt) {
+                if (axg::trd_smem_doubles(n, nsm, 8, gcl[c].cr, true) * 8 <= axg::TRD_SMEM_MAX) kind[m] = 2;
+                break;
+            }
+    }
+}
+
+// The launches of the reductions on chip: per size class, molecules grouped by the cluster size
+// that holds them. With SMs to spare (few molecules) the clusters grow: fewer columns per CTA, the
+// same bits. Measured at one molecule per launch, us for 2 / 4 / 8 / 16 CTAs: 235 / 207 / 213 / 229
+// at 120 AOs, 453 / 415 / 358 / 401 at 192, - / 1574 / 1033 / 1046 at 378; 3193 / 2738 for 9 / 16
+// at 600: clusters of up to 4 grow to at most 8, larger ones to 16.
+void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int nsm,
+                          const std::function<const int*(const vector<int>&)>& up) {
+    int nc = 0, ng = 0;
+    const axg::TrdClass* cls = axg::trd_classes(nc);
+    const axg::TrdClass* gcl = axg::trd_grid_classes(ng);
+    std::map<std::pair<int, int>, vector<int>> groups;  // (class, cluster size) -> molecules
+    vector<int> cl(nmol, 0), G(nmol, 0);
+    long long need = 0;
+    for (int m = 0; m < nmol; m++) {
+        int n = nao[m];
+        if (kind[m] == 2) {
+            int c = 0;
+            while (n > 256 * gcl[c].rt) c++;
+            trd_grid.push_back({gcl[c].fn, m, (int)(axg::trd_smem_doubles(n, nsm, 8, gcl[c].cr, true) * 8)});
+        }
+        if (kind[m] != 1) continue;
+        while (n > 32 * cls[cl[m]].rt) cl[m]++;
+        G[m] = 1;
+        while (axg::trd_smem_doubles(n, G[m], 1, cls[cl[m]].cr, false) * 8 > axg::TRD_SMEM_MAX) G[m]++;
+        need += G[m];
+    }
+    int widen = 1;
+    while (widen < 8 && need * widen * 2 <= nsm) widen *= 2;
+    for (int m = 0; m < nmol; m++)
+        if (kind[m] == 1) {
+            int g = G[m] <= 4 ? std::min(8, G[m] * widen) : widen > 1 ? 16 : G[m];
+            groups[{cl[m], g}].push_back(m);
+        }
+    for (auto& kv : groups) {
+        vector<int>& v = kv.second;
+        std::sort(v.begin(), v.end(), [&](int a, int b) { return nao[a] > nao[b]; });
+        const axg::TrdClass& c = cls[kv.first.first];
+        int g = kv.first.second;
+        long long sm = 0;
+        for (int m : v) sm = std::max(sm, axg::trd_smem_doubles(nao[m], g, 1, c.cr, false) * 8);
+        CK(cudaFuncSetAttribute(c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
+        if (g > 8) CK(cudaFuncSetAttribute(c.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        trd.push_back({c.fn, g, (int)v.size(), (int)sm, up(v), (double)nao[v[0]]});
+    }
+    std::sort(trd.begin(), trd.end(), [](const TrdLaunch& a, const TrdLaunch& b) { return a.cost > b.cost; });
+    for (auto& t : trd_grid) CK(cudaFuncSetAttribute(t.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
+    grid_sms = nsm;
+    // side streams: every launch after the first runs beside it
+    for (size_t i = 1; i < trd.size(); i++) {
+        cudaStream_t x;
+        CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+        side.push_back(x);
+    }
+    for (size_t i = 0; i < side.size() + 1; i++) {
+        cudaEvent_t e;
+        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        side_ev.push_back(e);
+    }
+}
+
+void AxtbBatch::launch_trd() {
+    for (auto& t : trd_grid) {
+        void* args[] = {&B, &S, &t.mol, &d_xpub, &P.cycles};
+        CK(cudaLaunchCooperativeKernel(t.fn, grid_sms, axg::TRD_THREADS, args, t.smem, st));
+        launches++;
+    }
+    if (trd.size() > 1) CK(cudaEventRecord(side_ev[0], st));
+    for (size_t i = 0; i < trd.size(); i++) {
+        TrdLaunch& t = trd[i];
+        cudaStream_t x = i == 0 ? st : side[i - 1];
+        if (i > 0) CK(cudaStreamWaitEvent(x, side_ev[0], 0));
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = t.G;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(t.G * t.count));
+        cfg.blockDim = dim3(axg::TRD_THREADS);
+        cfg.dynamicSmemBytes = t.smem;
+        cfg.stream = x;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        void* args[] = {&B, &S, &t.list, &P.cycles};
+        CK(cudaLaunchKernelExC(&cfg, t.fn, args));
+        launches++;
+        if (i > 0) {
+            CK(cudaEventRecord(side_ev[i], x));
+            CK(cudaStreamWaitEvent(st, side_ev[i], 0));
+        }
+    }
 }
 
 void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
@@ -632,6 +783,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     if (per <= 0) throw Fail(AXTB_ERR_DEVICE, "team kernel does not fit on a multiprocessor");
     grid = nsm * std::min(per, 2);
     vector<int> big, small_off(grid + 1, 0), small_list, head_off, head_list, tail_off, tail_list;
+    vector<int> trd_kind(nmol, 0);  // 1: k_trd on a cluster, 2: k_trd_grid
     {
         vector<std::pair<double, int>> smalls, heads, tails;
         // molecules from this many AOs on take the whole grid (AXTB_TEAM_BIG_NAO overrides, e.g.
@@ -641,6 +793,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         // the eigen phase of a molecule whose bulge chasing runs on chip is split over two team
         // launches (before and after k_chase), each balanced on its own: measured shares of a
         // two-stage eigen phase, ~0.2 before (F' and stage 1) and ~0.55 after
+        plan_trd(big_nao, o.grid_min_nao > 0, band_max, m_nao, nsm, trd_kind);
         for (int m = 0; m < nmol; m++) {
             int n = m_nao[m];
             if (n >= big_nao) {
@@ -650,8 +803,8 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
             double c = std::pow((double)n + 32.0, 3.0);
             bool chased = n > axg::BW + 1 && n < band_max && n <= chase_max;
             smalls.push_back({c, m});
-            heads.push_back({chased ? 0.2 * c : c, m});
-            if (chased) tails.push_back({0.55 * c, m});
+            heads.push_back({chased ? 0.2 * c : trd_kind[m] ? 0.06 * c : c, m});
+            if (chased || trd_kind[m]) tails.push_back({chased ? 0.55 * c : 0.4 * c, m});
         }
         // longest first onto the least loaded CTA
         auto lpt = [&](vector<std::pair<double, int>>& items, vector<int>& off, vector<int>& list) {
@@ -699,6 +852,10 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     addI(head_list.size() + 1);
     addI(tail_off.size());
     addI(tail_list.size() + 1);
+    addI(nmol);                                              // trd_kind
+    for (int c = 0; c < 128; c++) addI(1);                   // k_trd lists: at most one per class and cluster size
+    addI(nmol);
+    addD(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()));
     {  // the chase plan (k_chase): offsets per cluster and per CTA, molecule lists
         size_t ncl = (size_t)std::max(1, nsm / 2);
         addI(ncl + 1);
@@ -934,6 +1091,8 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     b.disp = o.dispersion ? 1 : 0;
     b.band_max = band_max;
     b.chase_max = chase_max;
+    b.m_trd = upI(trd_kind);
+    place_trd(trd_kind, m_nao, nsm, upI);
     vector<int> pair_off, pair_list, solo_off, solo_list;
     {
         // the plan: pairs (above CHASE_ROWS AOs) on clusters, then the rest one per CTA, longest
@@ -1083,6 +1242,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         s.sv_nbn = ar.take<int>(natT);
     }
     s.red = ar.take<double>((size_t)axg::team_red_doubles(grid));  // grid-team partials
+    d_xpub = ar.take<double>(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()));
     s.eeq_A = ar.take<double>((size_t)nsqT * 3);
     s.gam = ar.take<double>((size_t)std::max(ngamT, 1LL));
     // team plan
@@ -1407,7 +1567,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         ph = phase;
         Psmall = P;
         Psmall.nbig = 0;
-        if (P.nbig > 0 && phase != PH_EIGEN_TAIL) {  // no whole-grid molecule has a part after k_chase
+        if (P.nbig > 0) {
             CK(cudaLaunchCooperativeKernel((void*)k_team_grid, grid, TEAM_THREADS, args, SMEM_WORK_BYTES, st));
             launches++;
         }
@@ -1446,8 +1606,12 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
                     CP.cycles = P.cycles;
                     k_chase<<<chase_grid, CHASE_THREADS, CHASE_DYN_BYTES, st>>>(B, S, CP);
                     CK(cudaGetLastError());
+                    launches++;
+                }
+                launch_trd();
+                if (nchase > 0 || !trd.empty() || !trd_grid.empty()) {
                     team_launch(PH_EIGEN_TAIL);
-                    launches += 2;
+                    launches++;
                 }
             });
             LAUNCH("mulliken", 0, mat_bytes(act, 12.0),

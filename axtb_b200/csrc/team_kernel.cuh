@@ -197,6 +197,9 @@ __device__ void mol_eigen(const Team& t, const Batch& B, State& S, const TeamPla
         }
         team_sb2st(t, Fp, n, n, d, e, wk, S.W + mat);
         TEAM_PHASE(17);
+    } else if (B.m_trd && B.m_trd[m]) {  // the reduction and the rest in the next launches
+        if (P.cycles && t.tid() == 0) S.mol_cyc[m] = (double)(clock64() - tstart) * t.size;
+        return;
     } else {
         double* Vp = wk + 2 * n + (long long)nsl * n;  // the back-transform's vb area (64 n)
         team_tridiag_blocked<GRID_ROWS>(t, Fp, n, n, d, e, tau, Vp, Vp + (long long)NBP * n, vbuf, pbuf, ppart, S.red,
@@ -258,7 +261,7 @@ __device__ void mol_eigen(const Team& t, const Batch& B, State& S, const TeamPla
     t.sync();
     TEAM_PHASE(7);
     if (P.cycles && t.tid() == 0) {
-        double c = (double)(clock64() - tstart);
+        double c = (double)(clock64() - tstart) * t.size;
         if (after_chase) S.mol_cyc[m] += c;  // after the part before and the chase
         else S.mol_cyc[m] = c;
     }
@@ -307,7 +310,7 @@ __device__ void run_mol(const Team& t, const Batch& B, State& S, const TeamPlan&
         case PH_EEQ: mol_eeq(t, B, S, P, m); break;
         case PH_EIGEN:
         case PH_EIGEN_TAIL:
-            if (phase == PH_EIGEN || chased_on_chip(t, B, B.m_nao[m])) mol_eigen<GRID_ROWS>(t, B, S, P, m, phase == PH_EIGEN_TAIL);
+            if (phase == PH_EIGEN || chased_on_chip(t, B, B.m_nao[m]) || (B.m_trd && B.m_trd[m])) mol_eigen<GRID_ROWS>(t, B, S, P, m, phase == PH_EIGEN_TAIL);
             break;
         case PH_WDENS: mol_wdens(t, B, S, P, m); break;
         case PH_LEVELS: mol_levels(t, B, S, P, m); break;
