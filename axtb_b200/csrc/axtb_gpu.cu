@@ -422,68 +422,61 @@ AxtbBatch::~AxtbBatch() {
 // on the whole grid as long as the chip holds the matrix.
 constexpr int TRD_MIN_NAO = 100;
 void AxtbBatch::plan_trd(int big_nao, bool big_given, int band_max, const vector<int>& nao, int nsm, vector<int>& kind) {
-    int nc = 0, ng = 0, optin = 0, clusters = 0;
+    int optin = 0, clusters = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     CK(cudaDeviceGetAttribute(&clusters, cudaDevAttrClusterLaunch, device));
     if (optin < axg::TRD_SMEM_MAX || !clusters) return;
-    const axg::TrdClass* cls = axg::trd_classes(nc);
-    const axg::TrdClass* gcl = axg::trd_grid_classes(ng);
+    const int cluster_max = axg::TRD_CLUSTER_MAX_NAO;
     int large = 0;
-    for (int n : nao) large += n > 32 * cls[nc - 1].rt && n < big_nao;
+    for (int n : nao) large += n > cluster_max && n < big_nao;
     for (int m = 0; m < nmol; m++) {
         int n = nao[m];
         if (n < TRD_MIN_NAO) continue;
-        bool grid_mol = n >= big_nao || (n > 32 * cls[nc - 1].rt && !big_given && large <= 64);
+        bool grid_mol = n >= big_nao || (n > cluster_max && !big_given && large <= 64);
         if (!grid_mol) {
-            if (n > 32 * cls[nc - 1].rt || (n > axg::BW + 1 && n < band_max)) continue;
+            if (n > cluster_max || (n > axg::BW + 1 && n < band_max)) continue;
             kind[m] = 1;
             continue;
         }
-        for (int c = 0; c < ng; c++)
-            if (n <= 256 * gcl[c].rt) {
-                if (axg::trd_smem_doubles(n, nsm, 8, gcl[c].cr, true) * 8 <= axg::TRD_SMEM_MAX) kind[m] = 2;
-                break;
-            }
+        const axg::TrdClass* c = axg::trd_grid_class(n);
+        if (c && axg::trd_smem_doubles(n, nsm, 8, c->cr, true) * 8 <= axg::TRD_SMEM_MAX) kind[m] = 2;
     }
 }
 
 // The launches of the reductions on chip: per size class, molecules grouped by the cluster size
 // that holds them. With SMs to spare (few molecules) the clusters grow: fewer columns per CTA, the
-// same bits. Measured at one molecule per launch, us for 2 / 4 / 8 / 16 CTAs: 235 / 207 / 213 / 229
-// at 120 AOs, 453 / 415 / 358 / 401 at 192, - / 1574 / 1033 / 1046 at 378; 3193 / 2738 for 9 / 16
-// at 600: clusters of up to 4 grow to at most 8, larger ones to 16.
+// same bits. Measured, us per reflector of one molecule, for 1 / 2 / 4 / 8 / 16 CTAs: 2.24 / 1.87 /
+// 1.38 / 1.37 / - at 120 AOs, 3.88 / 2.14 / 1.76 / 1.48 / - at 192, - / 4.27 / 2.87 / 2.19 / 1.80 at
+// 258, - / - / 3.66 / 2.14 / 1.95 at 378, and 3.46 / 2.88 for 10 / 16 at 600: up to 8 CTAs to 192
+// AOs, up to 16 above. A full GPU is best filled by the smallest clusters (CTAs x us grows with
+// the cluster at every size).
 void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int nsm,
                           const std::function<const int*(const vector<int>&)>& up) {
-    int nc = 0, ng = 0;
-    const axg::TrdClass* cls = axg::trd_classes(nc);
-    const axg::TrdClass* gcl = axg::trd_grid_classes(ng);
-    std::map<std::pair<int, int>, vector<int>> groups;  // (class, cluster size) -> molecules
-    vector<int> cl(nmol, 0), G(nmol, 0);
+    std::map<std::pair<const axg::TrdClass*, int>, vector<int>> groups;  // (class, cluster size) -> molecules
+    vector<int> G(nmol, 0);
     long long need = 0;
     for (int m = 0; m < nmol; m++) {
         int n = nao[m];
         if (kind[m] == 2) {
-            int c = 0;
-            while (n > 256 * gcl[c].rt) c++;
-            trd_grid.push_back({gcl[c].fn, m, (int)(axg::trd_smem_doubles(n, nsm, 8, gcl[c].cr, true) * 8)});
+            const axg::TrdClass* c = axg::trd_grid_class(n);
+            trd_grid.push_back({c->fn, m, (int)(axg::trd_smem_doubles(n, nsm, 8, c->cr, true) * 8)});
         }
         if (kind[m] != 1) continue;
-        while (n > 32 * cls[cl[m]].rt) cl[m]++;
         G[m] = 1;
-        while (axg::trd_smem_doubles(n, G[m], 1, cls[cl[m]].cr, false) * 8 > axg::TRD_SMEM_MAX) G[m]++;
+        while (axg::trd_smem_doubles(n, G[m], 1, axg::trd_class(n)->cr, false) * 8 > axg::TRD_SMEM_MAX) G[m]++;
         need += G[m];
     }
     int widen = 1;
-    while (widen < 8 && need * widen * 2 <= nsm) widen *= 2;
+    while (widen < 16 && need * widen * 2 <= nsm) widen *= 2;
     for (int m = 0; m < nmol; m++)
         if (kind[m] == 1) {
-            int g = G[m] <= 4 ? std::min(8, G[m] * widen) : widen > 1 ? 16 : G[m];
-            groups[{cl[m], g}].push_back(m);
+            int g = std::min(nao[m] <= 192 ? 8 : 16, G[m] * widen);
+            groups[{axg::trd_class(nao[m], g), g}].push_back(m);
         }
     for (auto& kv : groups) {
         vector<int>& v = kv.second;
         std::sort(v.begin(), v.end(), [&](int a, int b) { return nao[a] > nao[b]; });
-        const axg::TrdClass& c = cls[kv.first.first];
+        const axg::TrdClass& c = *kv.first.first;
         int g = kv.first.second;
         long long sm = 0;
         for (int m : v) sm = std::max(sm, axg::trd_smem_doubles(nao[m], g, 1, c.cr, false) * 8);

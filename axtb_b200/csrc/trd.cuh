@@ -9,8 +9,11 @@
 // it with the new reflector also applies the previous one (A -= v w^T + w v^T, then y = A v', both
 // on the element while it is in a register: no panels, no dot products with them, no trailing
 // GEMMs), and the full matrix is stored, so a column's product is complete inside the warp that
-// owns the column: the CTAs exchange only y (each CTA its columns' entries) and the next column,
-// behind ONE barrier per reflector. Everything of size n (w, the next column brought up to date,
+// owns the column: the CTAs exchange only y and the next column (as the next row: each CTA its own
+// columns' two entries, so that no CTA serves a whole column to all the others). In a cluster every
+// warp pushes its columns' pairs into each CTA's shared memory as soon as it has them (st.async; a
+// transaction barrier counts the bytes), so one one-way trip is all that separates two reflectors;
+// the grid publishes them in global memory behind one grid barrier. Everything of size n (w, the next column brought up to date,
 // its norm, the next reflector) is then formed by every CTA for itself, with the same bits.
 //
 // Thread layout of a CTA (256 threads): warp = (row group rg of AW, column group cg of TC = 8/AW).
@@ -31,8 +34,9 @@ namespace axg {
 constexpr int TRD_THREADS = 256;
 constexpr int TRD_SMEM_MAX = 227 * 1024;
 
-// shared memory of one CTA (doubles): v (two buffers), w, the published column and y entries (two
-// buffers each, cluster only), reduction slots, the row groups' partial y (grid only), columns
+// shared memory of one CTA (doubles): v (two buffers), w, reduction slots and barriers; cluster: the
+// pairs (row element, y entry) received from all CTAs (two buffers) and the CTA's own pairs; grid: the
+// row groups' partial y; then 32 rows of the register columns, and the other columns
 __host__ __device__ constexpr int trd_stride(int n) { return (n + 31) & ~31; }
 __host__ __device__ constexpr int trd_slots(int n, int G, int TC) { return ((n + G - 1) / G + TC - 1) / TC; }
 __host__ __device__ constexpr int trd_smem_cols(int n, int G, int TC, int CR) {
@@ -40,8 +44,8 @@ __host__ __device__ constexpr int trd_smem_cols(int n, int G, int TC, int CR) {
 }
 __host__ __device__ constexpr int trd_ylen(int n, int G, int TC) { return trd_slots(n, G, TC) * TC; }
 __host__ __device__ constexpr long long trd_smem_doubles(int n, int G, int AW, int CR, bool grid) {
-    return (long long)trd_stride(n) * (grid ? 3 : 5) + 48 + (grid ? AW : 2) * trd_ylen(n, G, 8 / AW) +
-           (long long)trd_smem_cols(n, G, 8 / AW, CR) * trd_stride(n);
+    return (long long)trd_stride(n) * (grid ? 3 : 7) + 48 + (grid ? AW : 2) * trd_ylen(n, G, 8 / AW) +
+           32LL * CR * (8 / AW) + (long long)trd_smem_cols(n, G, 8 / AW, CR) * trd_stride(n);
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -50,48 +54,97 @@ __device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     return r;
 }
-__device__ __forceinline__ double ld_cluster(unsigned a) {
-    double v;
-    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
-    return v;
-}
 __device__ __forceinline__ void trd_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// a pair into another CTA's shared memory; its barrier there counts the bytes
+__device__ __forceinline__ void push_pair(unsigned dst, unsigned bar, double x, double y) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "d"(x), "d"(y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void bar_init(unsigned bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// waits (at most ~2^22 tries) for the barrier's phase to complete; false when it gave up
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned phase) {
+    for (int it = 0; it < (1 << 22); it++) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(phase)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+// a shared-memory load the compiler keeps where it is written (ahead of the branch that uses it)
+__device__ __forceinline__ double lds_now(unsigned a) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+}
+// sum of the eight warps' partials, in a fixed order
+__device__ __forceinline__ double sum8(const double* p) {
+    return ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+}
 
-// sums over the warp of four values per lane: the sum of value 2 b4 + b3 (b_k = bit k of the lane)
-__device__ __forceinline__ double warp_sum4(double y0, double y1, double y2, double y3) {
-    int lane = threadIdx.x & 31;
-    bool h = (lane & 16) != 0;
-    double a = (h ? y2 : y0) + __shfl_xor_sync(0xffffffffu, h ? y0 : y2, 16);
-    double b = (h ? y3 : y1) + __shfl_xor_sync(0xffffffffu, h ? y1 : y3, 16);
-    h = (lane & 8) != 0;
-    double s = (h ? b : a) + __shfl_xor_sync(0xffffffffu, h ? a : b, 8);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    return s;
+// sums over the warp of N values per lane (N = 1, 2, 4 or 8), each lane ending with the sum of one:
+// value `warp_sum_slot<N>(lane)`, the same tree for every value
+template <int N>
+__device__ __forceinline__ double warp_sum_n(const double* y) {
+    double t[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) t[u] = y[u];
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int w = N / 2; w >= 1; w >>= 1, o >>= 1) {
+        const bool h = (lane & o) != 0;
+#pragma unroll
+        for (int u = 0; u < w; u++) {
+            double keep = h ? t[w + u] : t[u], send = h ? t[u] : t[w + u];
+            t[u] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (; o >= 1; o >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
+    return t[0];
+}
+// the value a lane holds: its top log2(N) bits
+template <int N>
+__device__ __forceinline__ int warp_sum_slot(int lane) {
+    return N == 8 ? lane >> 2 : N == 4 ? lane >> 3 : N == 2 ? lane >> 4 : 0;
 }
 
 // One molecule: A = F (n x n, column-major, lower triangle valid) -> d, e, tau, and the reflectors
 // v_j over column j of F (zeros down to row j, one at row j + 1). xpub (grid only): 4 n doubles of
-// global memory for the published column and y.
+// global memory for the published pairs. false: a wait for the other CTAs gave up.
 template <int RT, int CR, int AW, bool GRID>
-__device__ __forceinline__ void trd_mol(int rank, int G, int n, double* __restrict__ F, double* __restrict__ d,
+__device__ __forceinline__ bool trd_mol(int rank, int G, int n, double* __restrict__ F, double* __restrict__ d,
                                         double* __restrict__ e, double* __restrict__ tau, double* xpub) {
     constexpr int TC = 8 / AW;
     constexpr int EQ = (32 * AW * RT + TRD_THREADS - 1) / TRD_THREADS;  // vector elements per thread
     constexpr int EB = EQ < 5 ? EQ : 5;                                  // ... in flight at a time
-    static_assert(GRID || EQ == EB, "cluster classes read a thread's elements in one go");
+    constexpr int GS = CR <= 8 ? CR : (CR + 1) / 2;  // register columns taken at a time
+    constexpr int NSUM = CR <= 4 ? 4 : 8, CY = (CR + NSUM - 1) / NSUM * NSUM;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int rg = wid % AW, cg = wid / AW;
     const int ns = trd_stride(n), ylen = trd_ylen(n, G, TC);
     const int nslot = trd_slots(n, G, TC);
     double* sv = s_work;              // two buffers
     double* sw = sv + 2 * ns;
-    double* sred = sw + ns;           // 2 x 8 partials, alpha
-    double* spub = sred + 48;         // cluster: y (2 x ylen) and column (2 x ns); grid: partial y (AW x ylen)
-    double* scol = GRID ? spub + AW * ylen : spub + 2 * ylen + 2 * ns;
+    double* sred = sw + ns;           // 2 x 8 partials, alpha; two barriers
+    double* rcv = sred + 48;          // cluster: received pairs (two buffers of ns)
+    double* stg = rcv + (GRID ? 0 : 4 * ns);  // cluster: own pairs; grid: partial y (AW x ylen)
+    double* spiv = stg + (GRID ? AW : 2) * ylen;  // register columns: the rows of the next row's block of 32
+    double* scol = spiv + 32 * CR * TC;
+    const unsigned bar0 = smem_addr(sred + 24);
     auto col_of = [&](int slot) { return (slot * TC + cg) * G + rank; };
     auto row_of = [&](int k) { return (k * AW + rg) * 32 + lane; };
     auto elem = [&](int r, int c) {
@@ -112,83 +165,112 @@ __device__ __forceinline__ void trd_mol(int rank, int G, int n, double* __restri
             if ((k * AW + rg) * 32 < ns) p[row_of(k)] = elem(row_of(k), c);
     }
     for (int i = tid; i < 3 * ns; i += TRD_THREADS) sv[i] = 0.0;
-    // publish column jn (held in register slot s of this warp's column group)
-    auto pub_reg = [&](double* dst, int s) {
+    if (!GRID && tid == 0) {
+        bar_init(bar0);
+        bar_init(bar0 + 8);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        bar_expect(bar0, 16 * n);
+    }
+    if (!GRID) {
+        __syncthreads();
+        trd_cluster_sync();  // the barriers are ready (and every CTA has read F: the reflectors go over it)
+    }
+    // element (next row, column of `slot`): global memory, or the CTA's own pairs
+    auto put_row = [&](int par, int slot, double a) {
+        const int l = slot * TC + cg, c = l * G + rank;
+        if (GRID) {
+            if (c < n) __stcg(xpub + 2 * ((long long)par * n + c), a);
+        } else stg[2 * l] = a;
+    };
+    // this lane's part of the pairs' distribution: CTA lane % G, slots lane / G, + 32 / G, ...
+    const int per = GRID ? 1 : 32 / G, dslot = GRID ? 0 : lane / G;
+    unsigned drcv = 0, dbar = 0;
+    if (!GRID) {
+        drcv = cluster_addr(smem_addr(rcv), lane % G);
+        dbar = cluster_addr(bar0, lane % G);
+    }
+    auto push = [&](int par, int first) {  // the warp's live columns (from column `first` on) to every CTA
+        if (GRID) return;
+        __syncwarp();
+        if (dslot < per)
+            for (int s = dslot; s < nslot; s += per) {
+                const int l = s * TC + cg, c = l * G + rank;
+                if (c >= first && c < n) {
+                    double2 v = reinterpret_cast<const double2*>(stg)[l];
+                    push_pair(drcv + 16 * (par * ns + c), dbar + 8 * par, v.x, v.y);
+                }
+            }
+        __syncwarp();
+    };
+    // The block of 32 rows that holds the next row lives in shared memory (one value per lane and
+    // register column): the register code then needs no row picked by a run-time index.
+    double* pv = spiv + 32 * cg + lane;
+    auto to_pivot = [&](int kb) {  // row slot kb of this thread
 #pragma unroll
-        for (int u = 0; u < CR; u++)
-            if (u == s) {
+        for (int k = 0; k < RT; k++)
+            if (k == kb) {
 #pragma unroll
-                for (int k = 0; k < RT; k++)
-                    if ((k * AW + rg) * 32 < ns) {
-                        if (GRID) {
-                            if (row_of(k) < n) __stcg(dst + row_of(k), A[k][u]);
-                        } else dst[row_of(k)] = A[k][u];
-                    }
+                for (int s = 0; s < CR; s++) pv[32 * TC * s] = A[k][s];
             }
     };
-    auto pub_col = [&](int par) { return GRID ? xpub + par * n : spub + 2 * ylen + par * ns; };
-    if (rank == 0 && cg == 0) pub_reg(pub_col(0), 0);
-    auto barrier = [&]() {
-        if (GRID) cg::this_grid().sync();
-        else trd_cluster_sync();
-    };
-    barrier();  // column 0 is published (and every CTA has read F: the reflectors go over it)
-    // cluster addresses of this thread's y entries (buffer 0)
-    unsigned yaddr[EQ];
-    if (!GRID) {
-#pragma unroll
-        for (int q = 0; q < EQ; q++) {
-            int i = tid + q * TRD_THREADS;
-            yaddr[q] = cluster_addr(smem_addr(spub) + 8 * (i / G), i % G);
+    // row 0 (= column 0) is published first
+    if (rg == 0) {
+        to_pivot(0);
+        if (lane == 0) {
+            for (int s = 0; s < nslot; s++)
+                put_row(0, s, s < CR ? pv[32 * TC * s] : scol[(long long)((s - CR) * TC + cg) * ns]);
+            if (!GRID)
+                for (int s = 0; s < nslot; s++) stg[2 * (s * TC + cg) + 1] = 0.0;
         }
     }
-    int cur = 0, own = 0, jl = 0;  // column j: CTA own, local column jl
+    push(0, 0);
+    bool ok = true;
+    if (GRID) cg::this_grid().sync();
+    int cur = 0, own = 0;  // own: the CTA that stores reflector j
     double tj = 0.0;
     for (int j = 0;; j++) {
         const int par = j & 1;
         double* v = sv + cur * ns;
         double* vn = sv + (cur ^ 1) * ns;
-        // (1) the published column j and y; y . v
-        unsigned ca = 0;
+        // (1) the published row j and y; y . v
         double yj;
+        const double2* prow;
         if (GRID) {
-            yj = j > 0 ? __ldcg(xpub + 2 * n + par * n + j) : 0.0;
+            prow = reinterpret_cast<const double2*>(xpub) + (long long)par * n;
+            yj = j > 0 ? __ldcg(&prow[j].y) : 0.0;
         } else {
-            ca = cluster_addr(smem_addr(pub_col(par)), own);
-            yj = j > 0 ? ld_cluster(cluster_addr(smem_addr(spub + par * ylen) + 8 * jl, own)) : 0.0;
+            // every pair has arrived: every warp with live columns, this CTA's too, has finished its
+            // last pass, and every CTA has read the buffer that the next pairs go to
+            if (ok) ok = bar_wait(bar0 + 8 * par, (j >> 1) & 1);
+            if (tid == 0 && j + 2 < n) bar_expect(bar0 + 8 * (par ^ 1), 16 * (n - min(j + 1, n - G)));
+            prow = reinterpret_cast<const double2*>(rcv) + par * ns;
+            yj = prow[j].y;
         }
         double dot = 0.0;
 #pragma unroll
         for (int q0 = 0; q0 < EQ; q0 += EB) {
-            double cv[EB], yv[EB];
+            double2 pv[EB];
 #pragma unroll
             for (int q = 0; q < EB; q++) {
                 int i = tid + (q0 + q) * TRD_THREADS;
-                bool ok = q0 + q < EQ && i >= j && i < n;
-                if (GRID) {
-                    cv[q] = ok ? __ldcg(xpub + par * n + i) : 0.0;
-                    yv[q] = ok && j > 0 ? __ldcg(xpub + 2 * n + par * n + i) : 0.0;
-                } else {
-                    cv[q] = ok ? ld_cluster(ca + 8 * i) : 0.0;
-                    yv[q] = ok && j > 0 ? ld_cluster(yaddr[q] + 8 * par * ylen) : 0.0;
-                }
+                pv[q] = make_double2(0.0, 0.0);
+                if (q0 + q < EQ && i >= j && i < n) pv[q] = GRID ? __ldcg(prow + i) : prow[i];
             }
 #pragma unroll
             for (int q = 0; q < EB; q++) {
                 int i = tid + (q0 + q) * TRD_THREADS;
                 if (q0 + q < EQ && i < ns) {
-                    dot = fma(yv[q], v[i], dot);
-                    vn[i] = cv[q];
-                    sw[i] = yv[q];
+                    double y = j > 0 ? pv[q].y : 0.0;  // no product yet before the first reflector
+                    dot = fma(y, v[i], dot);
+                    vn[i] = pv[q].x;
+                    sw[i] = y;
                 }
             }
         }
         dot = warp_sum(dot);
         if (lane == 0) sred[wid] = dot;
         __syncthreads();
-        double ds = 0.0;
-#pragma unroll
-        for (int q = 0; q < 8; q++) ds += sred[q];
+        const double ds = sum8(sred);
         // (2) w = tau (y - tau/2 (y.v) v); column j brought up to date with the previous reflector
         const double kap = 0.5 * tj * ds;
         const double vj = v[j], wj = tj * (yj - kap * vj);
@@ -219,19 +301,14 @@ __device__ __forceinline__ void trd_mol(int rank, int G, int n, double* __restri
             }
             const int c = n - 1;
             auto last = [&](double a) { d[n - 1] = a - v[c] * sw[c] - sw[c] * v[c]; };
-#pragma unroll
-            for (int s = 0; s < CR; s++)
-#pragma unroll
-                for (int k = 0; k < RT; k++)
-                    if (col_of(s) == c && row_of(k) == c) last(A[k][s]);
-            for (int s = CR; s < nslot; s++)
-                if (col_of(s) == c && (c >> 5) % AW == rg && (c & 31) == lane)
-                    last(scol[(long long)((s - CR) * TC + cg) * ns + c]);
+            const bool here = (c >> 5) % AW == rg && (c & 31) == lane;
+            if ((c & 31) == 0 && here) to_pivot(c / (32 * AW));  // a row block of its own, not reached before
+            for (int s = 0; s < nslot; s++)
+                if (col_of(s) == c && here)
+                    last(s < CR ? pv[32 * TC * s] : scol[(long long)((s - CR) * TC + cg) * ns + c]);
             break;
         }
-        double xn2 = 0.0;
-#pragma unroll
-        for (int q = 0; q < 8; q++) xn2 += sred[8 + q];
+        const double xn2 = sum8(sred + 8);
         // (3) the Householder vector of column j
         double beta, scale;
         if (xn2 == 0.0) {
@@ -239,14 +316,20 @@ __device__ __forceinline__ void trd_mol(int rank, int G, int n, double* __restri
             beta = alpha;
             scale = 0.0;
         } else {
-            beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-            tj = (beta - alpha) / beta;
+            // one reciprocal square root for both roots' uses: |beta| = sqrt(ss) after a Newton
+            // correction, tau = (beta - alpha) / beta = 1 + |alpha| / |beta|
+            const double ss = fma(alpha, alpha, xn2), r = rsqrt(ss), b0 = ss * r;
+            const double ab = fma(0.5 * r, fma(-b0, b0, ss), b0);
+            beta = -copysign(ab, alpha);
+            tj = fma(fabs(alpha), r, 1.0);
             scale = 1.0 / (alpha - beta);
         }
         if (tid == 0 && rank == 0) {
             e[j] = beta;
             tau[j] = tj;
         }
+        const bool mine = rank == own;
+        if (++own == G) own = 0;
 #pragma unroll
         for (int q = 0; q < EQ; q++) {
             int i = tid + q * TRD_THREADS;
@@ -254,130 +337,161 @@ __device__ __forceinline__ void trd_mol(int rank, int G, int n, double* __restri
                 double x = i > j + 1 ? vn[i] * scale : (i == j + 1 ? 1.0 : 0.0);
                 vn[i] = x;
                 if (i <= j) sw[i] = 0.0;
-                if (rank == own && i < n) F[i + (long long)j * n] = x;
+                if (mine && i < n) F[i + (long long)j * n] = x;
             }
         }
         __syncthreads();
         // (4) the pass: previous reflector applied, product with the new one
         const int jn = j + 1, npar = par ^ 1;
-        double* cdst = pub_col(npar);
-        auto put = [&](int slot, double y0, double y1, double y2, double y3, int cnt) {
-            double s = warp_sum4(y0, y1, y2, y3);
-            int u = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
-            if ((lane & 7) == 0 && u < cnt) {
-                int l = (slot + u) * TC + cg;
-                if (AW > 1) spub[rg * ylen + l] = s;
-                else if (GRID) {
-                    if (l * G + rank < n) __stcg(xpub + 2 * n + npar * n + l * G + rank, s);
-                } else spub[npar * ylen + l] = s;
-            }
+        auto put = [&](int slot, double s) {  // the product of column `slot`, its sum in this lane
+            const int l = slot * TC + cg;
+            if (GRID) stg[rg * ylen + l] = s;
+            else stg[2 * l + 1] = s;
         };
+        const unsigned av = smem_addr(v + rg * 32 + lane), aw = smem_addr(sw + rg * 32 + lane),
+                       an = smem_addr(vn + rg * 32 + lane);
+        const bool has_row = (jn >> 5) % AW == rg;  // this row group has the next row
+        const int kb = jn / (32 * AW);
+        if ((jn & 31) == 0 && has_row) to_pivot(kb);
+        const int b1 = AW == 1 ? 32 * RT : ns;  // AW = 1: RT is n's own, no row slot is empty
+        double y[CY];
 #pragma unroll
-        for (int g = 0; g < CR; g += 4) {
-            constexpr int GS = 4;
+        for (int u = 0; u < CY; u++) y[u] = 0.0;
+#pragma unroll
+        for (int g = 0; g < CR; g += GS) {
             // skipped: no columns of this molecule, or all of them done
-            if (g >= nslot || col_of(g + 3 < CR ? g + 3 : CR - 1) < jn) continue;
-            double wc[GS], vc[GS], y[GS];
+            if (g >= nslot || col_of(g + GS - 1 < CR ? g + GS - 1 : CR - 1) < jn) continue;
+            double wc[GS], vc[GS];
 #pragma unroll
             for (int u = 0; u < GS; u++) {
-                int c = col_of(g + u);
-                bool ok = g + u < CR && c < n;
-                wc[u] = ok ? sw[c] : 0.0;
-                vc[u] = ok ? v[c] : 0.0;
-                y[u] = 0.0;
+                int c = min(col_of(g + u), n - 1);  // a column the molecule does not have: never pushed
+                wc[u] = sw[c];
+                vc[u] = v[c];
+            }
+            double vr = lds_now(av), wr = lds_now(aw), nr = lds_now(an);
+            if (has_row) {
+                const double v0 = lds_now(av + 256 * AW * kb), w0 = lds_now(aw + 256 * AW * kb),
+                             n0 = lds_now(an + 256 * AW * kb);
+                double a[GS];
+#pragma unroll
+                for (int u = 0; u < GS; u++)
+                    if (g + u < CR) a[u] = pv[32 * TC * (g + u)];
+#pragma unroll
+                for (int u = 0; u < GS; u++)
+                    if (g + u < CR) {
+                        a[u] = fma(-v0, wc[u], a[u]);
+                        a[u] = fma(-w0, vc[u], a[u]);
+                        pv[32 * TC * (g + u)] = a[u];
+                        y[g + u] = a[u] * n0;
+                    }
+                if (lane == (jn & 31)) {
+#pragma unroll
+                    for (int u = 0; u < GS; u++)
+                        if (g + u < CR && g + u < nslot) put_row(npar, g + u, a[u]);
+                }
             }
 #pragma unroll
             for (int k = 0; k < RT; k++) {
                 const int b = (k * AW + rg) * 32;
-                if (b + 31 >= jn && b < ns) {
-                    double vr = v[b + lane], wr = sw[b + lane], nr = vn[b + lane];
+                const double v0 = vr, w0 = wr, n0 = nr;
+                if (k + 1 < RT && b + 32 * AW < b1) {  // the next row slot's vectors, in flight meanwhile
+                    vr = lds_now(av + 256 * AW * (k + 1));
+                    wr = lds_now(aw + 256 * AW * (k + 1));
+                    nr = lds_now(an + 256 * AW * (k + 1));
+                }
+                if (b > jn && b < b1) {
 #pragma unroll
                     for (int u = 0; u < GS; u++)
                         if (g + u < CR) {
                             double a = A[k][g + u];
-                            a = fma(-vr, wc[u], a);
-                            a = fma(-wr, vc[u], a);
+                            a = fma(-v0, wc[u], a);
+                            a = fma(-w0, vc[u], a);
                             A[k][g + u] = a;
-                            y[u] = fma(a, nr, y[u]);
+                            y[g + u] = fma(a, n0, y[g + u]);
                         }
                 }
             }
+        }
 #pragma unroll
-            for (int u = 0; u < GS; u++)
-                if (g + u < CR && col_of(g + u) == jn) pub_reg(cdst, g + u);
-            put(g, y[0], y[1], y[2], y[3], min(g + 4 <= CR ? 4 : CR - g, nslot - g));
+        for (int g = 0; g < CR; g += NSUM) {
+            if (g < nslot) {
+                double s = warp_sum_n<NSUM>(y + g);
+                const int u = warp_sum_slot<NSUM>(lane);
+                if ((lane & (32 / NSUM - 1)) == 0 && g + u < min(CR, nslot)) put(g + u, s);
+            }
         }
         const int k0 = jn / (32 * AW);  // row slots below hold finished rows only
+        const int k1 = min(RT, (ns / 32 - rg + AW - 1) / AW);
         for (int s = CR; s < nslot; s += 4) {
             const int cnt = min(4, nslot - s);
             if (col_of(s + cnt - 1) < jn) continue;
-            double wc[4], vc[4], y[4];
-            double* p = scol + (long long)((s - CR) * TC + cg) * ns;
-            const long long cs = (long long)TC * ns;
+            double wc[4], vc[4], ys[4];
+            const unsigned ac = smem_addr(scol + (long long)((s - CR) * TC + cg) * ns + rg * 32 + lane);
+            const unsigned cs = 8 * TC * ns;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                int c = col_of(s + u);
-                bool ok = u < cnt && c < n;
-                wc[u] = ok ? sw[c] : 0.0;
-                vc[u] = ok ? v[c] : 0.0;
-                y[u] = 0.0;
+                int c = min(col_of(s + u), n - 1);
+                wc[u] = sw[c];
+                vc[u] = v[c];
+                ys[u] = 0.0;
             }
             auto rows = [&](auto CN) {
                 constexpr int N = decltype(CN)::value;
-#pragma unroll 2
-                for (int k = k0; k < RT; k++) {
-                    const int b = (k * AW + rg) * 32;
-                    if (b >= ns) break;
-                    const int r = b + lane;
-                    double vr = v[r], wr = sw[r], nr = vn[r], a[N];
+                constexpr int KU = N == 1 ? 4 : N == 2 ? 3 : 2;  // rows loaded together
+                auto step = [&](auto KN, unsigned o) {
+                    constexpr int K = decltype(KN)::value;
+                    double v0[K], w0[K], n0[K], a[K][N];
 #pragma unroll
-                    for (int u = 0; u < N; u++) a[u] = p[u * cs + r];
+                    for (int k = 0; k < K; k++) {
+                        v0[k] = lds_now(av + o + 256 * AW * k);
+                        w0[k] = lds_now(aw + o + 256 * AW * k);
+                        n0[k] = lds_now(an + o + 256 * AW * k);
 #pragma unroll
-                    for (int u = 0; u < N; u++) {
-                        a[u] = fma(-vr, wc[u], a[u]);
-                        a[u] = fma(-wr, vc[u], a[u]);
-                        p[u * cs + r] = a[u];
-                        y[u] = fma(a[u], nr, y[u]);
+                        for (int u = 0; u < N; u++) a[k][u] = lds_now(ac + u * cs + o + 256 * AW * k);
                     }
+#pragma unroll
+                    for (int k = 0; k < K; k++)
+#pragma unroll
+                        for (int u = 0; u < N; u++) {
+                            double x = fma(-v0[k], wc[u], a[k][u]);
+                            x = fma(-w0[k], vc[u], x);
+                            asm volatile("st.shared.f64 [%0], %1;" ::"r"(ac + u * cs + o + 256 * AW * k), "d"(x));
+                            ys[u] = fma(x, n0[k], ys[u]);
+                        }
+                };
+                int k = k0;
+                for (; k + KU <= k1; k += KU) step(std::integral_constant<int, KU>(), 256 * AW * k);
+                for (; k < k1; k++) step(std::integral_constant<int, 1>(), 256 * AW * k);
+                if ((jn >> 5) % AW == rg && lane == (jn & 31)) {
+#pragma unroll
+                    for (int u = 0; u < N; u++) put_row(npar, s + u, lds_now(ac + u * cs + 8 * ((jn & ~31) - rg * 32)));
                 }
             };
             if (cnt == 4) rows(std::integral_constant<int, 4>());
             else if (cnt == 3) rows(std::integral_constant<int, 3>());
             else if (cnt == 2) rows(std::integral_constant<int, 2>());
             else rows(std::integral_constant<int, 1>());
-            for (int u = 0; u < cnt; u++)
-                if (col_of(s + u) == jn) {
-                    for (int k = 0; k < RT; k++) {
-                        const int b = (k * AW + rg) * 32;
-                        if (b >= ns) break;
-                        double a = p[u * cs + b + lane];
-                        if (GRID) {
-                            if (b + lane < n) __stcg(cdst + b + lane, a);
-                        } else cdst[b + lane] = a;
-                    }
-                }
-            put(s, y[0], y[1], y[2], y[3], cnt);
+            const double sum = warp_sum_n<4>(ys);
+            if ((lane & 7) == 0 && (lane >> 3) < cnt) put(s + (lane >> 3), sum);
         }
-        if (AW > 1) {
+        if (GRID) {
             __syncthreads();
             for (int l = tid; l < ylen; l += TRD_THREADS) {
                 int c = l * G + rank;
                 if (c >= jn && c < n) {
-                    double s = spub[l];
+                    double s = stg[l];
 #pragma unroll
-                    for (int q = 1; q < AW; q++) s += spub[q * ylen + l];
-                    __stcg(xpub + 2 * n + npar * n + c, s);
+                    for (int q = 1; q < AW; q++) s += stg[q * ylen + l];
+                    __stcg(xpub + 2 * ((long long)npar * n + c) + 1, s);
                 }
             }
-        }
-        barrier();
+            cg::this_grid().sync();
+        } else push(npar, min(jn, n - G));  // every CTA pushes at least one pair, live or not: none runs two ahead
         cur ^= 1;
-        if (++own == G) {
-            own = 0;
-            jl++;
-        }
     }
-    barrier();  // no CTA leaves (or starts the next molecule) while another reads its memory
+    // no CTA leaves (or starts the next molecule) while another writes its memory
+    if (!GRID) trd_cluster_sync();
+    return ok;
 }
 
 // SM cycles of the reduction into the profiler's counters (the molecule's counter in units of the
@@ -401,7 +515,9 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_trd(Batch B, State S, const 
     const int m = list[blockIdx.x / G];
     if (!S.active[m]) return;  // the same for the whole cluster
     const int n = B.m_nao[m], ao0 = B.m_ao0[m];
-    trd_mol<RT, CR, 1, false>((int)rank, (int)G, n, S.Fp + B.m_mat0[m], S.dtri + ao0, S.etri + ao0, S.tau + ao0, nullptr);
+    if (!trd_mol<RT, CR, 1, false>((int)rank, (int)G, n, S.Fp + B.m_mat0[m], S.dtri + ao0, S.etri + ao0, S.tau + ao0,
+                                   nullptr))
+        atomicOr(&S.status[m], ST_TIMEOUT);
     if (cycles) trd_cycles(S, m, (int)rank, (int)G, t0);
 }
 
@@ -416,27 +532,37 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_trd_grid(Batch B, State S, i
     if (cycles) trd_cycles(S, m, (int)blockIdx.x, (int)gridDim.x, t0);
 }
 
-// ---- size classes
+// ---- size classes: row slots per thread and register columns per warp (row group)
 struct TrdClass {
     int rt, cr;
     const void* fn;
 };
-// cluster path: row slots per thread (n <= 32 rt) and register columns per warp
-inline const TrdClass* trd_classes(int& count) {
-    static const TrdClass c[] = {{4, 16, (const void*)k_trd<4, 16>}, {6, 12, (const void*)k_trd<6, 12>},
-                                 {8, 9, (const void*)k_trd<8, 9>},   {12, 6, (const void*)k_trd<12, 6>},
-                                 {16, 5, (const void*)k_trd<16, 5>}, {19, 4, (const void*)k_trd<19, 4>},
-                                 {24, 3, (const void*)k_trd<24, 3>}};
-    count = 7;
-    return c;
+// cluster path: rt = ceil(n / 32) exactly; rt x cr values of the matrix per thread leave the other
+// ~90 of 255 registers to the pass. For clusters of G CTAs whose warps have few columns (clusters that
+// grew) a class with all of them in registers and nothing unrolled for columns that are not there.
+inline const TrdClass* trd_class(int n, int G = 0) {
+#define TRD_C(RT, CR) {RT, CR, (const void*)k_trd<RT, CR>}
+    static const TrdClass c[] = {TRD_C(4, 16), TRD_C(5, 13), TRD_C(6, 12), TRD_C(7, 10), TRD_C(8, 9),  TRD_C(9, 8),
+                                 TRD_C(10, 7), TRD_C(11, 7), TRD_C(12, 6), TRD_C(13, 6), TRD_C(14, 5), TRD_C(15, 5),
+                                 TRD_C(16, 5), TRD_C(17, 4), TRD_C(18, 4), TRD_C(19, 4), TRD_C(20, 4), TRD_C(21, 3),
+                                 TRD_C(22, 3), TRD_C(23, 3), TRD_C(24, 3)};
+    static const TrdClass f[] = {TRD_C(4, 4),  TRD_C(5, 4),  TRD_C(6, 4),  TRD_C(7, 4),  TRD_C(8, 4),  TRD_C(9, 4),
+                                 TRD_C(10, 4), TRD_C(11, 4), TRD_C(12, 4), TRD_C(13, 4), TRD_C(14, 4), TRD_C(15, 4),
+                                 TRD_C(16, 4), TRD_C(17, 5), TRD_C(18, 5), TRD_C(19, 5)};
+#undef TRD_C
+    const int rt = (n + 31) / 32;
+    if (rt < 4 || rt > 24) return nullptr;
+    return G > 0 && rt <= 19 && trd_slots(n, G, 8) <= f[rt - 4].cr ? f + (rt - 4) : c + (rt - 4);
 }
-// whole grid: n <= 256 rt, columns per CTA in registers
-inline const TrdClass* trd_grid_classes(int& count) {
-    static const TrdClass c[] = {{4, 8, (const void*)k_trd_grid<4, 8>},   {5, 9, (const void*)k_trd_grid<5, 9>},
-                                 {6, 11, (const void*)k_trd_grid<6, 11>}, {7, 12, (const void*)k_trd_grid<7, 12>},
-                                 {8, 10, (const void*)k_trd_grid<8, 10>}, {10, 8, (const void*)k_trd_grid<10, 8>}};
-    count = 6;
-    return c;
+constexpr int TRD_CLUSTER_MAX_NAO = 32 * 24;
+// whole grid: n <= 256 rt
+inline const TrdClass* trd_grid_class(int n) {
+#define TRD_C(RT, CR) {RT, CR, (const void*)k_trd_grid<RT, CR>}
+    static const TrdClass c[] = {TRD_C(4, 8), TRD_C(5, 9), TRD_C(6, 11), TRD_C(7, 11), TRD_C(8, 9), TRD_C(10, 9)};
+#undef TRD_C
+    for (const TrdClass& x : c)
+        if (n <= 256 * x.rt) return &x;
+    return nullptr;
 }
 
 }  // namespace axg
