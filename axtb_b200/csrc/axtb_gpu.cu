@@ -31,6 +31,8 @@
 #include "params/gfn2_tables.h"
 #include "team_kernel.cuh"
 #include "trd.cuh"
+#include "stages.cuh"
+#include "stages_chol.cuh"
 #include "chase.cuh"
 
 using std::vector;
@@ -345,13 +347,22 @@ struct AxtbBatch {
         const void* fn;
         int mol, smem;
     };
+    axg::StagePlan Q{};      // the molecules whose eigen phase runs in stages (those of trd and trd_grid)
+    long long q_full = 0, q_low = 0, q_rt = 0, q_vec = 0, q_col = 0;  // its tasks
+    bool q_wide = false, q_narrow = false;  // widths of the back-transformation's column blocks in use
+    int q_nmax = 0, q_natmax = 0;
+    int nteam_eigen = 0;     // the other molecules (team kernels)
     vector<TrdLaunch> trd;
     vector<TrdGrid> trd_grid;
     int grid_sms = 0;          // CTAs of k_trd_grid
     double* d_xpub = nullptr;  // what k_trd_grid's CTAs publish to one another
+    cudaStream_t fac_st = nullptr;   // the reflectors' triangular factors (stages.cuh)
+    cudaEvent_t fac_ev[2] = {nullptr, nullptr};
     vector<cudaStream_t> side;
     vector<cudaEvent_t> side_ev;  // fork, then one join per side stream
     void launch_trd();
+    void launch_stages();
+    void launch_cholesky(int eeq);
     void plan_trd(int big_nao, bool big_given, int band_max, const vector<int>& nao, int nsm, vector<int>& kind);
     void place_trd(const vector<int>& kind, const vector<int>& nao, int nsm,
                    const std::function<const int*(const vector<int>&)>& up);
@@ -407,6 +418,9 @@ AxtbBatch::~AxtbBatch() {
         if (e) cudaEventDestroy(e);
     for (auto& e : side_ev) cudaEventDestroy(e);
     for (auto& x : side) cudaStreamDestroy(x);
+    for (auto& e : fac_ev)
+        if (e) cudaEventDestroy(e);
+    if (fac_st) cudaStreamDestroy(fac_st);
     if (h_act) cudaFreeHost(h_act);
     if (h_stage) cudaFreeHost(h_stage);
     if (dmem) cudaFree(dmem);
@@ -503,6 +517,7 @@ void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int n
 void AxtbBatch::launch_trd() {
     for (auto& t : trd_grid) {
         void* args[] = {&B, &S, &t.mol, &d_xpub, &P.cycles};
+        CK(cudaMemsetAsync(d_xpub, 0, sizeof(double) * (4 * (size_t)mols[t.mol].nao + 1), st));  // no pair is there yet
         CK(cudaLaunchCooperativeKernel(t.fn, grid_sms, axg::TRD_THREADS, args, t.smem, st));
         launches++;
     }
@@ -530,6 +545,65 @@ void AxtbBatch::launch_trd() {
             CK(cudaStreamWaitEvent(st, side_ev[i], 0));
         }
     }
+}
+
+// The staged molecules' eigen phase (stages.cuh), between its tridiagonal reductions
+void AxtbBatch::launch_stages() {
+    using namespace axg;
+    const int W = SMEM_WORK_BYTES, T = TEAM_THREADS;
+    k_st_tiles<ST_X><<<(unsigned)q_full, T, W, st>>>(B, S, Q);
+    k_st_tiles<ST_FP><<<(unsigned)q_low, T, W, st>>>(B, S, Q);
+    launch_trd();
+    // the reflectors' triangular factors beside the levels and vectors of the tridiagonal matrices
+    CK(cudaEventRecord(fac_ev[0], st));
+    CK(cudaStreamWaitEvent(fac_st, fac_ev[0], 0));
+    k_st_tfac<<<(unsigned)q_rt, T, W, fac_st>>>(B, S, Q, P);
+    CK(cudaEventRecord(fac_ev[1], fac_st));
+    k_st_bisect<<<(unsigned)q_rt, T, 16 * (q_nmax + 32), st>>>(B, S, Q, 0);
+    k_st_fermi<<<(unsigned)Q.count, T, 24 * (q_nmax + 32), st>>>(B, S, Q);
+    for (int part = 0; part < 2; part++) {
+        k_st_invit<<<(unsigned)q_vec, 32, 16 * (q_nmax + 8), st>>>(B, S, Q, P, part);
+        k_st_gs<<<(unsigned)q_vec, 32, 0, st>>>(B, S, Q, P);
+    }
+    CK(cudaStreamWaitEvent(st, fac_ev[1], 0));
+    // the widest column blocks' shared memory is that of their largest molecule
+    if (q_narrow) k_st_apply<8><<<(unsigned)q_col, T, st_apply_doubles(q_nmax, 8) * 8, st>>>(B, S, Q, P);
+    if (q_wide) {
+        int n = q_nmax;
+        while (st_apply_doubles(n, 24) * 8 > TRD_SMEM_MAX) n -= 8;
+        k_st_apply<24><<<(unsigned)q_col, T, st_apply_doubles(n, 24) * 8, st>>>(B, S, Q, P);
+    }
+    k_st_tiles<ST_C><<<(unsigned)q_full, T, W, st>>>(B, S, Q);
+    k_st_tiles<ST_P><<<(unsigned)q_low, T, W, st>>>(B, S, Q);
+    launches += 11 + (q_narrow ? 1 : 0) + (q_wide ? 1 : 0);
+    CK(cudaGetLastError());
+}
+
+// Factor and inverse factor of the staged molecules' overlap matrices, or the EEQ charges from those
+// of their EEQ matrices
+void AxtbBatch::launch_cholesky(int eeq) {
+    using namespace axg;
+    const int W = SMEM_WORK_BYTES, T = TEAM_THREADS;
+    const int rt = ((eeq ? q_natmax : q_nmax) + CB - 1) / CB;
+    for (int c0 = 0; c0 < Q.count; c0 += 65535) {  // molecules along the grid's y
+        StagePlan q = Q;
+        q.mol = Q.mol + c0;
+        const unsigned cnt = (unsigned)std::min(65535, Q.count - c0);
+        k_ch_init<<<dim3(rt * rt, cnt), T, W, st>>>(B, S, q, P, eeq);
+        for (int p = 0; p < rt && rt > 1; p++) {
+            k_ch_panel<<<dim3(rt - 1, cnt), T, W, st>>>(B, S, q, P, p, eeq);
+            const int left = rt - 1 - p;
+            if (left > 0) k_ch_trail<<<dim3(left * (left + 1) / 2, cnt), T, W, st>>>(B, S, q, P, p, eeq);
+        }
+        launches += 2 * rt;
+        if (eeq) {
+            k_ch_eeq<<<dim3((q_natmax + 31) / 32, cnt), T, 0, st>>>(B, S, q, P, 0);
+            k_ch_eeq<<<dim3((q_natmax + 7) / 8, cnt), T, 0, st>>>(B, S, q, P, 1);
+            k_ch_eeq<<<dim3(1, cnt), T, 0, st>>>(B, S, q, P, 2);
+            launches += 3;
+        }
+    }
+    CK(cudaGetLastError());
 }
 
 void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
@@ -796,8 +870,9 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
             double c = std::pow((double)n + 32.0, 3.0);
             bool chased = n > axg::BW + 1 && n < band_max && n <= chase_max;
             smalls.push_back({c, m});
-            heads.push_back({chased ? 0.2 * c : trd_kind[m] ? 0.06 * c : c, m});
-            if (chased || trd_kind[m]) tails.push_back({chased ? 0.55 * c : 0.4 * c, m});
+            if (trd_kind[m]) continue;  // in stages
+            heads.push_back({chased ? 0.2 * c : c, m});
+            if (chased) tails.push_back({0.55 * c, m});
         }
         // longest first onto the least loaded CTA
         auto lpt = [&](vector<std::pair<double, int>>& items, vector<int>& off, vector<int>& list) {
@@ -846,9 +921,12 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     addI(tail_off.size());
     addI(tail_list.size() + 1);
     addI(nmol);                                              // trd_kind
+    addI(nmol);                                              // the stages' molecules, widths and tasks
+    addI(nmol);
+    for (int c = 0; c < 5; c++) addL((size_t)nmol + 1);
     for (int c = 0; c < 128; c++) addI(1);                   // k_trd lists: at most one per class and cluster size
     addI(nmol);
-    addD(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()));
+    addD(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()) + 1);
     {  // the chase plan (k_chase): offsets per cluster and per CTA, molecule lists
         size_t ncl = (size_t)std::max(1, nsm / 2);
         addI(ncl + 1);
@@ -1086,6 +1164,56 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     b.chase_max = chase_max;
     b.m_trd = upI(trd_kind);
     place_trd(trd_kind, m_nao, nsm, upI);
+    {  // the stages' tasks
+        vector<int> list, width;
+        for (int m = 0; m < nmol; m++)
+            if (trd_kind[m]) list.push_back(m);
+        // columns of the back-transformation per CTA: 24 (each block of reflectors read once per 24
+        // columns) when that fills the GPU and the molecule's rows fit, else 8
+        long long wide = 0;
+        for (int m : list) wide += (m_nao[m] / 2 + 23) / 24;
+        vector<long long> full{0}, low{0}, rts{0}, vec{0}, col{0};
+        for (int m : list) {
+            long long n = m_nao[m], rt = (n + axg::GT - 1) / axg::GT;
+            int w = wide >= nsm && axg::st_apply_doubles((int)n, 24) * 8 <= axg::TRD_SMEM_MAX ? 24 : 8;
+            width.push_back(w);
+            (w == 24 ? q_wide : q_narrow) = true;
+            q_nmax = std::max(q_nmax, (int)n);
+            q_natmax = std::max(q_natmax, mols[m].nat);
+            full.push_back(full.back() + rt * rt);
+            low.push_back(low.back() + rt * (rt + 1) / 2);
+            rts.push_back(rts.back() + rt);
+            vec.push_back(vec.back() + (n + 31) / 32);
+            col.push_back(col.back() + (n + w - 1) / w);
+        }
+        Q.count = (int)list.size();
+        nteam_eigen = nmol - Q.count;
+        q_full = full.back();
+        q_low = low.back();
+        q_rt = rts.back();
+        q_vec = vec.back();
+        q_col = col.back();
+        Q.mol = upI(list);
+        Q.width = upI(width);
+        Q.off_full = upL(full);
+        Q.off_low = upL(low);
+        Q.off_rt = upL(rts);
+        Q.off_vec = upL(vec);
+        Q.off_col = upL(col);
+        if (Q.count > 0) {
+            CK(cudaStreamCreateWithFlags(&fac_st, cudaStreamNonBlocking));
+            for (auto& e : fac_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            const void* tiles[] = {(const void*)axg::k_st_tiles<axg::ST_X>, (const void*)axg::k_st_tiles<axg::ST_FP>,
+                                   (const void*)axg::k_st_tiles<axg::ST_C>, (const void*)axg::k_st_tiles<axg::ST_P>,
+                                   (const void*)axg::k_st_tiles<axg::ST_W>, (const void*)axg::k_st_tfac,
+                                   (const void*)axg::k_st_bisect, (const void*)axg::k_st_fermi, (const void*)axg::k_ch_init,
+                                   (const void*)axg::k_ch_panel, (const void*)axg::k_ch_trail};
+            for (const void* f : tiles)
+                CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::SMEM_WORK_BYTES));
+            CK(cudaFuncSetAttribute(axg::k_st_apply<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
+            CK(cudaFuncSetAttribute(axg::k_st_apply<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
+        }
+    }
     vector<int> pair_off, pair_list, solo_off, solo_list;
     {
         // the plan: pairs (above CHASE_ROWS AOs) on clusters, then the rest one per CTA, longest
@@ -1235,7 +1363,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         s.sv_nbn = ar.take<int>(natT);
     }
     s.red = ar.take<double>((size_t)axg::team_red_doubles(grid));  // grid-team partials
-    d_xpub = ar.take<double>(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()));
+    d_xpub = ar.take<double>(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()) + 1);
     s.eeq_A = ar.take<double>((size_t)nsqT * 3);
     s.gam = ar.take<double>((size_t)std::max(ngamT, 1LL));
     // team plan
@@ -1560,7 +1688,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         ph = phase;
         Psmall = P;
         Psmall.nbig = 0;
-        if (P.nbig > 0) {
+        if (P.nbig > 0 && phase != PH_EIGEN_TAIL) {  // no whole-grid molecule has a part after k_chase
             CK(cudaLaunchCooperativeKernel((void*)k_team_grid, grid, TEAM_THREADS, args, SMEM_WORK_BYTES, st));
             launches++;
         }
@@ -1568,8 +1696,10 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     };
     double chol_flops = 0.0;
     for (int m = 0; m < nmol; m++) chol_flops += (1.0 / 3.0 + 2.0 / 3.0) * std::pow((double)mols[m].nao, 3.0);
-    LAUNCH("team_overlap", chol_flops, 0,
-           team_launch(PH_OVERLAP));
+    LAUNCH("team_overlap", chol_flops, 0, {
+        if (nteam_eigen > 0) team_launch(PH_OVERLAP);
+        if (Q.count > 0) launch_cholesky(0);
+    });
     bool eeq = opt.guess == 0 && eeq_guess && !warm;
     if (warm) {
         LAUNCH("start", 0, 0, k_start_warm<<<nmol, T, 0, st>>>(B, S, mixer_kind, nullptr));
@@ -1577,7 +1707,10 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         LAUNCH("eeq_matrix", 0, 0, k_eeq_matrix<<<blocks_for(nsqT, T), T, 0, st>>>(B, S, d_sq0, P.eeq_rhs, nsqT));
         double f = 0.0;
         for (int m = 0; m < nmol; m++) f += 3.0 * std::pow((double)mols[m].nat, 3.0);
-        LAUNCH("team_eeq", f, 0, team_launch(PH_EEQ));
+        LAUNCH("team_eeq", f, 0, {
+            if (nteam_eigen > 0) team_launch(PH_EEQ);
+            if (Q.count > 0) launch_cholesky(1);
+        });
     }
     if (!warm) LAUNCH("start", 0, 0, k_start<<<nmol, T, 0, st>>>(B, S, P.eeq_q, eeq ? 1 : 0, mixer_kind, nullptr));
     // restarts: a molecule with converged moments from the previous run starts from them
@@ -1594,18 +1727,17 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
             LAUNCH("fock", 0, mat_bytes(act, 12.0), k_fock<<<(unsigned)ntiles, T, 0, st>>>(B, S, d_tile0, ntiles));
             // the eigen phase: one launch, or three when k_chase takes stage 2 of some molecules
             LAUNCH("team_eigen", eig_flops(act), 0, {
-                team_launch(PH_EIGEN);
-                if (nchase > 0) {
-                    CP.cycles = P.cycles;
-                    k_chase<<<chase_grid, CHASE_THREADS, CHASE_DYN_BYTES, st>>>(B, S, CP);
-                    CK(cudaGetLastError());
-                    launches++;
+                if (nteam_eigen > 0) {
+                    team_launch(PH_EIGEN);
+                    if (nchase > 0) {
+                        CP.cycles = P.cycles;
+                        k_chase<<<chase_grid, CHASE_THREADS, CHASE_DYN_BYTES, st>>>(B, S, CP);
+                        CK(cudaGetLastError());
+                        team_launch(PH_EIGEN_TAIL);
+                        launches += 2;
+                    }
                 }
-                launch_trd();
-                if (nchase > 0 || !trd.empty() || !trd_grid.empty()) {
-                    team_launch(PH_EIGEN_TAIL);
-                    launches++;
-                }
+                if (Q.count > 0) launch_stages();
             });
             LAUNCH("mulliken", 0, mat_bytes(act, 12.0),
                    k_mulliken<<<blocks_for((long long)naoT * 32, T), T, 0, st>>>(B, S));
@@ -1662,11 +1794,21 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         CK(cudaMemcpyAsync(S.have_guess, S.conv, sizeof(int) * nmol, cudaMemcpyDeviceToDevice, st));
     }
     if (want_levels) {
-        LAUNCH("team_levels", 0, 0, team_launch(PH_LEVELS));
+        LAUNCH("team_levels", 0, 0, {
+            if (nteam_eigen > 0) team_launch(PH_LEVELS);
+            if (Q.count > 0) k_st_bisect<<<(unsigned)q_rt, TEAM_THREADS, 16 * (q_nmax + 32), st>>>(B, S, Q, 1);
+        });
     }
     CK(cudaEventRecord(phase_ev[2], st));
     if (want_grad) {
-        LAUNCH("team_wdens", w_flops(all), 0, team_launch(PH_WDENS));
+        LAUNCH("team_wdens", w_flops(all), 0, {
+            if (nteam_eigen > 0) team_launch(PH_WDENS);
+            if (Q.count > 0) {
+                k_st_scale<<<(unsigned)q_full, TEAM_THREADS, 0, st>>>(B, S, Q);
+                k_st_tiles<ST_W><<<(unsigned)q_low, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+                launches++;
+            }
+        });
         if (B.output_aes)
             LAUNCH("gradient_potentials", 0, 0,
                    k_gradient_potentials_aes<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));

@@ -197,9 +197,6 @@ __device__ void mol_eigen(const Team& t, const Batch& B, State& S, const TeamPla
         }
         team_sb2st(t, Fp, n, n, d, e, wk, S.W + mat);
         TEAM_PHASE(17);
-    } else if (B.m_trd && B.m_trd[m]) {  // the reduction and the rest in the next launches
-        if (P.cycles && t.tid() == 0) S.mol_cyc[m] = (double)(clock64() - tstart) * t.size;
-        return;
     } else {
         double* Vp = wk + 2 * n + (long long)nsl * n;  // the back-transform's vb area (64 n)
         team_tridiag_blocked<GRID_ROWS>(t, Fp, n, n, d, e, tau, Vp, Vp + (long long)NBP * n, vbuf, pbuf, ppart, S.red,
@@ -261,7 +258,7 @@ __device__ void mol_eigen(const Team& t, const Batch& B, State& S, const TeamPla
     t.sync();
     TEAM_PHASE(7);
     if (P.cycles && t.tid() == 0) {
-        double c = (double)(clock64() - tstart) * t.size;
+        double c = (double)(clock64() - tstart);
         if (after_chase) S.mol_cyc[m] += c;  // after the part before and the chase
         else S.mol_cyc[m] = c;
     }
@@ -297,7 +294,9 @@ __device__ void mol_levels(const Team& t, const Batch& B, State& S, const TeamPl
     team_bisect(t, d, e, n, S.emo + ao0, wk, kc, n);
 }
 
-__device__ __forceinline__ bool phase_wants(const State& S, int phase, int m) {
+// staged molecules (stages.cuh, stages_chol.cuh) have no part here
+__device__ __forceinline__ bool phase_wants(const Batch& B, const State& S, int phase, int m) {
+    if (B.m_trd[m]) return false;
     if (phase == PH_EIGEN || phase == PH_EIGEN_TAIL) return S.active[m] != 0;
     if (phase == PH_WDENS) return S.conv[m] != 0;
     return true;
@@ -310,7 +309,7 @@ __device__ void run_mol(const Team& t, const Batch& B, State& S, const TeamPlan&
         case PH_EEQ: mol_eeq(t, B, S, P, m); break;
         case PH_EIGEN:
         case PH_EIGEN_TAIL:
-            if (phase == PH_EIGEN || chased_on_chip(t, B, B.m_nao[m]) || (B.m_trd && B.m_trd[m])) mol_eigen<GRID_ROWS>(t, B, S, P, m, phase == PH_EIGEN_TAIL);
+            if (phase == PH_EIGEN || chased_on_chip(t, B, B.m_nao[m])) mol_eigen<GRID_ROWS>(t, B, S, P, m, phase == PH_EIGEN_TAIL);
             break;
         case PH_WDENS: mol_wdens(t, B, S, P, m); break;
         case PH_LEVELS: mol_levels(t, B, S, P, m); break;
@@ -323,14 +322,14 @@ __global__ void __launch_bounds__(TEAM_THREADS, 2) k_team(Batch B, State S, Team
     Team g{(int)blockIdx.x, (int)gridDim.x, true};
     for (int i = 0; i < P.nbig; i++) {
         int m = P.big[i];
-        if (phase_wants(S, phase, m)) run_mol<false>(g, B, S, P, phase, m);  // uniform across the grid
+        if (phase_wants(B, S, phase, m)) run_mol<false>(g, B, S, P, phase, m);  // uniform across the grid
     }
     Team one{0, 1, false};
     const int* off = phase == PH_EIGEN ? P.head_off : phase == PH_EIGEN_TAIL ? P.tail_off : P.small_off;
     const int* list = phase == PH_EIGEN ? P.head_list : phase == PH_EIGEN_TAIL ? P.tail_list : P.small_list;
     for (int i = off[blockIdx.x]; i < off[blockIdx.x + 1]; i++) {
         int m = list[i];
-        if (phase_wants(S, phase, m)) run_mol<false>(one, B, S, P, phase, m);
+        if (phase_wants(B, S, phase, m)) run_mol<false>(one, B, S, P, phase, m);
     }
 }
 
@@ -344,7 +343,7 @@ __global__ void __launch_bounds__(TEAM_THREADS, 2) k_team_grid(Batch B, State S,
     Team g{(int)blockIdx.x, (int)gridDim.x, true};
     for (int i = 0; i < P.nbig; i++) {
         int m = P.big[i];
-        if (phase_wants(S, phase, m)) run_mol<true>(g, B, S, P, phase, m);  // uniform across the grid
+        if (phase_wants(B, S, phase, m)) run_mol<true>(g, B, S, P, phase, m);  // uniform across the grid
     }
 }
 
