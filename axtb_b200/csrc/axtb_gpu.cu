@@ -358,12 +358,14 @@ struct AxtbBatch {
     double* d_xpub = nullptr;  // what k_trd_grid's CTAs publish to one another
     cudaStream_t fac_st = nullptr;   // the reflectors' triangular factors (stages.cuh)
     cudaEvent_t fac_ev[2] = {nullptr, nullptr};
+    cudaStream_t team_st = nullptr;  // the one-CTA molecules beside the stages
+    cudaEvent_t team_ev[2] = {nullptr, nullptr};
     vector<cudaStream_t> side;
     vector<cudaEvent_t> side_ev;  // fork, then one join per side stream
     void launch_trd();
     void launch_stages();
     void launch_cholesky(int eeq);
-    void plan_trd(int big_nao, bool big_given, int band_max, const vector<int>& nao, int nsm, vector<int>& kind);
+    void plan_trd(int big_nao, int band_max, const vector<int>& nao, int nsm, vector<int>& kind);
     void place_trd(const vector<int>& kind, const vector<int>& nao, int nsm,
                    const std::function<const int*(const vector<int>&)>& up);
     void* dmem = nullptr;
@@ -420,7 +422,10 @@ AxtbBatch::~AxtbBatch() {
     for (auto& x : side) cudaStreamDestroy(x);
     for (auto& e : fac_ev)
         if (e) cudaEventDestroy(e);
+    for (auto& e : team_ev)
+        if (e) cudaEventDestroy(e);
     if (fac_st) cudaStreamDestroy(fac_st);
+    if (team_st) cudaStreamDestroy(team_st);
     if (h_act) cudaFreeHost(h_act);
     if (h_stage) cudaFreeHost(h_stage);
     if (dmem) cudaFree(dmem);
@@ -428,14 +433,17 @@ AxtbBatch::~AxtbBatch() {
     if (st) cudaStreamDestroy(st);
 }
 
-// Which molecules reduce to tridiagonal form on chip (trd.cuh). From TRD_MIN_NAO AOs on (below it
-// the one-CTA reduction keeps the bits that some chaotic SCFs follow: the largest molecule that
-// does so in the recorded sets has 99 AOs), one molecule per cluster as long as 16 CTAs hold it
-// (768 AOs); from big_nao on, and above 768 AOs in batches of at most 64 such molecules (one after
-// the other on the whole grid at ~2.5 us per column beats one CTA each only while there are few),
-// on the whole grid as long as the chip holds the matrix.
-constexpr int TRD_MIN_NAO = 100;
-void AxtbBatch::plan_trd(int big_nao, bool big_given, int band_max, const vector<int>& nao, int nsm, vector<int>& kind) {
+// Which molecules' eigen phase runs in stages with the reduction on chip (stages.cuh, trd.cuh): from
+// TRD_MIN_NAO AOs on. Below it there is nothing to win (one water of 6 AOs: 121 us per iteration in
+// the one-CTA kernel, ~110 in stages, most of it launches), and the SCF of a water stretched to 3 A,
+// recorded as a failure in the tblite conventions, follows the one-CTA kernel's bits. A molecule sits
+// on a cluster as long as 16 CTAs hold it (768 AOs); from big_nao on, and above 768 AOs in batches of
+// at most 64 such molecules (one after the other at ~2.8 us per reflector they beat one CTA each, 296
+// at a time and ~85 ms, only while they are few), on the whole grid as long as the chip holds the
+// matrix (2400 AOs). A band_max_nao above its default asks for the two-stage reduction below it.
+constexpr int TRD_MIN_NAO = 12;
+void AxtbBatch::plan_trd(int big_nao, int band_max, const vector<int>& nao, int nsm, vector<int>& kind) {
+    const bool two_stage_asked = band_max > DEFAULT_BAND_MAX_NAO;
     int optin = 0, clusters = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     CK(cudaDeviceGetAttribute(&clusters, cudaDevAttrClusterLaunch, device));
@@ -446,9 +454,9 @@ void AxtbBatch::plan_trd(int big_nao, bool big_given, int band_max, const vector
     for (int m = 0; m < nmol; m++) {
         int n = nao[m];
         if (n < TRD_MIN_NAO) continue;
-        bool grid_mol = n >= big_nao || (n > cluster_max && !big_given && large <= 64);
+        bool grid_mol = n >= big_nao || (n > cluster_max && large <= 64);
         if (!grid_mol) {
-            if (n > cluster_max || (n > axg::BW + 1 && n < band_max)) continue;
+            if (n > cluster_max || (two_stage_asked && n > axg::BW + 1 && n < band_max)) continue;
             kind[m] = 1;
             continue;
         }
@@ -458,17 +466,16 @@ void AxtbBatch::plan_trd(int big_nao, bool big_given, int band_max, const vector
 }
 
 // The launches of the reductions on chip: per size class, molecules grouped by the cluster size
-// that holds them. With SMs to spare (few molecules) the clusters grow: fewer columns per CTA, the
-// same bits. Measured, us per reflector of one molecule, for 1 / 2 / 4 / 8 / 16 CTAs: 2.24 / 1.87 /
+// that holds them. The clusters of the molecules that would take longer than the whole batch's share
+// of the SMs grow: fewer columns per CTA, the same bits. Measured, us per reflector of one molecule, for 1 / 2 / 4 / 8 / 16 CTAs: 2.24 / 1.87 /
 // 1.38 / 1.37 / - at 120 AOs, 3.88 / 2.14 / 1.76 / 1.48 / - at 192, - / 4.27 / 2.87 / 2.19 / 1.80 at
 // 258, - / - / 3.66 / 2.14 / 1.95 at 378, and 3.46 / 2.88 for 10 / 16 at 600: up to 8 CTAs to 192
-// AOs, up to 16 above. A full GPU is best filled by the smallest clusters (CTAs x us grows with
-// the cluster at every size).
+// AOs, up to 16 above. A full GPU is best filled by the smallest clusters (CTAs x us grows with the
+// cluster at every size).
 void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int nsm,
                           const std::function<const int*(const vector<int>&)>& up) {
     std::map<std::pair<const axg::TrdClass*, int>, vector<int>> groups;  // (class, cluster size) -> molecules
     vector<int> G(nmol, 0);
-    long long need = 0;
     for (int m = 0; m < nmol; m++) {
         int n = nao[m];
         if (kind[m] == 2) {
@@ -478,13 +485,31 @@ void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int n
         if (kind[m] != 1) continue;
         G[m] = 1;
         while (axg::trd_smem_doubles(n, G[m], 1, axg::trd_class(n)->cr, false) * 8 > axg::TRD_SMEM_MAX) G[m]++;
-        need += G[m];
     }
-    int widen = 1;
-    while (widen < 16 && need * widen * 2 <= nsm) widen *= 2;
+    // us per reflector (a fit to the figures above): the chain, then the columns of a warp in registers
+    // and in shared memory
+    auto cost = [&](int n, int g) {
+        const int slots = axg::trd_slots(n, g, 8), cr = axg::trd_class(n, g)->cr;
+        return n * (1.0 + 0.0012 * n + n / 192.0 * (0.06 * std::min(slots, cr) + 0.13 * std::max(0, slots - cr)));
+    };
+    for (int grown = 1; grown;) {
+        double load = 0.0;
+        for (int m = 0; m < nmol; m++)
+            if (kind[m] == 1) load += G[m] * cost(nao[m], G[m]) / nsm;
+        grown = 0;
+        for (int m = 0; m < nmol; m++) {
+            const int n = nao[m], g = 2 * G[m];
+            if (kind[m] != 1 || g > (n <= 192 ? 8 : 16) || 8 * g > n) continue;
+            const double t = cost(n, G[m]);
+            if (t > 0.8 * load && cost(n, g) < 0.93 * t) {
+                G[m] = g;
+                grown = 1;
+            }
+        }
+    }
     for (int m = 0; m < nmol; m++)
         if (kind[m] == 1) {
-            int g = std::min(nao[m] <= 192 ? 8 : 16, G[m] * widen);
+            const int g = G[m];
             groups[{axg::trd_class(nao[m], g), g}].push_back(m);
         }
     for (auto& kv : groups) {
@@ -559,23 +584,32 @@ void AxtbBatch::launch_stages() {
     CK(cudaStreamWaitEvent(fac_st, fac_ev[0], 0));
     k_st_tfac<<<(unsigned)q_rt, T, W, fac_st>>>(B, S, Q, P);
     CK(cudaEventRecord(fac_ev[1], fac_st));
-    k_st_bisect<<<(unsigned)q_rt, T, 16 * (q_nmax + 32), st>>>(B, S, Q, 0);
+    k_st_bisect<<<(unsigned)q_vec, ST_POINTS, 16 * (q_nmax + 32), st>>>(B, S, Q, 0);
     k_st_fermi<<<(unsigned)Q.count, T, 24 * (q_nmax + 32), st>>>(B, S, Q);
     for (int part = 0; part < 2; part++) {
-        k_st_invit<<<(unsigned)q_vec, 32, 16 * (q_nmax + 8), st>>>(B, S, Q, P, part);
+        k_st_invit<<<(unsigned)q_vec, 32, st_invit_bytes(q_nmax), st>>>(B, S, Q, P, part);
         k_st_gs<<<(unsigned)q_vec, 32, 0, st>>>(B, S, Q, P);
     }
     CK(cudaStreamWaitEvent(st, fac_ev[1], 0));
-    // the widest column blocks' shared memory is that of their largest molecule
-    if (q_narrow) k_st_apply<8><<<(unsigned)q_col, T, st_apply_doubles(q_nmax, 8) * 8, st>>>(B, S, Q, P);
-    if (q_wide) {
-        int n = q_nmax;
-        while (st_apply_doubles(n, 24) * 8 > TRD_SMEM_MAX) n -= 8;
-        k_st_apply<24><<<(unsigned)q_col, T, st_apply_doubles(n, 24) * 8, st>>>(B, S, Q, P);
+    auto apply = [&](auto NC, auto NW, int n_lo, int n_hi) {
+        constexpr int C_ = decltype(NC)::value, W_ = decltype(NW)::value;
+        k_st_apply<C_, W_><<<(unsigned)q_col, 32 * W_, st_apply_doubles(n_hi, C_) * 8, st>>>(B, S, Q, P, n_lo, n_hi);
+        launches++;
+    };
+    std::integral_constant<int, 8> c8;
+    std::integral_constant<int, 16> c16;
+    std::integral_constant<int, 24> c24;
+    if (q_narrow) apply(c8, c16, 0, q_nmax);
+    if (q_wide) {  // molecules of which two CTAs fit a multiprocessor in a launch of their own
+        int half = q_nmax, all = q_nmax;
+        while (st_apply_doubles(half, 24) * 8 > TRD_SMEM_MAX / 2 - 1024) half -= 8;
+        while (st_apply_doubles(all, 24) * 8 > TRD_SMEM_MAX) all -= 8;
+        apply(c24, c8, 0, half);
+        if (all > half) apply(c24, c16, half, all);
     }
     k_st_tiles<ST_C><<<(unsigned)q_full, T, W, st>>>(B, S, Q);
     k_st_tiles<ST_P><<<(unsigned)q_low, T, W, st>>>(B, S, Q);
-    launches += 11 + (q_narrow ? 1 : 0) + (q_wide ? 1 : 0);
+    launches += 11;
     CK(cudaGetLastError());
 }
 
@@ -860,9 +894,10 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         // the eigen phase of a molecule whose bulge chasing runs on chip is split over two team
         // launches (before and after k_chase), each balanced on its own: measured shares of a
         // two-stage eigen phase, ~0.2 before (F' and stage 1) and ~0.55 after
-        plan_trd(big_nao, o.grid_min_nao > 0, band_max, m_nao, nsm, trd_kind);
+        plan_trd(big_nao, band_max, m_nao, nsm, trd_kind);
         for (int m = 0; m < nmol; m++) {
             int n = m_nao[m];
+            if (trd_kind[m]) continue;  // in stages
             if (n >= big_nao) {
                 big.push_back(m);
                 continue;
@@ -870,7 +905,6 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
             double c = std::pow((double)n + 32.0, 3.0);
             bool chased = n > axg::BW + 1 && n < band_max && n <= chase_max;
             smalls.push_back({c, m});
-            if (trd_kind[m]) continue;  // in stages
             heads.push_back({chased ? 0.2 * c : c, m});
             if (chased) tails.push_back({0.55 * c, m});
         }
@@ -1202,7 +1236,9 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         Q.off_col = upL(col);
         if (Q.count > 0) {
             CK(cudaStreamCreateWithFlags(&fac_st, cudaStreamNonBlocking));
+            CK(cudaStreamCreateWithFlags(&team_st, cudaStreamNonBlocking));
             for (auto& e : fac_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            for (auto& e : team_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             const void* tiles[] = {(const void*)axg::k_st_tiles<axg::ST_X>, (const void*)axg::k_st_tiles<axg::ST_FP>,
                                    (const void*)axg::k_st_tiles<axg::ST_C>, (const void*)axg::k_st_tiles<axg::ST_P>,
                                    (const void*)axg::k_st_tiles<axg::ST_W>, (const void*)axg::k_st_tfac,
@@ -1210,8 +1246,10 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
                                    (const void*)axg::k_ch_panel, (const void*)axg::k_ch_trail};
             for (const void* f : tiles)
                 CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::SMEM_WORK_BYTES));
-            CK(cudaFuncSetAttribute(axg::k_st_apply<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
-            CK(cudaFuncSetAttribute(axg::k_st_apply<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
+            const void* wide_smem[] = {(const void*)axg::k_st_apply<8, 16>, (const void*)axg::k_st_apply<24, 8>,
+                                       (const void*)axg::k_st_apply<24, 16>, (const void*)axg::k_st_invit};
+            for (const void* f : wide_smem)
+                CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
         }
     }
     vector<int> pair_off, pair_list, solo_off, solo_list;
@@ -1223,7 +1261,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         vector<std::pair<double, int>> pairs, solos;
         for (int m = 0; m < nmol; m++) {
             int n = m_nao[m];
-            if (is_big[m] || n <= axg::BW + 1 || n >= b.band_max || n > b.chase_max) continue;
+            if (is_big[m] || trd_kind[m] || n <= axg::BW + 1 || n >= b.band_max || n > b.chase_max) continue;
             if (n > axg::CHASE_ROWS) pairs.push_back({3.9 * n, m});
             else solos.push_back({3.0 * n, m});
         }
@@ -1684,15 +1722,17 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     TeamPlan Psmall = P;
     Psmall.nbig = 0;
     void* args_small[] = {&B, &S, &Psmall, &ph};
-    auto team_launch = [&](int phase) {
+    // (no one-CTA molecule needs the others' CTAs: a plain launch, which shares the GPU)
+    auto team_launch = [&](int phase, cudaStream_t on = nullptr) {
+        if (!on) on = st;
         ph = phase;
         Psmall = P;
         Psmall.nbig = 0;
         if (P.nbig > 0 && phase != PH_EIGEN_TAIL) {  // no whole-grid molecule has a part after k_chase
-            CK(cudaLaunchCooperativeKernel((void*)k_team_grid, grid, TEAM_THREADS, args, SMEM_WORK_BYTES, st));
+            CK(cudaLaunchCooperativeKernel((void*)k_team_grid, grid, TEAM_THREADS, args, SMEM_WORK_BYTES, on));
             launches++;
         }
-        CK(cudaLaunchCooperativeKernel((void*)k_team, grid, TEAM_THREADS, args_small, SMEM_WORK_BYTES, st));
+        CK(cudaLaunchKernel((void*)k_team, grid, TEAM_THREADS, args_small, SMEM_WORK_BYTES, on));
     };
     double chol_flops = 0.0;
     for (int m = 0; m < nmol; m++) chol_flops += (1.0 / 3.0 + 2.0 / 3.0) * std::pow((double)mols[m].nao, 3.0);
@@ -1727,17 +1767,26 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
             LAUNCH("fock", 0, mat_bytes(act, 12.0), k_fock<<<(unsigned)ntiles, T, 0, st>>>(B, S, d_tile0, ntiles));
             // the eigen phase: one launch, or three when k_chase takes stage 2 of some molecules
             LAUNCH("team_eigen", eig_flops(act), 0, {
+                // the one-CTA molecules beside the staged ones
+                const bool beside = nteam_eigen > 0 && Q.count > 0;
+                cudaStream_t x = beside ? team_st : st;
+                if (beside) {
+                    CK(cudaEventRecord(team_ev[0], st));
+                    CK(cudaStreamWaitEvent(x, team_ev[0], 0));
+                }
                 if (nteam_eigen > 0) {
-                    team_launch(PH_EIGEN);
+                    team_launch(PH_EIGEN, x);
                     if (nchase > 0) {
                         CP.cycles = P.cycles;
-                        k_chase<<<chase_grid, CHASE_THREADS, CHASE_DYN_BYTES, st>>>(B, S, CP);
+                        k_chase<<<chase_grid, CHASE_THREADS, CHASE_DYN_BYTES, x>>>(B, S, CP);
                         CK(cudaGetLastError());
-                        team_launch(PH_EIGEN_TAIL);
+                        team_launch(PH_EIGEN_TAIL, x);
                         launches += 2;
                     }
                 }
+                if (beside) CK(cudaEventRecord(team_ev[1], x));
                 if (Q.count > 0) launch_stages();
+                if (beside) CK(cudaStreamWaitEvent(st, team_ev[1], 0));
             });
             LAUNCH("mulliken", 0, mat_bytes(act, 12.0),
                    k_mulliken<<<blocks_for((long long)naoT * 32, T), T, 0, st>>>(B, S));
@@ -1796,7 +1845,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     if (want_levels) {
         LAUNCH("team_levels", 0, 0, {
             if (nteam_eigen > 0) team_launch(PH_LEVELS);
-            if (Q.count > 0) k_st_bisect<<<(unsigned)q_rt, TEAM_THREADS, 16 * (q_nmax + 32), st>>>(B, S, Q, 1);
+            if (Q.count > 0) k_st_bisect<<<(unsigned)q_vec, ST_POINTS, 16 * (q_nmax + 32), st>>>(B, S, Q, 1);
         });
     }
     CK(cudaEventRecord(phase_ev[2], st));

@@ -1,7 +1,7 @@
 // The eigen phase of the molecules whose tridiagonal reduction runs on chip (trd.cuh), one launch
 // per stage over all of them, each stage cut into the tasks that are independent in it:
 //   k_st_tiles   64 x 64 tiles of X = L^-1 F, F' = X L^-T, C = L^-T Z, P = (C f) C^T, W
-//   k_st_bisect  64 orbital energies per CTA
+//   k_st_bisect  32 orbital energies per CTA
 //   k_st_fermi   the filling, a CTA per molecule
 //   k_st_invit   one eigenvector of the tridiagonal matrix per thread, 32 per CTA
 //   k_st_gs      the clusters of close levels, a warp each
@@ -24,7 +24,7 @@ struct StagePlan {
     const long long* off_full;   // rt^2 tiles, rt = ceil(n / 64)
     const long long* off_low;    // rt (rt + 1) / 2 tiles on and below the diagonal
     const long long* off_rt;     // rt blocks of 64
-    const long long* off_vec;    // ceil(n / 32) blocks of 32 vectors
+    const long long* off_vec;    // ceil(n / 32) blocks of 32 levels or vectors
     const long long* off_col;    // column blocks of the back-transformation
     const int* width;            // ... and their width (8 or 24), per molecule
 };
@@ -197,24 +197,25 @@ __device__ int cta_tridiagonal(const double* d, const double* e, int n, double2*
 }
 
 // The levels k0 + (thread / 4) below k1 of one tridiagonal matrix, four threads a level: the counts
-// at 256 points of the Gershgorin interval bracket every level, then each group cuts its bracket
-// into five per pass (20 passes over the matrix where bisection takes 55: at one molecule the
+// at 128 points of the Gershgorin interval bracket every level, then each group cuts its bracket
+// into five per pass (21 passes over the matrix where bisection takes 55: at one molecule the
 // passes are a latency chain, and a full batch has the issue slots to spare).
+constexpr int ST_POINTS = 128;
 __device__ void cta_levels(const double2* de, int nb, const double* g, int k0, int k1, double* w) {
-    __shared__ int cnt[TEAM_THREADS];
+    __shared__ int cnt[ST_POINTS];
     const int tid = threadIdx.x;
-    const double step = (g[1] - g[0]) * (1.0 / (TEAM_THREADS + 1));
-    cnt[tid] = sturm_det(de, nb, g[0] + step * (tid + 1), g[2]);
+    const double step = (g[1] - g[0]) * (1.0 / (ST_POINTS + 1));
+    if (tid < ST_POINTS) cnt[tid] = sturm_det(de, nb, g[0] + step * (tid + 1), g[2]);
     __syncthreads();
     const int k = k0 + (tid >> 2), sub = tid & 3;
     bool live = k < k1;
-    int a = 0, b = TEAM_THREADS;  // smallest point with a count above k
+    int a = 0, b = ST_POINTS;  // smallest point with a count above k
     while (a < b) {
         int mid = (a + b) >> 1;
         if (cnt[mid] > k) b = mid;
         else a = mid + 1;
     }
-    double lo = a > 0 ? g[0] + step * a : g[0], hi = a < TEAM_THREADS ? g[0] + step * (a + 1) : g[1];
+    double lo = a > 0 ? g[0] + step * a : g[0], hi = a < ST_POINTS ? g[0] + step * (a + 1) : g[1];
     for (int it = 0; it < 200; it++) {
         double wd = hi - lo;
         if (bisect_done(lo, hi, g[2]) || lo + 0.2 * wd <= lo || lo + 0.8 * wd >= hi) live = false;
@@ -238,13 +239,15 @@ __device__ __forceinline__ int first_levels(const Batch& B, int m, int n) {
     return min(n, (int)ceil(fmax(B.m_nalpha[m], B.m_nbeta[m])) + max(16, n / 16));
 }
 
-// 64 levels per CTA. The SCF takes the lowest ceil(n_occ) + max(16, n/16) and gives the others the
-// Gershgorin bound; rest: those others (every orbital energy of the result).
-__global__ void __launch_bounds__(TEAM_THREADS) k_st_bisect(Batch B, State S, StagePlan Q, int rest) {
-    const int i = stage_find(Q.off_rt, Q.count, blockIdx.x), m = Q.mol[i];
+// 32 levels per CTA (128 threads: one warp per scheduler, so that the chain's latency and not its
+// issue slots set the time of a single molecule). The SCF takes the lowest ceil(n_occ) + max(16,
+// n/16) and gives the others the Gershgorin bound; rest: those others (every orbital energy of the
+// result).
+__global__ void __launch_bounds__(ST_POINTS) k_st_bisect(Batch B, State S, StagePlan Q, int rest) {
+    const int i = stage_find(Q.off_vec, Q.count, blockIdx.x), m = Q.mol[i];
     if (!rest && !S.active[m]) return;
     const int n = B.m_nao[m], ao0 = B.m_ao0[m], kc = first_levels(B, m, n);
-    const int k0 = 64 * (int)(blockIdx.x - Q.off_rt[i]), k1 = min(n, k0 + 64);
+    const int k0 = 32 * (int)(blockIdx.x - Q.off_vec[i]), k1 = min(n, k0 + 32);
     const int lo = rest ? max(k0, kc) : k0, hi = rest ? k1 : min(k1, kc);
     if (rest && lo >= hi) return;
     double2* de = reinterpret_cast<double2*>(s_work);
@@ -332,8 +335,8 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_fermi(Batch B, State S, Sta
 // and solves once, part 1 solves again, each followed by k_st_gs for the clusters (one thread took a
 // whole cluster before, and a launch was as long as its largest). The first forward substitution
 // rides on the factorisation, the factors hold reciprocal pivots (one division per row instead of
-// three), norms are summed as the solution is made and applied by the next reader, and eight rows'
-// loads are in flight while eight are worked on. The vectors stay where they are made,
+// three), norms are summed as the solution is made and applied by the next reader, and rows come
+// through a ring of asynchronous copies, 28 ahead. The vectors stay where they are made,
 // row-interleaved in the P plane ([row * n + vector]).
 struct Clusters {  // the clusters of a molecule's levels and the shifts of the solves
     double ctol, pert, pivmin;
@@ -348,6 +351,7 @@ __device__ __forceinline__ Clusters warp_clusters(const double* d, const double*
     return {1e-6 * tnrm, 10.0 * DBL_EPSILON * tnrm, DBL_EPSILON * tnrm};
 }
 
+__host__ __device__ constexpr int st_invit_bytes(int n) { return 8 * (2 * (n + 8) + 32 * 3 * 32); }
 __device__ __forceinline__ double* stage_norms(const TeamPlan& P, int m) { return P.wk + P.m_wk0[m] + 32; }
 
 __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, TeamPlan P, int part) {
@@ -366,12 +370,15 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
     __syncwarp();
     const Clusters cl = warp_clusters(sd, se, n);
     if (q >= k) return;
-    double* __restrict__ u0 = S.scr1 + mat + q;  // reciprocal pivots
-    double* __restrict__ u1 = S.scr2 + mat + q;
-    double* __restrict__ lm = S.scr3 + mat + q;
-    double* __restrict__ x = S.P + mat + q;
-    unsigned char* __restrict__ piv = S.piv + mat + q;
-    constexpr int U = 8;  // rows whose loads are in flight while the U before them are worked on
+    double* u0 = S.scr1 + mat + q;  // reciprocal pivots
+    double* u1 = S.scr2 + mat + q;
+    double* lm = S.scr3 + mat + q;
+    double* x = S.P + mat + q;
+    unsigned* swaps = reinterpret_cast<unsigned*>(S.piv + mat) + q;  // a bit per row, a word per 32 rows
+    // the thread's own ring of rows on their way from L2 or HBM
+    constexpr int GR = 4, NG = 8, R = GR * NG;
+    double* ring = s_work + 2 * (n + 8) + threadIdx.x;
+    auto slot = [&](int step, int f) { return ring + ((step & (R - 1)) * 3 + f) * 32; };
     double cur;
     if (part == 0) {
         // the shift: the level, kept apart from the cluster's earlier ones
@@ -381,6 +388,7 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
         for (int p = q0 + 1; p <= q; p++) lam = fmax(w[p], lam + cl.pert);
         // LU with partial pivoting of T - lam I, the start vector eliminated along
         double ca = sd[0] - lam, cb = se[0];
+        unsigned bits = 0;
         cur = hash_uniform((unsigned)q, 0u);
 #pragma unroll 4
         for (int i = 0; i + 1 < n; i++) {
@@ -394,78 +402,97 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
             u0[ix] = inv;
             u1[ix] = t1;
             lm[ix] = l;
-            piv[ix] = p;
             x[ix] = p ? nxt : cur;
+            bits |= (unsigned)p << (i & 31);
+            if ((i & 31) == 31) {
+                swaps[(i >> 5) * LD] = bits;
+                bits = 0;
+            }
             cur = (p ? cur : nxt) - l * (p ? nxt : cur);
             ca = (p ? cb : a1) - l * t1;
             cb = p ? -l * b1 : b1;
         }
+        swaps[((n - 1) >> 5) * LD] = bits;
         u0[(n - 1) * LD] = 1.0 / (ca == 0.0 ? cl.pivmin : ca);
     } else {
         // forward: L with the row interchanges, the first solution normalised on the way
         const double nr = stage_norms(P, m)[q];
-        cur = x[0] * nr;
-        double xv[2][U], l[2][U];
-        unsigned char pp[2][U];
-        auto fetch = [&](int i0, int h) {
+        auto issue = [&](int g) {
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                const long long ix = (long long)min(i0 + u, n - 2) * LD;
-                xv[h][u] = x[ix + LD];
-                l[h][u] = lm[ix];
-                pp[h][u] = piv[ix];
-            }
-        };
-        auto work = [&](int i0, int h) {
-#pragma unroll
-            for (int u = 0; u < U; u++)
-                if (i0 + u + 1 < n) {
-                    const double nxt = xv[h][u] * nr, top = pp[h][u] ? nxt : cur;
-                    x[(long long)(i0 + u) * LD] = top;
-                    cur = (pp[h][u] ? cur : nxt) - l[h][u] * top;
+            for (int u = 0; u < GR; u++) {
+                const int i = g * GR + u;
+                if (i + 1 < n) {
+                    cp_async8(slot(i, 0), x + (i + 1) * LD, true);
+                    cp_async8(slot(i, 1), lm + i * LD, true);
                 }
+            }
+            cp_async_commit();
         };
-        fetch(0, 0);
-        for (int i0 = 0; i0 + 1 < n; i0 += 2 * U) {
-            fetch(i0 + U, 1);
-            work(i0, 0);
-            fetch(i0 + 2 * U, 0);
-            work(i0 + U, 1);
+        cur = x[0] * nr;
+        unsigned bits = 0;
+        for (int g = 0; g < NG - 1; g++) issue(g);
+        for (int g = 0; g * GR + 1 < n; g++) {
+            cp_async_wait<NG - 2>();
+            if ((g * GR & 31) == 0) bits = swaps[(g * GR >> 5) * LD];
+            double xv[GR], l[GR];
+#pragma unroll
+            for (int u = 0; u < GR; u++) xv[u] = *slot(g * GR + u, 0), l[u] = *slot(g * GR + u, 1);
+            issue(g + NG - 1);
+#pragma unroll
+            for (int u = 0; u < GR; u++) {
+                const int i = g * GR + u;
+                if (i + 1 < n) {
+                    const bool p = bits >> (i & 31) & 1;
+                    const double nxt = xv[u] * nr, top = p ? nxt : cur;
+                    x[i * LD] = top;
+                    cur = (p ? cur : nxt) - l[u] * top;
+                }
+            }
         }
+        cp_async_wait<0>();
     }
     x[(n - 1) * LD] = cur;
     // backward: U with up to two superdiagonals (e_{i+1} after an interchange)
     double xn1 = 0.0, xn2 = 0.0, ss = 0.0;
-    double xv[2][U], f0[2][U], f1[2][U], f2[2][U];
-    auto fetch = [&](int i1, int h) {
+    auto issue = [&](int g) {
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int i = max(i1 - u, 0);
-            const long long ix = (long long)i * LD;
-            xv[h][u] = x[ix];
-            f0[h][u] = u0[ix];
-            f1[h][u] = i + 1 < n ? u1[ix] : 0.0;
-            f2[h][u] = i + 2 < n && piv[ix] ? se[i + 1] : 0.0;
+        for (int u = 0; u < GR; u++) {
+            const int st = g * GR + u, i = n - 1 - st;
+            if (i >= 0) {
+                cp_async8(slot(st, 0), x + i * LD, true);
+                cp_async8(slot(st, 1), u0 + i * LD, true);
+                cp_async8(slot(st, 2), u1 + i * LD, true);
+            }
         }
+        cp_async_commit();
     };
-    auto work = [&](int i1, int h) {
+    for (int g = 0; g < NG - 1; g++) issue(g);
+    unsigned bits = swaps[((n - 1) >> 5) * LD];
+    for (int g = 0; g * GR < n; g++) {
+        cp_async_wait<NG - 2>();
+        double xv[GR], f0[GR], f1[GR];
 #pragma unroll
-        for (int u = 0; u < U; u++)
-            if (i1 - u >= 0) {
-                double v = fma(-f1[h][u], xn1, fma(-f2[h][u], xn2, xv[h][u])) * f0[h][u];
-                x[(long long)(i1 - u) * LD] = v;
+        for (int u = 0; u < GR; u++) {
+            xv[u] = *slot(g * GR + u, 0);
+            f0[u] = *slot(g * GR + u, 1);
+            f1[u] = *slot(g * GR + u, 2);
+        }
+        issue(g + NG - 1);
+#pragma unroll
+        for (int u = 0; u < GR; u++) {
+            const int i = n - 1 - (g * GR + u);
+            if (i >= 0) {
+                if ((i & 31) == 31) bits = swaps[(i >> 5) * LD];
+                const double c1 = i + 1 < n ? f1[u] : 0.0, c2 = i + 2 < n && (bits >> (i & 31) & 1) ? se[i + 1] : 0.0;
+                double v = fma(-c1, xn1, fma(-c2, xn2, xv[u])) * f0[u];
+                x[i * LD] = v;
                 xn2 = xn1;
                 xn1 = v;
                 ss = fma(v, v, ss);
             }
-    };
-    fetch(n - 1, 0);
-    for (int i1 = n - 1; i1 >= 0; i1 -= 2 * U) {
-        fetch(i1 - U, 1);
-        work(i1, 0);
-        fetch(i1 - 2 * U, 0);
-        work(i1 - U, 1);
+        }
     }
+    cp_async_wait<0>();
     if (!(ss > 0.0) || !isfinite(ss)) {
         atomicOr(&S.status[m], ST_INVIT);
         ss = 1.0;
@@ -576,26 +603,28 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_tfac(Batch B, State S, Stag
     for (int e = threadIdx.x; e < ST_NB * ST_NB; e += blockDim.x) T[e] = st[(e / ST_NB) * LT + e % ST_NB];
 }
 
-// shared memory of k_st_apply (doubles): the columns, row by row, then two 64 x NC blocks. NC is 8
+// shared memory of k_st_apply (doubles): the columns, row by row, then three 64 x NC blocks. NC is 8
 // or 24: a row pitch of 8 mod 16 doubles serves the fragments without bank conflicts as it is.
-__host__ __device__ constexpr long long st_apply_doubles(int n, int nc) { return (long long)((n + 7) / 8 * 8 + 2 * ST_NB) * nc; }
+__host__ __device__ constexpr long long st_apply_doubles(int n, int nc) { return (long long)((n + 7) / 8 * 8 + 3 * ST_NB) * nc; }
 
 // Z <- Q Z for NC columns, held in shared memory from the first block of reflectors to the last:
 // per block Y = V^T Z, Y <- T Y, Z -= V Y on the FP64 tensor cores, V straight from L2 into the
-// fragments. Y's sum over the rows runs in four interleaved chains (row / 4 mod 4), added in order.
-template <int NC>
-__global__ void __launch_bounds__(TEAM_THREADS) k_st_apply(Batch B, State S, StagePlan Q, TeamPlan P) {
+// fragments. Y's sum over the rows runs in halves (row / 64 mod 2) of four interleaved chains (row / 4
+// mod 4), added in order: by 16 warps at once, or by 8 one half after the other (two CTAs per SM).
+template <int NC, int NW>
+__global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1) k_st_apply(Batch B, State S, StagePlan Q, TeamPlan P, int n_lo, int n_hi) {
     constexpr int NT = NC / 8, LP = NC;
     static_assert(NC % 16 == 8, "row pitch");
     const int ti = stage_find(Q.off_col, Q.count, blockIdx.x), m = Q.mol[ti];
     if (!S.active[m] || Q.width[ti] != NC) return;
     const int n = B.m_nao[m], k = S.kocc[m], c0 = NC * (int)(blockIdx.x - Q.off_col[ti]);
-    if (c0 >= k) return;
+    if (c0 >= k || n <= n_lo || n > n_hi) return;  // another launch's molecules: each asks for its own shared memory
     const long long mat = B.m_mat0[m];
     const int n8 = (n + 7) / 8 * 8, nrefl = n - 2;
     double* z = s_work;
     double* ya = z + (long long)n8 * LP;
-    double* yb = ya + ST_NB * LP;
+    double* yh = ya + ST_NB * LP;
+    double* yb = yh + ST_NB * LP;
     const double* V = S.Fp + mat;
     const double* X = S.P + mat;
     const double* T0 = P.wk + P.m_wk0[m] + stage_t_offset(n);
@@ -605,20 +634,20 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_apply(Batch B, State S, Sta
         z[r * LP + c] = r < n && c0 + c < k ? X[(long long)r * n + c0 + c] * norm[c0 + c] : 0.0;
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3, mt = warp & 7;
     for (int b0 = (nrefl - 1) / ST_NB * ST_NB; b0 >= 0; b0 -= ST_NB) {
         const int jb = min(ST_NB, nrefl - b0);
-        // Y: this warp's eight reflectors (one per lane group of four), rows from b0 on (zeros above b0 + 1)
-        {
-            const int c = b0 + 8 * warp + lr;
-            const bool in = 8 * warp + lr < jb;
+        // Y: eight reflectors per warp (one per lane group of four), rows from b0 on (zeros above b0 + 1)
+        for (int hf = warp >> 3; hf < 2; hf += NW / 8) {
+            const int c = b0 + 8 * mt + lr;
+            const bool in = 8 * mt + lr < jb;
             const double* vc = V + (long long)(in ? c : b0) * n;
             double acc[4][NT][2];
 #pragma unroll
             for (int s = 0; s < 4; s++)
 #pragma unroll
                 for (int t = 0; t < NT; t++) acc[s][t][0] = acc[s][t][1] = 0.0;
-            for (int r0 = b0; r0 < n; r0 += 64) {  // sixteen loads in flight per lane
+            for (int r0 = b0 + 64 * hf; r0 < n; r0 += 128) {  // sixteen loads in flight per lane
                 double a[16];
 #pragma unroll
                 for (int s = 0; s < 16; s++) {
@@ -634,27 +663,28 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_apply(Batch B, State S, Sta
                     for (int t = 0; t < NT; t++) dmma_8x8x4(acc[s & 3][t][0], acc[s & 3][t][1], a[s], zr[8 * t]);
                 }
             }
+            double* dst = hf ? yh : ya;
 #pragma unroll
             for (int t = 0; t < NT; t++)
-                *reinterpret_cast<double2*>(ya + (8 * warp + lr) * LP + 8 * t + 2 * lc) =
+                *reinterpret_cast<double2*>(dst + (8 * mt + lr) * LP + 8 * t + 2 * lc) =
                     make_double2(((acc[0][t][0] + acc[1][t][0]) + acc[2][t][0]) + acc[3][t][0],
                                  ((acc[0][t][1] + acc[1][t][1]) + acc[2][t][1]) + acc[3][t][1]);
         }
         __syncthreads();
-        {  // Y <- T Y (T upper triangular: rows from the warp's own on)
+        if (warp < 8) {  // Y <- T Y (T upper triangular: rows from the warp's own on)
             const double* T = T0 + (long long)b0 * ST_NB;
             double acc[NT][2];
 #pragma unroll
             for (int t = 0; t < NT; t++) acc[t][0] = acc[t][1] = 0.0;
-            for (int q = 8 * warp; q < ST_NB; q += 4) {
-                double a = T[8 * warp + lr + (q + lc) * ST_NB];
-                const double* yr = ya + (q + lc) * LP + lr;
+            for (int q = 8 * mt; q < ST_NB; q += 4) {
+                double a = T[8 * mt + lr + (q + lc) * ST_NB];
+                const int o = (q + lc) * LP + lr;
 #pragma unroll
-                for (int t = 0; t < NT; t++) dmma_8x8x4(acc[t][0], acc[t][1], a, yr[8 * t]);
+                for (int t = 0; t < NT; t++) dmma_8x8x4(acc[t][0], acc[t][1], a, ya[o + 8 * t] + yh[o + 8 * t]);
             }
 #pragma unroll
             for (int t = 0; t < NT; t++)
-                *reinterpret_cast<double2*>(yb + (8 * warp + lr) * LP + 8 * t + 2 * lc) = make_double2(acc[t][0], acc[t][1]);
+                *reinterpret_cast<double2*>(yb + (8 * mt + lr) * LP + 8 * t + 2 * lc) = make_double2(acc[t][0], acc[t][1]);
         }
         __syncthreads();
         // Z -= V Y: eight rows at a time per warp, the next eight rows of V in flight
@@ -668,11 +698,11 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_apply(Batch B, State S, Sta
             }
         };
         fetch(b0 + 8 * warp);
-        for (int r0 = b0 + 8 * warp; r0 < n; r0 += 64) {
+        for (int r0 = b0 + 8 * warp; r0 < n; r0 += 8 * NW) {
             double av[16];
 #pragma unroll
             for (int q = 0; q < 16; q++) av[q] = a[q];
-            fetch(r0 + 64);
+            fetch(r0 + 8 * NW);
             double acc[NT][2];
 #pragma unroll
             for (int t = 0; t < NT; t++) acc[t][0] = acc[t][1] = 0.0;

@@ -614,17 +614,17 @@ struct TrdClass {
 // grew) a class with all of them in registers and nothing unrolled for columns that are not there.
 inline const TrdClass* trd_class(int n, int G = 0) {
 #define TRD_C(RT, CR) {RT, CR, (const void*)k_trd<RT, CR>}
-    static const TrdClass c[] = {TRD_C(4, 16), TRD_C(5, 13), TRD_C(6, 12), TRD_C(7, 10), TRD_C(8, 9),  TRD_C(9, 8),
+    static const TrdClass c[] = {TRD_C(1, 4),  TRD_C(2, 8),  TRD_C(3, 12), TRD_C(4, 16), TRD_C(5, 13), TRD_C(6, 12), TRD_C(7, 10), TRD_C(8, 9),  TRD_C(9, 8),
                                  TRD_C(10, 7), TRD_C(11, 7), TRD_C(12, 6), TRD_C(13, 6), TRD_C(14, 5), TRD_C(15, 5),
                                  TRD_C(16, 5), TRD_C(17, 4), TRD_C(18, 4), TRD_C(19, 4), TRD_C(20, 4), TRD_C(21, 3),
                                  TRD_C(22, 3), TRD_C(23, 3), TRD_C(24, 3)};
-    static const TrdClass f[] = {TRD_C(4, 4),  TRD_C(5, 4),  TRD_C(6, 4),  TRD_C(7, 4),  TRD_C(8, 4),  TRD_C(9, 4),
+    static const TrdClass f[] = {TRD_C(1, 4),  TRD_C(2, 4),  TRD_C(3, 4),  TRD_C(4, 4),  TRD_C(5, 4),  TRD_C(6, 4),  TRD_C(7, 4),  TRD_C(8, 4),  TRD_C(9, 4),
                                  TRD_C(10, 4), TRD_C(11, 4), TRD_C(12, 4), TRD_C(13, 4), TRD_C(14, 4), TRD_C(15, 4),
                                  TRD_C(16, 4), TRD_C(17, 5), TRD_C(18, 5), TRD_C(19, 5)};
 #undef TRD_C
     const int rt = (n + 31) / 32;
-    if (rt < 4 || rt > 24) return nullptr;
-    return G > 0 && rt <= 19 && trd_slots(n, G, 8) <= f[rt - 4].cr ? f + (rt - 4) : c + (rt - 4);
+    if (rt < 1 || rt > 24) return nullptr;
+    return G > 0 && rt <= 19 && trd_slots(n, G, 8) <= f[rt - 1].cr ? f + (rt - 1) : c + (rt - 1);
 }
 constexpr int TRD_CLUSTER_MAX_NAO = 32 * 24;
 // whole grid: n <= 256 rt

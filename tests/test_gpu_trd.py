@@ -1,8 +1,7 @@
 """The tridiagonal reduction on chip (k_trd on a cluster, k_trd_grid on the whole grid; GPU).
 
 Sizes at the edges of the reduction's classes (a class holds 32 rows per row slot of a thread, a
-cluster grows by a CTA when its registers and shared memory are full, column slots come in groups
-of four), the smallest molecule that takes it and whole-grid sizes with columns in shared memory:
+cluster grows by a CTA when its registers and shared memory are full, column slots come in groups), the smallest molecule that takes it and whole-grid sizes with columns in shared memory:
 orbital energies from a plain generalized eigensolve of the engine's own Fock and overlap matrices
 (scipy, the eigenvalues' absolute error bounded by n eps ||F'||), the density's idempotency
 P S P = 2 P and electron count (round-off of n-term sums of elements of order 1), and the same bits
@@ -26,8 +25,9 @@ def _check(b, i, r):
     assert abs(np.trace(p @ s) - r.focc.sum()) < 4.0 * n * tol
 
 
-# basis functions: 102 (first), 128/132, 192/194, 252/258, 378/390, 510/516, 606/612, 768
-@pytest.mark.parametrize("sizes", [[17, 21, -21, -22], [32, -32, 42, 43], [63, 65], [85, 86, 101], [102, 128]])
+# basis functions: 12 and 14 (first), 30/32/36, 62/66, 96/98, 102, 126/128/132/134, 192/194, 252/258,
+# 378/390, 510/516, 606/612, 768
+@pytest.mark.parametrize("sizes", [[2, -2, 5, -5, 6], [-10, 11, 16, -16], [17, 21, -21, -22], [32, -32, 42, 43], [63, 65], [85, 86, 101], [102, 128]])
 def test_cluster_reduction(engine, sizes):
     from axtb_b200 import structures as S
 
