@@ -433,6 +433,79 @@ AxtbBatch::~AxtbBatch() {
     if (st) cudaStreamDestroy(st);
 }
 
+// ---- launches of the stages (stages.cuh, stages_chol.cuh, trd.cuh), shared by the batch engine and
+// the allocation-free entry point
+struct StageCounts {  // tasks; nmax: the largest matrix
+    int nmax;
+    long long full, low, rt, vec, col;
+};
+static void stage_attributes() {
+    using namespace axg;
+    const void* work[] = {(const void*)k_st_tiles<ST_X>, (const void*)k_st_tiles<ST_FP>, (const void*)k_st_tiles<ST_C>,
+                          (const void*)k_st_tiles<ST_P>, (const void*)k_st_tiles<ST_W>,  (const void*)k_st_tfac,
+                          (const void*)k_st_bisect,      (const void*)k_st_fermi,        (const void*)k_ch_init,
+                          (const void*)k_ch_panel,       (const void*)k_ch_trail};
+    for (const void* f : work) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WORK_BYTES));
+    const void* all[] = {(const void*)k_st_apply<8, 16>, (const void*)k_st_apply<24, 8>, (const void*)k_st_apply<24, 16>,
+                         (const void*)k_st_invit};
+    for (const void* f : all) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, TRD_SMEM_MAX));
+}
+// F' = L^-1 F L^-T
+static void stage_transform(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
+                            cudaStream_t st) {
+    using namespace axg;
+    k_st_tiles<ST_X><<<(unsigned)c.full, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+    k_st_tiles<ST_FP><<<(unsigned)c.low, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+}
+// count reductions of one class on clusters of G CTAs
+static void stage_reduce(const void* fn, int G, int count, int smem, const axg::Batch& B, const axg::State& S, const int* list,
+                         int cycles, cudaStream_t st) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = G;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(G * count));
+    cfg.blockDim = dim3(axg::TRD_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    void* args[] = {(void*)&B, (void*)&S, (void*)&list, (void*)&cycles};
+    CK(cudaLaunchKernelExC(&cfg, fn, args));
+}
+// levels, filling and vectors of the tridiagonal matrices
+static void stage_vectors(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P,
+                          const StageCounts& c, cudaStream_t st) {
+    using namespace axg;
+    k_st_bisect<<<(unsigned)c.vec, ST_POINTS, 16 * (c.nmax + 32), st>>>(B, S, Q, 0);
+    k_st_fermi<<<(unsigned)Q.count, TEAM_THREADS, 24 * (c.nmax + 32), st>>>(B, S, Q);
+    for (int part = 0; part < 2; part++) {
+        k_st_invit<<<(unsigned)c.vec, 32, st_invit_bytes(c.nmax), st>>>(B, S, Q, P, part);
+        k_st_gs<<<(unsigned)c.vec, 32, 0, st>>>(B, S, Q, P);
+    }
+}
+// C = L^-T Z and P = (C f) C^T
+static void stage_density(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
+                          cudaStream_t st) {
+    using namespace axg;
+    k_st_tiles<ST_C><<<(unsigned)c.full, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+    k_st_tiles<ST_P><<<(unsigned)c.low, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+}
+// factor and inverse factor of the overlap matrices, or of the EEQ matrices; nmax: the largest
+static void stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P, int nmax,
+                           int eeq, cudaStream_t st) {
+    using namespace axg;
+    const int W = SMEM_WORK_BYTES, T = TEAM_THREADS, rt = (nmax + CB - 1) / CB;
+    const unsigned cnt = (unsigned)Q.count;
+    k_ch_init<<<dim3(rt * rt, cnt), T, W, st>>>(B, S, Q, P, eeq);
+    for (int p = 0; p < rt && rt > 1; p++) {
+        k_ch_panel<<<dim3(rt - 1, cnt), T, W, st>>>(B, S, Q, P, p, eeq);
+        const int left = rt - 1 - p;
+        if (left > 0) k_ch_trail<<<dim3(left * (left + 1) / 2, cnt), T, W, st>>>(B, S, Q, P, p, eeq);
+    }
+}
+
 // Which molecules' eigen phase runs in stages with the reduction on chip (stages.cuh, trd.cuh): from
 // TRD_MIN_NAO AOs on. Below it there is nothing to win (one water of 6 AOs: 121 us per iteration in
 // the one-CTA kernel, ~110 in stages, most of it launches), and the SCF of a water stretched to 3 A,
@@ -551,19 +624,7 @@ void AxtbBatch::launch_trd() {
         TrdLaunch& t = trd[i];
         cudaStream_t x = i == 0 ? st : side[i - 1];
         if (i > 0) CK(cudaStreamWaitEvent(x, side_ev[0], 0));
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = t.G;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)(t.G * t.count));
-        cfg.blockDim = dim3(axg::TRD_THREADS);
-        cfg.dynamicSmemBytes = t.smem;
-        cfg.stream = x;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        void* args[] = {&B, &S, &t.list, &P.cycles};
-        CK(cudaLaunchKernelExC(&cfg, t.fn, args));
+        stage_reduce(t.fn, t.G, t.count, t.smem, B, S, t.list, P.cycles, x);
         launches++;
         if (i > 0) {
             CK(cudaEventRecord(side_ev[i], x));
@@ -575,21 +636,15 @@ void AxtbBatch::launch_trd() {
 // The staged molecules' eigen phase (stages.cuh), between its tridiagonal reductions
 void AxtbBatch::launch_stages() {
     using namespace axg;
-    const int W = SMEM_WORK_BYTES, T = TEAM_THREADS;
-    k_st_tiles<ST_X><<<(unsigned)q_full, T, W, st>>>(B, S, Q);
-    k_st_tiles<ST_FP><<<(unsigned)q_low, T, W, st>>>(B, S, Q);
+    const StageCounts cnt{q_nmax, q_full, q_low, q_rt, q_vec, q_col};
+    stage_transform(B, S, Q, cnt, st);
     launch_trd();
     // the reflectors' triangular factors beside the levels and vectors of the tridiagonal matrices
     CK(cudaEventRecord(fac_ev[0], st));
     CK(cudaStreamWaitEvent(fac_st, fac_ev[0], 0));
-    k_st_tfac<<<(unsigned)q_rt, T, W, fac_st>>>(B, S, Q, P);
+    k_st_tfac<<<(unsigned)q_rt, TEAM_THREADS, SMEM_WORK_BYTES, fac_st>>>(B, S, Q, P);
     CK(cudaEventRecord(fac_ev[1], fac_st));
-    k_st_bisect<<<(unsigned)q_vec, ST_POINTS, 16 * (q_nmax + 32), st>>>(B, S, Q, 0);
-    k_st_fermi<<<(unsigned)Q.count, T, 24 * (q_nmax + 32), st>>>(B, S, Q);
-    for (int part = 0; part < 2; part++) {
-        k_st_invit<<<(unsigned)q_vec, 32, st_invit_bytes(q_nmax), st>>>(B, S, Q, P, part);
-        k_st_gs<<<(unsigned)q_vec, 32, 0, st>>>(B, S, Q, P);
-    }
+    stage_vectors(B, S, Q, P, cnt, st);
     CK(cudaStreamWaitEvent(st, fac_ev[1], 0));
     auto apply = [&](auto NC, auto NW, int n_lo, int n_hi) {
         constexpr int C_ = decltype(NC)::value, W_ = decltype(NW)::value;
@@ -607,8 +662,7 @@ void AxtbBatch::launch_stages() {
         apply(c24, c8, 0, half);
         if (all > half) apply(c24, c16, half, all);
     }
-    k_st_tiles<ST_C><<<(unsigned)q_full, T, W, st>>>(B, S, Q);
-    k_st_tiles<ST_P><<<(unsigned)q_low, T, W, st>>>(B, S, Q);
+    stage_density(B, S, Q, cnt, st);
     launches += 11;
     CK(cudaGetLastError());
 }
@@ -617,18 +671,14 @@ void AxtbBatch::launch_stages() {
 // of their EEQ matrices
 void AxtbBatch::launch_cholesky(int eeq) {
     using namespace axg;
-    const int W = SMEM_WORK_BYTES, T = TEAM_THREADS;
+    const int T = TEAM_THREADS;
     const int rt = ((eeq ? q_natmax : q_nmax) + CB - 1) / CB;
     for (int c0 = 0; c0 < Q.count; c0 += 65535) {  // molecules along the grid's y
         StagePlan q = Q;
         q.mol = Q.mol + c0;
         const unsigned cnt = (unsigned)std::min(65535, Q.count - c0);
-        k_ch_init<<<dim3(rt * rt, cnt), T, W, st>>>(B, S, q, P, eeq);
-        for (int p = 0; p < rt && rt > 1; p++) {
-            k_ch_panel<<<dim3(rt - 1, cnt), T, W, st>>>(B, S, q, P, p, eeq);
-            const int left = rt - 1 - p;
-            if (left > 0) k_ch_trail<<<dim3(left * (left + 1) / 2, cnt), T, W, st>>>(B, S, q, P, p, eeq);
-        }
+        q.count = (int)cnt;
+        stage_cholesky(B, S, q, P, eeq ? q_natmax : q_nmax, eeq, st);
         launches += 2 * rt;
         if (eeq) {
             k_ch_eeq<<<dim3((q_natmax + 31) / 32, cnt), T, 0, st>>>(B, S, q, P, 0);
@@ -983,6 +1033,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     addD((size_t)nshT + (size_t)natT * 10);          // start moments
     addD((size_t)nshT * 3 + (size_t)natT * 2 + (size_t)natT * 6 + (size_t)natT * 12 + (size_t)nshT + natT * 10);
     addD((size_t)natT * 14);
+    addD((size_t)natT * 14);
     addD((size_t)naoT * 11);
     addD((size_t)nvecT * 4 + (size_t)nhist * 2 + (size_t)nmol * hist_cap * hist_cap * 2 + (size_t)nmol * hist_cap);
     addD((size_t)nmol * 14);
@@ -1239,17 +1290,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
             CK(cudaStreamCreateWithFlags(&team_st, cudaStreamNonBlocking));
             for (auto& e : fac_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             for (auto& e : team_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            const void* tiles[] = {(const void*)axg::k_st_tiles<axg::ST_X>, (const void*)axg::k_st_tiles<axg::ST_FP>,
-                                   (const void*)axg::k_st_tiles<axg::ST_C>, (const void*)axg::k_st_tiles<axg::ST_P>,
-                                   (const void*)axg::k_st_tiles<axg::ST_W>, (const void*)axg::k_st_tfac,
-                                   (const void*)axg::k_st_bisect, (const void*)axg::k_st_fermi, (const void*)axg::k_ch_init,
-                                   (const void*)axg::k_ch_panel, (const void*)axg::k_ch_trail};
-            for (const void* f : tiles)
-                CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::SMEM_WORK_BYTES));
-            const void* wide_smem[] = {(const void*)axg::k_st_apply<8, 16>, (const void*)axg::k_st_apply<24, 8>,
-                                       (const void*)axg::k_st_apply<24, 16>, (const void*)axg::k_st_invit};
-            for (const void* f : wide_smem)
-                CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
+            stage_attributes();
         }
     }
     vector<int> pair_off, pair_list, solo_off, solo_list;
@@ -1363,6 +1404,8 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     s.vqp = ar.take<double>(natT * 6);
     s.gw = ar.take<double>(natT * 7);
     s.dgw = ar.take<double>(natT * 7);
+    s.gwk = ar.take<double>(natT * 7);
+    s.dgwk = ar.take<double>(natT * 7);
     s.ao_part = ar.take<double>((size_t)naoT * 11);
     s.q_in = ar.take<double>(nvecT);
     s.dq = ar.take<double>(nvecT);
@@ -1691,10 +1734,11 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     LAUNCH("repulsion", 0, 0, k_repulsion<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));
     LAUNCH("mol_sum", 0, 0, k_mol_sum<<<nmol, T, 0, st>>>(B, S.e_atom, S.e_fixed));
     CK(cudaMemsetAsync(S.e_atom, 0, sizeof(double) * natT, st));
+    LAUNCH("d4_weights", 0, 0, k_d4_cn_weights<<<blocks_for((long long)natT * MAXREF, T), T, 0, st>>>(B, S));
     // D4 three-body at q = 0 with dgw/dCN weights (none without the D4 term)
     if (B.disp) {
         CK(cudaMemsetAsync(P.eeq_q, 0, sizeof(double) * natT, st));
-        LAUNCH("d4_weights", 0, 0, k_d4_weights<<<blocks_for(natT, T), T, 0, st>>>(B, S, P.eeq_q, 1));
+        LAUNCH("d4_weights", 0, 0, k_d4_weights<<<blocks_for((long long)natT * MAXREF, T), T, 0, st>>>(B, S, P.eeq_q, 1));
         LAUNCH("atm_tables", 0, 0, k_atm_tables<<<blocks_for(nsqT, T), T, 0, st>>>(B, S, d_wt, d_tt, d_sq0, nsqT));
         if (npairT > 0)
             LAUNCH("atm", 0, 0,
@@ -1760,7 +1804,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     // for the molecules it left unconverged DIIS from the same start (auto); or one mixer alone
     auto scf_attempt = [&](bool diis) {
         for (int it = 1; it <= opt.max_iter; it++) {
-            LAUNCH("d4_weights", 0, 0, k_d4_weights<<<blocks_for(natT, T), T, 0, st>>>(B, S, S.qat_in, 0));
+            LAUNCH("d4_weights", 0, 0, k_d4_weights<<<blocks_for((long long)natT * MAXREF, T), T, 0, st>>>(B, S, S.qat_in, 0));
             LAUNCH("potentials", 0, 0, k_potentials<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));
             if (B.solv)
                 LAUNCH("solv_potential", 0, 0, k_solv_potential<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));
@@ -1791,7 +1835,6 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
             LAUNCH("mulliken", 0, mat_bytes(act, 12.0),
                    k_mulliken<<<blocks_for((long long)naoT * 32, T), T, 0, st>>>(B, S));
             LAUNCH("moments", 0, 0, k_moments<<<blocks_for(natT, T), T, 0, st>>>(B, S));
-            LAUNCH("d4_weights", 0, 0, k_d4_weights<<<blocks_for(natT, T), T, 0, st>>>(B, S, S.qat_out, 2));
             LAUNCH("energy", 0, 0, k_energy<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));
             if (B.solv)
                 LAUNCH("solv_energy", 0, 0, k_solv_energy<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));
@@ -1865,7 +1908,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
             LAUNCH("h0_gradient", 0, mat_bytes(all, 2.0),
                    k_h0_gradient<<<blocks_for(npairT, 128), 128, 0, st>>>(B, S, d_pair0, npairT, S.pair_buf));
         LAUNCH("h0_gather", 0, 0, k_h0_gather<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S, d_pair0, S.pair_buf));
-        LAUNCH("d4_weights", 0, 0, k_d4_weights<<<blocks_for(natT, T), T, 0, st>>>(B, S, S.qat_out, 1));
+        LAUNCH("d4_weights", 0, 0, k_d4_weights<<<blocks_for((long long)natT * MAXREF, T), T, 0, st>>>(B, S, S.qat_out, 1));
         LAUNCH("grad_pairs", 0, 0, k_grad_pairs<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));
         if (B.solv) {
             unsigned wb = blocks_for((long long)natT * 32, T);
@@ -1898,7 +1941,7 @@ static_assert(STATIC_WK >= axg::band_workspace(STATIC_MAX_NAO) && STATIC_WK >= a
               "the static workspace holds the eigen phase's layout at the largest molecule");
 constexpr long long STATIC_VEC = 8LL * STATIC_MAX_NAO;                           // d, e, tau + spare
 constexpr long long STATIC_PIV = STATIC_PLANE / 8;                               // pivot bytes, as doubles
-constexpr long long STATIC_PAR = 64;                                             // small parameters
+constexpr long long STATIC_PAR = 128;                                            // small parameters
 constexpr long long STATIC_DOUBLES = 8 * STATIC_PLANE + STATIC_WK + STATIC_VEC + STATIC_PIV + STATIC_PAR;
 static __device__ __align__(256) double g_density_scratch[STATIC_DOUBLES];  // 4.89 MiB
 
@@ -1907,19 +1950,21 @@ double* g_static_addr[256] = {nullptr};
 }  // namespace
 
 namespace axg {
-// one CTA: parameters into the static area, then the factorisation and the eigen phase
+// parameters into the static area (one thread); off: the stages' task offsets, {0, count} each
+__device__ void density_static_setup(const Batch& B, State& S, const TeamPlan& P, int nao, double nalpha, double nbeta) {
+    *const_cast<int*>(B.m_nao) = nao;
+    *const_cast<int*>(B.m_ao0) = 0;
+    *const_cast<long long*>(B.m_mat0) = 0;
+    *const_cast<long long*>(P.m_wk0) = 0;
+    *const_cast<double*>(B.m_nalpha) = nalpha;
+    *const_cast<double*>(B.m_nbeta) = nbeta;
+    S.status[0] = 0;  // the array keeps the previous call's words
+    S.kocc[0] = 0;
+}
+// one CTA: the factorisation and the eigen phase of a molecule below TRD_MIN_NAO
 __global__ void __launch_bounds__(TEAM_THREADS)
     k_density_static(Batch B, State S, TeamPlan P, int nao, double nalpha, double nbeta, int* d_status) {
-    if (threadIdx.x == 0) {
-        *const_cast<int*>(B.m_nao) = nao;
-        *const_cast<int*>(B.m_ao0) = 0;
-        *const_cast<long long*>(B.m_mat0) = 0;
-        *const_cast<long long*>(P.m_wk0) = 0;
-        *const_cast<double*>(B.m_nalpha) = nalpha;
-        *const_cast<double*>(B.m_nbeta) = nbeta;
-        S.status[0] = 0;  // the array keeps the previous call's words
-        S.kocc[0] = 0;
-    }
+    if (threadIdx.x == 0) density_static_setup(B, S, P, nao, nalpha, nbeta);
     __syncthreads();
     Team one{0, 1, false};
     mol_overlap(one, B, S, P, 0);
@@ -1927,6 +1972,15 @@ __global__ void __launch_bounds__(TEAM_THREADS)
     mol_levels(one, B, S, P, 0);  // every orbital energy, not only the ones the filling needs
     if (threadIdx.x == 0 && d_status) *d_status = S.status[0];
 }
+__global__ void k_density_setup(Batch B, State S, TeamPlan P, StagePlan Q, int nao, double nalpha, double nbeta, int width) {
+    density_static_setup(B, S, P, nao, nalpha, nbeta);
+    S.active[0] = 1;
+    *const_cast<int*>(Q.mol) = 0;
+    *const_cast<int*>(Q.width) = width;
+    const long long* off[] = {Q.off_full, Q.off_low, Q.off_rt, Q.off_vec, Q.off_col};
+    for (const long long* o : off) *const_cast<long long*>(o) = 0;
+}
+__global__ void k_density_status(State S, int* d_status) { *d_status = S.status[0]; }
 }  // namespace axg
 
 extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_overlap, int32_t nao, double nalpha,
@@ -1960,6 +2014,15 @@ extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_ove
             if (e == cudaSuccess)  // the kernel's dynamic shared work area (no device allocation)
                 e = cudaFuncSetAttribute((const void*)axg::k_density_static, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          axg::SMEM_WORK_BYTES);
+            try {
+                stage_attributes();
+                for (int n = TRD_MIN_NAO; n <= STATIC_MAX_NAO; n++)
+                    for (int g = 1; g <= 8; g *= 2)
+                        CK(cudaFuncSetAttribute(axg::trd_class(n, g)->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                axg::TRD_SMEM_MAX));
+            } catch (const std::exception&) {
+                e = cudaErrorUnknown;
+            }
             if (e != cudaSuccess) {
                 g_static_addr[dev] = nullptr;
                 g_last_error = std::string("axtb_gpu_density_static: device set-up: ") + cudaGetErrorString(e);
@@ -2011,8 +2074,45 @@ extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_ove
     B.kt = kt;
     B.band_max = STATIC_BAND_MAX_NAO;
     B.chase_max = 0;  // stage 2 in this kernel
-    axg::k_density_static<<<1, axg::TEAM_THREADS, axg::SMEM_WORK_BYTES, (cudaStream_t)stream>>>(B, S, P, nao, nalpha, nbeta,
-                                                                                              d_status);
+    cudaStream_t on = (cudaStream_t)stream;
+    if (nao < TRD_MIN_NAO) {
+        axg::k_density_static<<<1, axg::TEAM_THREADS, axg::SMEM_WORK_BYTES, on>>>(B, S, P, nao, nalpha, nbeta, d_status);
+    } else {  // the batch engine's stages for the one molecule, all on the caller's stream
+        using namespace axg;
+        StagePlan Q{};
+        Q.count = 1;
+        Q.mol = reinterpret_cast<const int*>(par + 80);
+        Q.width = reinterpret_cast<const int*>(par + 81);
+        Q.off_full = reinterpret_cast<const long long*>(par + 82);
+        Q.off_low = reinterpret_cast<const long long*>(par + 83);
+        Q.off_rt = reinterpret_cast<const long long*>(par + 84);
+        Q.off_vec = reinterpret_cast<const long long*>(par + 85);
+        Q.off_col = reinterpret_cast<const long long*>(par + 86);
+        S.active = reinterpret_cast<int*>(par + 87);
+        S.mol_cyc = par + 88;
+        k_density_setup<<<1, 1, 0, on>>>(B, S, P, Q, nao, nalpha, nbeta, 8);
+        const long long rt = (nao + GT - 1) / GT;
+        const StageCounts c{nao, rt * rt, rt * (rt + 1) / 2, rt, (nao + 31) / 32, (nao + 7) / 8};
+        int G = 1;  // the cluster that holds the matrix, grown while each warp keeps a column
+        while (trd_smem_doubles(nao, G, 1, trd_class(nao, G)->cr, false) * 8 > TRD_SMEM_MAX) G *= 2;
+        while (G < 8 && 16 * G <= nao) G *= 2;
+        const TrdClass* cls = trd_class(nao, G);
+        const int cycles = 0;
+        try {
+            stage_cholesky(B, S, Q, P, nao, 0, on);
+            stage_transform(B, S, Q, c, on);
+            stage_reduce(cls->fn, G, 1, (int)(trd_smem_doubles(nao, G, 1, cls->cr, false) * 8), B, S, Q.mol, cycles, on);
+            k_st_tfac<<<(unsigned)c.rt, TEAM_THREADS, SMEM_WORK_BYTES, on>>>(B, S, Q, P);
+            stage_vectors(B, S, Q, P, c, on);
+            k_st_apply<8, 16><<<(unsigned)c.col, 512, st_apply_doubles(nao, 8) * 8, on>>>(B, S, Q, P, 0, nao);
+            stage_density(B, S, Q, c, on);
+            k_st_bisect<<<(unsigned)c.vec, ST_POINTS, 16 * (nao + 32), on>>>(B, S, Q, 1);
+        } catch (const Fail& f) {
+            g_last_error = std::string("axtb_gpu_density_static: launch: ") + f.what();
+            return AXTB_ERR_DEVICE;
+        }
+        if (d_status) k_density_status<<<1, 1, 0, on>>>(S, d_status);
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         g_last_error = std::string("axtb_gpu_density_static: launch: ") + cudaGetErrorString(e);

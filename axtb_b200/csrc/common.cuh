@@ -108,6 +108,7 @@ struct State {
     double *qsh_out, *qat_out, *dp_out, *qp_out;
     double *vsh, *vat, *vdp, *vqp;  // potentials of the last Fock build
     double *gw, *dgw;               // D4 weights and their charge (or CN) derivatives [natT][MAXREF]
+    double *gwk, *dgwk;             // their CN parts and CN derivatives (once per geometry)
     double *ao_part;                // naoT * 11: per-AO column dots (S, D3, Q6, H0)
     // mixer
     double *q_in, *dq, *qlast, *dqlast, *df, *u, *amat, *omega;  // vecs; df/u: hist x vec

@@ -144,59 +144,72 @@ __global__ void k_repulsion(Batch B, State S) {
 }
 
 // D4 reference weights (crates/d4/src/model.rs:474-570) at charges q; mode 0: dgw = dgw/dq,
-// 1: dgw = dgw/dCN, 2: no derivative. One thread per atom.
+// 1: dgw = dgw/dCN, 2: no derivative.
+// charge scaling of reference r's weight (gwk, dgwk: its CN part) into gw and its derivative into dgw
+__device__ __forceinline__ void d4_weight(const Batch& B, const State& S, int a, int r, double qa, int mode) {
+    const int sp = B.a_sp[a];
+    double gw = 0.0, dg = 0.0;
+    if (r < B.sp_nref[sp]) {
+        const double zi = B.sp_zeff[sp], gi = B.sp_gi[sp], gwk = S.gwk[(long long)a * MAXREF + r];
+        double qref = B.sp_refq[sp * MAXREF + r] + zi, qmod = qa + zi;
+        double z, dz = 0.0;
+        if (qmod < 0.0) {
+            z = exp(D4_GA);
+        } else {
+            double e = exp(gi * (1.0 - qref / qmod));
+            z = exp(D4_GA * (1.0 - e));
+            dz = -((D4_GA * gi * e * z * qref) / (qmod * qmod));
+        }
+        gw = gwk * z;
+        if (mode == 0) dg = gwk * dz;
+        else if (mode == 1) dg = S.dgwk[(long long)a * MAXREF + r] * z;
+    }
+    S.gw[(long long)a * MAXREF + r] = gw;
+    S.dgw[(long long)a * MAXREF + r] = dg;
+}
+// mode 0: derivatives by charge, 1: by CN, 2: none; a thread per atom and reference (one thread per
+// atom with the CN parts formed again in each call was a chain of ~60 exponentials: 10 us a launch)
 __global__ void k_d4_weights(Batch B, State S, const double* q, int mode) {
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= B.natT) return;
+    int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= B.natT * MAXREF) return;
+    int a = g / MAXREF;
+    d4_weight(B, S, a, g - a * MAXREF, q[a], mode);
+}
+// the CN parts of the weights and their derivatives, once per geometry
+__global__ void k_d4_cn_weights(Batch B, State S) {
+    int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= B.natT * MAXREF) return;
+    const int a = g / MAXREF, r = g - a * MAXREF;
     int sp = B.a_sp[a];
     int nr = B.sp_nref[sp];
+    if (r >= nr) return;
     const int* ngw = B.sp_ngw + sp * MAXREF;
     const double* refcn = B.sp_refcn + sp * MAXREF;
-    const double* refq = B.sp_refq + sp * MAXREF;
-    double zi = B.sp_zeff[sp], gi = B.sp_gi[sp], cni = S.cn_d4[a];
+    double cni = S.cn_d4[a];
     double norm = 0.0, dnorm = 0.0;
-    for (int r = 0; r < nr; r++)
-        for (int ig = 1; ig <= ngw[r]; ig++) {
-            double wf = ig * D4_WF, dd = cni - refcn[r];
+    for (int t = 0; t < nr; t++)
+        for (int ig = 1; ig <= ngw[t]; ig++) {
+            double wf = ig * D4_WF, dd = cni - refcn[t];
             double g = exp(-(wf * (dd * dd)));
             norm += g;
-            dnorm += 2.0 * wf * (refcn[r] - cni) * g;
+            dnorm += 2.0 * wf * (refcn[t] - cni) * g;
         }
     norm = fabs(norm) > sqrt(DBL_MIN) ? 1.0 / norm : 0.0;
     double maxcn = -INFINITY;
-    for (int r = 0; r < nr; r++) maxcn = fmax(maxcn, refcn[r]);
-    for (int r = 0; r < MAXREF; r++) {
-        double gw = 0.0, dg = 0.0;
-        if (r < nr) {
-            double expw = 0.0, expd = 0.0;
-            for (int ig = 1; ig <= ngw[r]; ig++) {
-                double wf = ig * D4_WF, dd = cni - refcn[r];
-                double g = exp(-(wf * (dd * dd)));
-                expw += g;
-                expd += 2.0 * wf * (refcn[r] - cni) * g;
-            }
-            double gwk = expw * norm;
-            if (!isfinite(gwk) || norm == 0.0) gwk = fabs(maxcn - refcn[r]) < 1e-12 ? 1.0 : 0.0;
-            double qref = refq[r] + zi, qmod = q[a] + zi;
-            double z, dz = 0.0;
-            if (qmod < 0.0) {
-                z = exp(D4_GA);
-            } else {
-                double e = exp(gi * (1.0 - qref / qmod));
-                z = exp(D4_GA * (1.0 - e));
-                dz = -((D4_GA * gi * e * z * qref) / (qmod * qmod));
-            }
-            gw = gwk * z;
-            if (mode == 0) dg = gwk * dz;
-            else if (mode == 1) {
-                double dgwk = norm * (expd - expw * dnorm * norm);
-                if (!isfinite(dgwk) || norm == 0.0) dgwk = 0.0;
-                dg = dgwk * z;
-            }
-        }
-        S.gw[(long long)a * MAXREF + r] = gw;
-        S.dgw[(long long)a * MAXREF + r] = dg;
+    for (int t = 0; t < nr; t++) maxcn = fmax(maxcn, refcn[t]);
+    double expw = 0.0, expd = 0.0;
+    for (int ig = 1; ig <= ngw[r]; ig++) {
+        double wf = ig * D4_WF, dd = cni - refcn[r];
+        double g = exp(-(wf * (dd * dd)));
+        expw += g;
+        expd += 2.0 * wf * (refcn[r] - cni) * g;
     }
+    double gwk = expw * norm;
+    if (!isfinite(gwk) || norm == 0.0) gwk = fabs(maxcn - refcn[r]) < 1e-12 ? 1.0 : 0.0;
+    double dgwk = norm * (expd - expw * dnorm * norm);
+    if (!isfinite(dgwk) || norm == 0.0) dgwk = 0.0;
+    S.gwk[g] = gwk;
+    S.dgwk[g] = dgwk;
 }
 
 // C6 of a pair and its derivatives through the weight derivatives dgw (crates/d4/src/model.rs:577-631)

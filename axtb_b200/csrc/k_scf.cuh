@@ -250,6 +250,7 @@ __global__ void k_moments(Batch B, State S) {
         qa += q;
     }
     S.qat_out[a] = qa;
+    for (int r = 0; r < MAXREF; r++) d4_weight(B, S, a, r, qa, 2);  // the D4 weights of the output charge
     for (int k = 0; k < 3; k++) S.dp_out[3 * a + k] = dp[k];
     for (int k = 0; k < 6; k++) S.qp_out[6 * a + k] = qp[k];
     S.e_atom[a] = band;  // band part of the atom's electronic energy; the rest is added next
@@ -321,6 +322,7 @@ __global__ void k_energy(Batch B, State S) {
 }
 
 // ----------------------------------------------------------------------------- Broyden
+constexpr int BROYDEN_SMALL = 24;  // a system of up to this many vectors is solved in shared memory
 __device__ double cta_sum(double v) {
     __shared__ double red[32];
     __shared__ double out;
@@ -336,6 +338,29 @@ __device__ double cta_sum(double v) {
     }
     __syncthreads();
     return out;
+}
+
+// sums of N values per thread, each in cta_sum's order, behind one set of barriers
+template <int N>
+__device__ void cta_sums(double (&v)[N]) {
+    __shared__ double red[N][32];
+    __shared__ double out[N];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int u = 0; u < N; u++) v[u] = warp_sum(v[u]);
+    __syncthreads();
+    if (l == 0)
+#pragma unroll
+        for (int u = 0; u < N; u++) red[u][w] = v[u];
+    __syncthreads();
+    if (threadIdx.x < N) {
+        double s = 0.0;
+        for (int k = 0; k < nw; k++) s += red[threadIdx.x][k];
+        out[threadIdx.x] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < N; u++) v[u] = out[u];
 }
 
 __device__ __forceinline__ void pack_moment(const Batch& B, int m, const double* qsh, const double* dp, const double* qp,
@@ -364,36 +389,25 @@ __device__ bool scf_iteration_end(const Batch& B, const State& S, int m) {
     double* q_in = S.q_in + v0;
     double* dq = S.dq + v0;
     // energy and terms (sums in atom order per thread stripe, reduced deterministically)
-    double e = 0.0, t2 = 0.0, t3 = 0.0, ta = 0.0, td = 0.0, tb = 0.0;
+    double v[7] = {};  // energy, its five terms, squared residual
     for (int a = tid; a < nat; a += nthr) {
-        e += S.e_atom[a0 + a];
-        t2 += S.e_terms[5 * (a0 + a) + 0];
-        t3 += S.e_terms[5 * (a0 + a) + 1];
-        ta += S.e_terms[5 * (a0 + a) + 2];
-        td += S.e_terms[5 * (a0 + a) + 3];
-        tb += S.e_terms[5 * (a0 + a) + 4];
+        v[0] += S.e_atom[a0 + a];
+        for (int k = 0; k < 5; k++) v[1 + k] += S.e_terms[5 * (a0 + a) + k];
     }
-    e = cta_sum(e) + S.ts[m];
     if (B.solv) {  // the solvation term (crates/axtb/src/calculator.rs:314)
         double es = 0.0;
         for (int a = tid; a < nat; a += nthr) es += S.sv_eatom[a0 + a];
         es = cta_sum(es);
         if (tid == 0) S.sv_emol[m] = es;
     }
-    t2 = cta_sum(t2);
-    t3 = cta_sum(t3);
-    ta = cta_sum(ta);
-    td = cta_sum(td);
-    tb = cta_sum(tb);
     // residual dq = pack(out) - q_in
     pack_moment(B, m, S.qsh_out, S.dp_out, S.qp_out, dq, tid, nthr);
-    __syncthreads();
-    double rr = 0.0;
-    for (int i = tid; i < dim; i += nthr) {
+    for (int i = tid; i < dim; i += nthr) {  // the elements this thread has packed
         dq[i] -= q_in[i];
-        rr += dq[i] * dq[i];
+        v[6] += dq[i] * dq[i];
     }
-    rr = cta_sum(rr);
+    cta_sums(v);
+    const double e = v[0] + S.ts[m], t2 = v[1], t3 = v[2], ta = v[3], td = v[4], tb = v[5], rr = v[6];
     __shared__ int s_done;
     if (tid == 0) {
         double res = sqrt(rr / dim);
@@ -504,49 +518,58 @@ __global__ void k_broyden(Batch B, State S, int hist_cap) {
         }
         int nh = itn;  // memory = max_iter >= iterations: the whole history
         double* dfi = df + (long long)it1 * dim;
-        double nr = 0.0;
-        for (int i = tid; i < dim; i += nthr) nr += dq[i] * dq[i];
-        nr = sqrt(cta_sum(nr));
+        double sums[2] = {};  // |dq|^2 and |dq - dqlast|^2
+        for (int i = tid; i < dim; i += nthr) {
+            double v = dq[i] - dqlast[i];
+            dfi[i] = v;
+            sums[0] += dq[i] * dq[i];
+            sums[1] += v * v;
+        }
+        cta_sums(sums);
+        const double nr = sqrt(sums[0]), dn = sums[1];
         const double OMEGA0 = 0.01, MINW = 1.0, MAXW = 100000.0, WFAC = 0.01;
         double om = nr > WFAC / MAXW ? WFAC / nr : MAXW;
         if (om < MINW) om = MINW;
         if (tid == 0) omega[it1] = om;
-        double dn = 0.0;
-        for (int i = tid; i < dim; i += nthr) {
-            double v = dq[i] - dqlast[i];
-            dfi[i] = v;
-            dn += v * v;
-        }
-        dn = cta_sum(dn);
         double inv = 1.0 / fmax(sqrt(dn), DBL_EPSILON);
         for (int i = tid; i < dim; i += nthr) dfi[i] *= inv;
-        __syncthreads();
         // a[it1][j] = df_it1 . df_j (j <= it1), c[j] = omega_j df_j . dq
         __shared__ double cvec[BROYDEN_MAX_HIST];
         __shared__ int s_piv;
-        for (int j = 0; j < nh; j++) {
-            double* dfj = df + (long long)j * dim;
-            double s1 = 0.0, s2 = 0.0;
+        for (int j0 = 0; j0 < nh; j0 += 8) {  // eight vectors per pass and set of barriers
+            double s12[16] = {};
             for (int i = tid; i < dim; i += nthr) {
-                s1 += dfi[i] * dfj[i];
-                s2 += dfj[i] * dq[i];
+                const double a = dfi[i], b = dq[i];
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (j0 + u < nh) {
+                        const double x = df[(long long)(j0 + u) * dim + i];
+                        s12[u] += a * x;
+                        s12[8 + u] += x * b;
+                    }
             }
-            s1 = cta_sum(s1);
-            s2 = cta_sum(s2);
-            if (tid == 0) {
-                amat[it1 * hist_cap + j] = s1;
-                amat[j * hist_cap + it1] = s1;
-                cvec[j] = s2;  // times omega below
-            }
+            cta_sums(s12);
+            if (tid == 0)
+                for (int u = 0; u < 8 && j0 + u < nh; u++) {
+                    amat[it1 * hist_cap + j0 + u] = s12[u];
+                    amat[(j0 + u) * hist_cap + it1] = s12[u];
+                    cvec[j0 + u] = s12[8 + u];  // times omega below
+                }
         }
         __syncthreads();
         // beta (kept in the tail of amat's slab) = omega_i omega_j a_ij + omega0^2 delta_ij
+        __shared__ double s_beta[BROYDEN_SMALL * BROYDEN_SMALL];
         double* bt = S.amat + (long long)B.nmol * hist_cap * hist_cap + (long long)m * hist_cap * hist_cap;
+        int ldb = hist_cap;
+        if (nh <= BROYDEN_SMALL) {
+            bt = s_beta;
+            ldb = BROYDEN_SMALL;
+        }
         for (int e = tid; e < nh * nh; e += nthr) {
             int i = e / nh, j = e % nh;
             double v = omega[i] * omega[j] * amat[i * hist_cap + j];
             if (i == j) v += OMEGA0 * OMEGA0;
-            bt[i * hist_cap + j] = v;
+            bt[i * ldb + j] = v;
         }
         __syncthreads();
         if (tid == 0) {
@@ -559,8 +582,8 @@ __global__ void k_broyden(Batch B, State S, int hist_cap) {
             if (tid == 0) {
                 int piv = col;
                 for (int i = col + 1; i < nh; i++)
-                    if (fabs(bt[i * hist_cap + col]) >= fabs(bt[piv * hist_cap + col])) piv = i;
-                if (bt[piv * hist_cap + col] == 0.0) s_ok = 0;
+                    if (fabs(bt[i * ldb + col]) >= fabs(bt[piv * ldb + col])) piv = i;
+                if (bt[piv * ldb + col] == 0.0) s_ok = 0;
                 s_piv = piv;
             }
             __syncthreads();
@@ -568,9 +591,9 @@ __global__ void k_broyden(Batch B, State S, int hist_cap) {
             int piv = s_piv;
             if (piv != col) {
                 for (int k = tid; k < nh; k += nthr) {
-                    double tmp = bt[col * hist_cap + k];
-                    bt[col * hist_cap + k] = bt[piv * hist_cap + k];
-                    bt[piv * hist_cap + k] = tmp;
+                    double tmp = bt[col * ldb + k];
+                    bt[col * ldb + k] = bt[piv * ldb + k];
+                    bt[piv * ldb + k] = tmp;
                 }
                 if (tid == 0) {
                     double tmp = cvec[col];
@@ -579,9 +602,9 @@ __global__ void k_broyden(Batch B, State S, int hist_cap) {
                 }
                 __syncthreads();
             }
-            const double* prow = bt + (long long)col * hist_cap;
+            const double* prow = bt + (long long)col * ldb;
             for (int row = col + 1 + tid; row < nh; row += nthr) {
-                double* rrow = bt + (long long)row * hist_cap;
+                double* rrow = bt + (long long)row * ldb;
                 double f = rrow[col] / prow[col];
                 if (f != 0.0) {
                     for (int k = col; k < nh; k++) rrow[k] -= f * prow[k];
@@ -593,8 +616,8 @@ __global__ void k_broyden(Batch B, State S, int hist_cap) {
         if (tid == 0 && s_ok)
             for (int col = nh - 1; col >= 0; col--) {
                 double s = cvec[col];
-                for (int k = col + 1; k < nh; k++) s -= bt[col * hist_cap + k] * cvec[k];
-                cvec[col] = s / bt[col * hist_cap + col];
+                for (int k = col + 1; k < nh; k++) s -= bt[col * ldb + k] * cvec[k];
+                cvec[col] = s / bt[col * ldb + col];
             }
         __syncthreads();
         if (!s_ok) {
