@@ -9,6 +9,7 @@ from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 SRC = HERE / "csrc" / "axtb_gpu.cu"
+TRD = HERE / "csrc" / "trd.cu"  # the tridiagonal reduction's kernels: their own unit, compiled beside the engine
 OUT = HERE / "libaxtb_gpu.so"
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
          "-shared"]
@@ -22,7 +23,7 @@ def nvcc() -> str:
 
 
 def sources():
-    return [SRC] + sorted((HERE / "csrc").glob("*.cuh")) + [HERE / "csrc" / "params" / "gfn2_tables.h"] + \
+    return [SRC, TRD] + sorted((HERE / "csrc").glob("*.cuh")) + [HERE / "csrc" / "trd_classes.h"] + [HERE / "csrc" / "params" / "gfn2_tables.h"] + \
         sorted((HERE.parent / "include").glob("*.h"))
 
 
@@ -30,8 +31,17 @@ def build(force: bool = False) -> Path:
     if not force and OUT.exists() and OUT.stat().st_mtime >= max(p.stat().st_mtime for p in sources()):
         return OUT
     tmp = OUT.with_suffix(".so.tmp")
-    cmd = [nvcc(), *FLAGS, "-o", str(tmp), str(SRC)]
-    subprocess.run(cmd, check=True)
+    objs = [OUT.parent / (p.stem + ".o") for p in (SRC, TRD)]
+    flags = [f for f in FLAGS if f != "-shared"]
+    jobs = [subprocess.Popen([nvcc(), *flags, "-c", "-o", str(o), str(p)]) for p, o in zip((SRC, TRD), objs)]
+    for job in jobs:
+        job.wait()
+    for job in jobs:
+        if job.returncode:
+            raise subprocess.CalledProcessError(job.returncode, job.args)
+    subprocess.run([nvcc(), *FLAGS, "-o", str(tmp), *map(str, objs)], check=True)
+    for o in objs:
+        o.unlink()
     tmp.replace(OUT)
     return OUT
 

@@ -30,7 +30,7 @@
 #include "k_solvation.cuh"
 #include "params/gfn2_tables.h"
 #include "team_kernel.cuh"
-#include "trd.cuh"
+#include "trd_classes.h"
 #include "stages.cuh"
 #include "stages_chol.cuh"
 #include "chase.cuh"

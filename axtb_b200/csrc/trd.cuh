@@ -24,29 +24,17 @@
 // runs over the thread's rows in order, then over the lanes by a butterfly, then (AW > 1) over the
 // row groups in order: its bits depend on n only, not on the number of CTAs.
 #pragma once
-#include <cfloat>
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
-#include "team_la.cuh"
+#include "common.cuh"
+#include "trd_classes.h"
 
 namespace axg {
+namespace cg = cooperative_groups;
 
-constexpr int TRD_THREADS = 256;
-constexpr int TRD_SMEM_MAX = 227 * 1024;
-
-// shared memory of one CTA (doubles): v (two buffers), w, reduction slots and barriers; cluster: the
-// pairs (row element, y entry) received from all CTAs (two buffers) and the CTA's own pairs; grid: the
-// row groups' partial y; then 32 rows of the register columns, and the other columns
-__host__ __device__ constexpr int trd_stride(int n) { return (n + 31) & ~31; }
-__host__ __device__ constexpr int trd_slots(int n, int G, int TC) { return ((n + G - 1) / G + TC - 1) / TC; }
-__host__ __device__ constexpr int trd_smem_cols(int n, int G, int TC, int CR) {
-    return trd_slots(n, G, TC) > CR ? (trd_slots(n, G, TC) - CR) * TC : 0;
-}
-__host__ __device__ constexpr int trd_ylen(int n, int G, int TC) { return trd_slots(n, G, TC) * TC; }
-__host__ __device__ constexpr long long trd_smem_doubles(int n, int G, int AW, int CR, bool grid) {
-    return (long long)trd_stride(n) * (grid ? 3 : 7) + 48 + (grid ? AW : 2) * trd_ylen(n, G, 8 / AW) +
-           32LL * CR * (8 / AW) + (grid ? trd_ylen(n, G, 8 / AW) : 0) + (long long)trd_smem_cols(n, G, 8 / AW, CR) * trd_stride(n);
-}
+extern __shared__ __align__(16) double s_trd[];
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank) {
@@ -166,7 +154,7 @@ __device__ __forceinline__ bool trd_mol(int rank, int G, int n, double* __restri
     const int rg = wid % AW, cg = wid / AW;
     const int ns = trd_stride(n), ylen = trd_ylen(n, G, TC);
     const int nslot = trd_slots(n, G, TC);
-    double* sv = s_work;              // two buffers
+    double* sv = s_trd;              // two buffers
     double* sw = sv + 2 * ns;
     double* sred = sw + ns;           // 2 x 8 partials, alpha; two barriers
     double* rcv = sred + 48;          // cluster: received pairs (two buffers of ns)
@@ -565,14 +553,9 @@ __device__ __forceinline__ bool trd_mol(int rank, int G, int n, double* __restri
     return ok;
 }
 
-// SM cycles of the reduction into the profiler's counters (the molecule's counter in units of the
-// team kernel's half-SM CTAs)
+// SM cycles of the reduction into the molecule's counter (in units of the team kernel's half-SM CTAs)
 __device__ __forceinline__ void trd_cycles(const State& S, int m, int rank, int G, long long t0) {
-    if (rank == 0 && threadIdx.x == 0) {
-        double c = 2.0 * G * (double)(clock64() - t0);
-        S.mol_cyc[m] += c;
-        atomicAdd(&g_team_cycles[1], (unsigned long long)c);
-    }
+    if (rank == 0 && threadIdx.x == 0) S.mol_cyc[m] += 2.0 * G * (double)(clock64() - t0);
 }
 
 // One cluster per molecule of `list` (one-CTA-team molecules of the batch), CTAs of a cluster by
@@ -602,39 +585,6 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_trd_grid(Batch B, State S, i
                                   S.tau + ao0, xpub, &S.status[m]))
         atomicOr(&S.status[m], ST_TIMEOUT);
     if (cycles) trd_cycles(S, m, (int)blockIdx.x, (int)gridDim.x, t0);
-}
-
-// ---- size classes: row slots per thread and register columns per warp (row group)
-struct TrdClass {
-    int rt, cr;
-    const void* fn;
-};
-// cluster path: rt = ceil(n / 32) exactly; rt x cr values of the matrix per thread leave the other
-// ~90 of 255 registers to the pass. For clusters of G CTAs whose warps have few columns (clusters that
-// grew) a class with all of them in registers and nothing unrolled for columns that are not there.
-inline const TrdClass* trd_class(int n, int G = 0) {
-#define TRD_C(RT, CR) {RT, CR, (const void*)k_trd<RT, CR>}
-    static const TrdClass c[] = {TRD_C(1, 4),  TRD_C(2, 8),  TRD_C(3, 12), TRD_C(4, 16), TRD_C(5, 13), TRD_C(6, 12), TRD_C(7, 10), TRD_C(8, 9),  TRD_C(9, 8),
-                                 TRD_C(10, 7), TRD_C(11, 7), TRD_C(12, 6), TRD_C(13, 6), TRD_C(14, 5), TRD_C(15, 5),
-                                 TRD_C(16, 5), TRD_C(17, 4), TRD_C(18, 4), TRD_C(19, 4), TRD_C(20, 4), TRD_C(21, 3),
-                                 TRD_C(22, 3), TRD_C(23, 3), TRD_C(24, 3)};
-    static const TrdClass f[] = {TRD_C(1, 4),  TRD_C(2, 4),  TRD_C(3, 4),  TRD_C(4, 4),  TRD_C(5, 4),  TRD_C(6, 4),  TRD_C(7, 4),  TRD_C(8, 4),  TRD_C(9, 4),
-                                 TRD_C(10, 4), TRD_C(11, 4), TRD_C(12, 4), TRD_C(13, 4), TRD_C(14, 4), TRD_C(15, 4),
-                                 TRD_C(16, 4), TRD_C(17, 5), TRD_C(18, 5), TRD_C(19, 5)};
-#undef TRD_C
-    const int rt = (n + 31) / 32;
-    if (rt < 1 || rt > 24) return nullptr;
-    return G > 0 && rt <= 19 && trd_slots(n, G, 8) <= f[rt - 1].cr ? f + (rt - 1) : c + (rt - 1);
-}
-constexpr int TRD_CLUSTER_MAX_NAO = 32 * 24;
-// whole grid: n <= 256 rt
-inline const TrdClass* trd_grid_class(int n) {
-#define TRD_C(RT, CR) {RT, CR, (const void*)k_trd_grid<RT, CR>}
-    static const TrdClass c[] = {TRD_C(4, 8), TRD_C(5, 9), TRD_C(6, 11), TRD_C(7, 11), TRD_C(8, 9), TRD_C(10, 9)};
-#undef TRD_C
-    for (const TrdClass& x : c)
-        if (n <= 256 * x.rt) return &x;
-    return nullptr;
 }
 
 }  // namespace axg
