@@ -318,6 +318,7 @@ size_t padded(size_t n) {
 
 // ------------------------------------------------------------------ the batch engine
 struct Moments;  // a molecule's SCC moments (capi.cuh)
+struct StageCounts;
 struct AxtbBatch {
     int device = 0;
     cudaStream_t st = nullptr;
@@ -348,7 +349,7 @@ struct AxtbBatch {
         int mol, smem;
     };
     axg::StagePlan Q{};      // the molecules whose eigen phase runs in stages (those of trd and trd_grid)
-    long long q_full = 0, q_low = 0, q_rt = 0, q_vec = 0, q_col = 0;  // its tasks
+    long long q_full = 0, q_low = 0, q_rt = 0, q_vec = 0, q_col = 0, q_full32 = 0, q_low32 = 0;  // its tasks
     bool q_wide = false, q_narrow = false;  // widths of the back-transformation's column blocks in use
     int q_nmax = 0, q_natmax = 0;
     int nteam_eigen = 0;     // the other molecules (team kernels)
@@ -364,6 +365,7 @@ struct AxtbBatch {
     vector<cudaEvent_t> side_ev;  // fork, then one join per side stream
     void launch_trd();
     void launch_stages();
+    StageCounts stage_counts() const;
     void launch_cholesky(int eeq);
     void plan_trd(int big_nao, int band_max, const vector<int>& nao, int nsm, vector<int>& kind);
     void place_trd(const vector<int>& kind, const vector<int>& nao, int nsm,
@@ -435,10 +437,19 @@ AxtbBatch::~AxtbBatch() {
 
 // ---- launches of the stages (stages.cuh, stages_chol.cuh, trd.cuh), shared by the batch engine and
 // the allocation-free entry point
-struct StageCounts {  // tasks; nmax: the largest matrix
+struct StageCounts {  // tasks; nmax: the largest matrix; full32 > 0: the products in tiles of 32
     int nmax;
-    long long full, low, rt, vec, col;
+    long long full, low, rt, vec, col, full32, low32;
 };
+// the products of a stage in tiles of 64, or of 32 where those of 64 would leave SMs without any
+template <int MODE, bool LOW>
+static void stage_tiles(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
+                        cudaStream_t st) {
+    using namespace axg;
+    if (c.full32 > 0)
+        k_st_tiles32<MODE><<<(unsigned)(LOW ? c.low32 : c.full32), 128, GSTAGES * G32_STAGE * 8, st>>>(B, S, Q);
+    else k_st_tiles<MODE><<<(unsigned)(LOW ? c.low : c.full), TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+}
 static void stage_attributes() {
     using namespace axg;
     const void* work[] = {(const void*)k_st_tiles<ST_X>, (const void*)k_st_tiles<ST_FP>, (const void*)k_st_tiles<ST_C>,
@@ -454,8 +465,8 @@ static void stage_attributes() {
 static void stage_transform(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                             cudaStream_t st) {
     using namespace axg;
-    k_st_tiles<ST_X><<<(unsigned)c.full, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
-    k_st_tiles<ST_FP><<<(unsigned)c.low, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+    stage_tiles<ST_X, false>(B, S, Q, c, st);
+    stage_tiles<ST_FP, true>(B, S, Q, c, st);
 }
 // count reductions of one class on clusters of G CTAs
 static void stage_reduce(const void* fn, int G, int count, int smem, const axg::Batch& B, const axg::State& S, const int* list,
@@ -489,8 +500,8 @@ static void stage_vectors(const axg::Batch& B, const axg::State& S, const axg::S
 static void stage_density(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                           cudaStream_t st) {
     using namespace axg;
-    k_st_tiles<ST_C><<<(unsigned)c.full, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
-    k_st_tiles<ST_P><<<(unsigned)c.low, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+    stage_tiles<ST_C, false>(B, S, Q, c, st);
+    stage_tiles<ST_P, true>(B, S, Q, c, st);
 }
 // factor and inverse factor of the overlap matrices, or of the EEQ matrices; nmax: the largest
 static void stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P, int nmax,
@@ -633,10 +644,12 @@ void AxtbBatch::launch_trd() {
     }
 }
 
+StageCounts AxtbBatch::stage_counts() const { return {q_nmax, q_full, q_low, q_rt, q_vec, q_col, q_full32, q_low32}; }
+
 // The staged molecules' eigen phase (stages.cuh), between its tridiagonal reductions
 void AxtbBatch::launch_stages() {
     using namespace axg;
-    const StageCounts cnt{q_nmax, q_full, q_low, q_rt, q_vec, q_col};
+    const StageCounts cnt = stage_counts();
     stage_transform(B, S, Q, cnt, st);
     launch_trd();
     // the reflectors' triangular factors beside the levels and vectors of the tridiagonal matrices
@@ -1007,7 +1020,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     addI(nmol);                                              // trd_kind
     addI(nmol);                                              // the stages' molecules, widths and tasks
     addI(nmol);
-    for (int c = 0; c < 5; c++) addL((size_t)nmol + 1);
+    for (int c = 0; c < 7; c++) addL((size_t)nmol + 1);
     for (int c = 0; c < 128; c++) addI(1);                   // k_trd lists: at most one per class and cluster size
     addI(nmol);
     addD(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()) + 1);
@@ -1257,7 +1270,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         // columns) when that fills the GPU and the molecule's rows fit, else 8
         long long wide = 0;
         for (int m : list) wide += (m_nao[m] / 2 + 23) / 24;
-        vector<long long> full{0}, low{0}, rts{0}, vec{0}, col{0};
+        vector<long long> full{0}, low{0}, rts{0}, vec{0}, col{0}, full32{0}, low32{0};
         for (int m : list) {
             long long n = m_nao[m], rt = (n + axg::GT - 1) / axg::GT;
             int w = wide >= nsm && axg::st_apply_doubles((int)n, 24) * 8 <= axg::TRD_SMEM_MAX ? 24 : 8;
@@ -1267,6 +1280,9 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
             q_natmax = std::max(q_natmax, mols[m].nat);
             full.push_back(full.back() + rt * rt);
             low.push_back(low.back() + rt * (rt + 1) / 2);
+            const long long r32 = (n + axg::G32 - 1) / axg::G32;
+            full32.push_back(full32.back() + r32 * r32);
+            low32.push_back(low32.back() + r32 * (r32 + 1) / 2);
             rts.push_back(rts.back() + rt);
             vec.push_back(vec.back() + (n + 31) / 32);
             col.push_back(col.back() + (n + w - 1) / w);
@@ -1282,6 +1298,12 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         Q.width = upI(width);
         Q.off_full = upL(full);
         Q.off_low = upL(low);
+        Q.off_full32 = upL(full32);
+        Q.off_low32 = upL(low32);
+        if (q_low < nsm && !b.split) {
+            q_full32 = full32.back();
+            q_low32 = low32.back();
+        }
         Q.off_rt = upL(rts);
         Q.off_vec = upL(vec);
         Q.off_col = upL(col);
@@ -1897,7 +1919,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
             if (nteam_eigen > 0) team_launch(PH_WDENS);
             if (Q.count > 0) {
                 k_st_scale<<<(unsigned)q_full, TEAM_THREADS, 0, st>>>(B, S, Q);
-                k_st_tiles<ST_W><<<(unsigned)q_low, TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+                stage_tiles<ST_W, true>(B, S, Q, stage_counts(), st);
                 launches++;
             }
         });
@@ -1977,7 +1999,7 @@ __global__ void k_density_setup(Batch B, State S, TeamPlan P, StagePlan Q, int n
     S.active[0] = 1;
     *const_cast<int*>(Q.mol) = 0;
     *const_cast<int*>(Q.width) = width;
-    const long long* off[] = {Q.off_full, Q.off_low, Q.off_rt, Q.off_vec, Q.off_col};
+    const long long* off[] = {Q.off_full, Q.off_low, Q.off_rt, Q.off_vec, Q.off_col, Q.off_full32, Q.off_low32};
     for (const long long* o : off) *const_cast<long long*>(o) = 0;
 }
 __global__ void k_density_status(State S, int* d_status) { *d_status = S.status[0]; }
@@ -2088,11 +2110,14 @@ extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_ove
         Q.off_rt = reinterpret_cast<const long long*>(par + 84);
         Q.off_vec = reinterpret_cast<const long long*>(par + 85);
         Q.off_col = reinterpret_cast<const long long*>(par + 86);
+        Q.off_full32 = reinterpret_cast<const long long*>(par + 89);
+        Q.off_low32 = reinterpret_cast<const long long*>(par + 90);
         S.active = reinterpret_cast<int*>(par + 87);
         S.mol_cyc = par + 88;
         k_density_setup<<<1, 1, 0, on>>>(B, S, P, Q, nao, nalpha, nbeta, 8);
         const long long rt = (nao + GT - 1) / GT;
-        const StageCounts c{nao, rt * rt, rt * (rt + 1) / 2, rt, (nao + 31) / 32, (nao + 7) / 8};
+        const long long r32 = (nao + G32 - 1) / G32;
+        const StageCounts c{nao, rt * rt, rt * (rt + 1) / 2, rt, (nao + 31) / 32, (nao + 7) / 8, r32 * r32, r32 * (r32 + 1) / 2};
         int G = 1;  // the cluster that holds the matrix, grown while each warp keeps a column
         while (trd_smem_doubles(nao, G, 1, trd_class(nao, G)->cr, false) * 8 > TRD_SMEM_MAX) G *= 2;
         while (G < 8 && 16 * G <= nao) G *= 2;

@@ -1,6 +1,7 @@
 // The eigen phase of the molecules whose tridiagonal reduction runs on chip (trd.cuh), one launch
 // per stage over all of them, each stage cut into the tasks that are independent in it:
-//   k_st_tiles   64 x 64 tiles of X = L^-1 F, F' = X L^-T, C = L^-T Z, P = (C f) C^T, W
+//   k_st_tiles   64 x 64 tiles of X = L^-1 F, F' = X L^-T, C = L^-T Z, P = (C f) C^T, W (k_st_tiles32:
+//                32 x 32 when those are few)
 //   k_st_bisect  32 orbital energies per CTA
 //   k_st_fermi   the filling, a CTA per molecule
 //   k_st_invit   one eigenvector of the tridiagonal matrix per thread, 32 per CTA
@@ -23,6 +24,8 @@ struct StagePlan {
     const int* mol;
     const long long* off_full;   // rt^2 tiles, rt = ceil(n / 64)
     const long long* off_low;    // rt (rt + 1) / 2 tiles on and below the diagonal
+    const long long* off_full32; // the same in tiles of 32
+    const long long* off_low32;
     const long long* off_rt;     // rt blocks of 64
     const long long* off_vec;    // ceil(n / 32) blocks of 32 levels or vectors
     const long long* off_col;    // column blocks of the back-transformation
@@ -99,6 +102,130 @@ __global__ void __launch_bounds__(TEAM_THREADS, 2) k_st_tiles(Batch B, State S, 
             if (r < n && r > c) out[c + (long long)r * n] = s_work[(e / GT) * (GT + 1) + e % GT];
         }
     }
+}
+
+// The same products in 32 x 32 tiles of four warps, for batches with fewer 64 x 64 tiles than the GPU
+// has SMs: a tile is bound by its SM's FP64 tensor rate (192 AOs: 18 us a stage in 9 tiles on 148
+// SMs, 9 in 36). Every element sums the same k-steps in the same order; FP64 only.
+constexpr int G32 = 32, G32_STAGE = 2 * GK * (G32 + 2);
+struct Tile32 {
+    const double *A, *B;
+    int lda, ldb;
+    bool ta, tb;
+    int M, N, k0, ke;
+};
+__device__ __forceinline__ void gemm_tile32(const Tile32& t, int row0, int col0, double (&acc)[2][2][2]) {
+    typedef double Stage[2][GK][G32 + 2];
+    Stage* stg = reinterpret_cast<Stage*>(s_work);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wm = warp & 1, wn = warp >> 1, lr = lane >> 2, lc = lane & 3;
+    const int nk = (t.ke - t.k0 + GK - 1) / GK;
+    auto issue = [&](int ks) {
+        if (ks < nk) {
+            Stage& S = stg[ks % GSTAGES];
+            const int kb = t.k0 + ks * GK;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                int e = tid + q * 128;
+                int mm = t.ta ? e / GK : e % G32, kk = t.ta ? e % GK : e / G32;
+                int gr = row0 + mm, gk = kb + kk;
+                bool ok = gr < t.M && gk < t.ke;
+                long long off = t.ta ? gk + (long long)gr * t.lda : gr + (long long)gk * t.lda;
+                cp_async8(&S[0][kk][mm], ok ? t.A + off : t.A, ok);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                int e = tid + q * 128;
+                int nn = t.tb ? e % G32 : e / GK, kk = t.tb ? e / G32 : e % GK;
+                int gc = col0 + nn, gk = kb + kk;
+                bool ok = gc < t.N && gk < t.ke;
+                long long off = t.tb ? gc + (long long)gk * t.ldb : gk + (long long)gc * t.ldb;
+                cp_async8(&S[1][kk][nn], ok ? t.B + off : t.B, ok);
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int ks = 0; ks < GSTAGES - 1; ks++) issue(ks);
+    for (int ks = 0; ks < nk; ks++) {
+        cp_async_wait<GSTAGES - 2>();
+        __syncthreads();
+        issue(ks + GSTAGES - 1);
+        Stage& S = stg[ks % GSTAGES];
+#pragma unroll
+        for (int kk = 0; kk < GK; kk += 4) {
+            double af[2], bf[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) af[i] = S[0][kk + lc][wm * 16 + i * 8 + lr];
+#pragma unroll
+            for (int j = 0; j < 2; j++) bf[j] = S[1][kk + lc][wn * 16 + j * 8 + lr];
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) dmma_8x8x4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(128) k_st_tiles32(Batch B, State S, StagePlan Q) {
+    constexpr bool LOW = MODE == ST_FP || MODE == ST_P || MODE == ST_W;
+    const long long* off = LOW ? Q.off_low32 : Q.off_full32;
+    const int i = stage_find(off, Q.count, blockIdx.x), m = Q.mol[i];
+    if (MODE == ST_W ? !S.conv[m] : !S.active[m]) return;
+    const int n = B.m_nao[m], rt = (n + G32 - 1) / G32, ao0 = B.m_ao0[m];
+    const long long mat = B.m_mat0[m];
+    int tile = (int)(blockIdx.x - off[i]), bi, bj;
+    if (LOW) {
+        bj = 0;
+        while (tile >= rt - bj) tile -= rt - bj, bj++;
+        bi = bj + tile;
+    } else {
+        bi = rt - 1 - tile % rt;
+        bj = tile / rt;
+    }
+    const int k = MODE >= ST_C ? S.kocc[m] : n, row0 = bi * G32, col0 = bj * G32;
+    if (MODE == ST_C && col0 >= k) return;
+    if (MODE == ST_X && tile == 0 && threadIdx.x == 0) S.mol_cyc[m] = 0.0;
+    const double* Li = S.Linv + mat;
+    double* out;
+    Tile32 t;
+    if (MODE == ST_X) {
+        t = {Li, S.F + mat, n, n, false, false, n, n, 0, min(n, row0 + G32)};
+        out = S.scr1 + mat;
+    } else if (MODE == ST_FP) {
+        t = {S.scr1 + mat, Li, n, n, false, true, n, n, 0, min(n, col0 + G32)};
+        out = S.Fp + mat;
+    } else if (MODE == ST_C) {
+        t = {Li, S.Z + mat, n, n, true, false, n, k, row0, n};
+        out = S.C + mat;
+    } else {
+        t = {S.scr1 + mat, S.C + mat, n, n, false, true, n, n, 0, k};
+        out = (MODE == ST_P ? S.P : S.W) + mat;
+    }
+    double acc[2][2][2];
+    gemm_tile32(t, row0, col0, acc);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+#pragma unroll
+    for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int y = 0; y < 2; y++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int r = row0 + (warp & 1) * 16 + x * 8 + lr, c = col0 + (warp >> 1) * 16 + y * 8 + lc * 2 + h;
+                if (r >= n || c >= t.N) continue;
+                const double v = acc[x][y][h];
+                if (MODE == ST_P || MODE == ST_W) {  // the lower triangle and its mirror image
+                    if (r < c) continue;
+                    out[c + (long long)r * n] = v;
+                }
+                out[r + (long long)c * n] = v;
+                if (MODE == ST_C) S.scr1[mat + r + (long long)c * n] = v * S.focc[ao0 + c];
+            }
 }
 
 // scr1 = C (f e), the left factor of W
@@ -332,8 +459,9 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_fermi(Batch B, State S, Sta
 // ---------------------------------------------------------------------------------- vectors
 // Inverse iteration as in team_invit (two solves from a hashed start; the vectors of a cluster, closer
 // than 1e-6 ||T||, made orthogonal after each), one thread per vector, 32 per CTA: part 0 factorises
-// and solves once, part 1 solves again, each followed by k_st_gs for the clusters (one thread took a
-// whole cluster before, and a launch was as long as its largest). The first forward substitution
+// and solves (twice for a vector outside the clusters), part 1 solves again for the clusters' vectors,
+// each followed by k_st_gs (one thread took a whole cluster before, and a launch was as long as its
+// largest). The first forward substitution
 // rides on the factorisation, the factors hold reciprocal pivots (one division per row instead of
 // three), norms are summed as the solution is made and applied by the next reader, and rows come
 // through a ring of asynchronous copies, 28 ahead. The vectors stay where they are made,
@@ -370,6 +498,9 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
     __syncwarp();
     const Clusters cl = warp_clusters(sd, se, n);
     if (q >= k) return;
+    // alone: no level close by, so nothing to be made orthogonal to, and part 0 takes both solves
+    const bool alone = !(q > 0 && w[q] - w[q - 1] <= cl.ctol) && !(q + 1 < k && w[q + 1] - w[q] <= cl.ctol);
+    if (part == 1 && alone) return;
     double* u0 = S.scr1 + mat + q;  // reciprocal pivots
     double* u1 = S.scr2 + mat + q;
     double* lm = S.scr3 + mat + q;
@@ -378,8 +509,113 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
     // the thread's own ring of rows on their way from L2 or HBM
     constexpr int GR = 4, NG = 8, R = GR * NG;
     double* ring = s_work + 2 * (n + 8) + threadIdx.x;
-    auto slot = [&](int step, int f) { return ring + ((step & (R - 1)) * 3 + f) * 32; };
-    double cur;
+    auto slot = [&](int step, int f) { return ring + ((step & (R - 1)) * 3 + f) * 32; };  // f beyond 2: later rows
+    double ss = 1.0;
+    // L with the row interchanges, the first solution (1 / its norm: nr) normalised on the way
+    auto forward = [&](double nr) {
+        const long long st = LD;
+        auto issue = [&](int g) {
+            const double *px = x + (g * GR + 1) * st, *pl = lm + g * GR * st;
+            if (g * GR + GR < n) {
+#pragma unroll
+                for (int u = 0; u < GR; u++, px += st, pl += st) {
+                    cp_async8(slot(g * GR, 3 * u), px, true);
+                    cp_async8(slot(g * GR, 3 * u + 1), pl, true);
+                }
+            } else {
+                for (int u = 0; g * GR + u + 1 < n; u++, px += st, pl += st) {
+                    cp_async8(slot(g * GR, 3 * u), px, true);
+                    cp_async8(slot(g * GR, 3 * u + 1), pl, true);
+                }
+            }
+            cp_async_commit();
+        };
+        double cur = x[0] * nr;
+        unsigned bits = 0;
+        for (int g = 0; g < NG - 1; g++) issue(g);
+        double* px = x;
+        for (int g = 0; g * GR + 1 < n; g++) {
+            cp_async_wait<NG - 2>();
+            if ((g * GR & 31) == 0) bits = swaps[(g * GR >> 5) * st];
+            double xv[GR], l[GR];
+#pragma unroll
+            for (int u = 0; u < GR; u++) xv[u] = *slot(g * GR, 3 * u), l[u] = *slot(g * GR, 3 * u + 1);
+            issue(g + NG - 1);
+#pragma unroll
+            for (int u = 0; u < GR; u++) {
+                if (g * GR + u + 1 < n) {
+                    const bool p = bits & 1;
+                    bits >>= 1;
+                    const double nxt = xv[u] * nr, top = p ? nxt : cur;
+                    *px = top;
+                    px += st;
+                    cur = (p ? cur : nxt) - l[u] * top;
+                }
+            }
+        }
+        cp_async_wait<0>();
+        x[(n - 1) * st] = cur;
+    };
+    // U with up to two superdiagonals (e_{i+1} after an interchange); the squared norm into ss
+    auto backward = [&]() {
+        const long long st = LD;
+        auto issue = [&](int g) {  // rows n - 1 - 4 g downwards
+            const long long o = (n - 1 - g * GR) * st;
+            const double *px = x + o, *p0 = u0 + o, *p1 = u1 + o;
+            const int cnt = min(GR, n - g * GR);
+            if (cnt == GR) {
+#pragma unroll
+                for (int u = 0; u < GR; u++, px -= st, p0 -= st, p1 -= st) {
+                    cp_async8(slot(g * GR, 3 * u), px, true);
+                    cp_async8(slot(g * GR, 3 * u + 1), p0, true);
+                    cp_async8(slot(g * GR, 3 * u + 2), p1, true);
+                }
+            } else {
+                for (int u = 0; u < cnt; u++, px -= st, p0 -= st, p1 -= st) {
+                    cp_async8(slot(g * GR, 3 * u), px, true);
+                    cp_async8(slot(g * GR, 3 * u + 1), p0, true);
+                    cp_async8(slot(g * GR, 3 * u + 2), p1, true);
+                }
+            }
+            cp_async_commit();
+        };
+        double xn1 = 0.0, xn2 = 0.0;
+        ss = 0.0;
+        for (int g = 0; g < NG - 1; g++) issue(g);
+        unsigned bits = swaps[((n - 1) >> 5) * st] << (31 - ((n - 1) & 31));
+        double* px = x + (n - 1) * st;
+        for (int g = 0; g * GR < n; g++) {
+            cp_async_wait<NG - 2>();
+            double xv[GR], f0[GR], f1[GR];
+#pragma unroll
+            for (int u = 0; u < GR; u++) {
+                xv[u] = *slot(g * GR, 3 * u);
+                f0[u] = *slot(g * GR, 3 * u + 1);
+                f1[u] = *slot(g * GR, 3 * u + 2);
+            }
+            issue(g + NG - 1);
+#pragma unroll
+            for (int u = 0; u < GR; u++) {
+                const int i = n - 1 - (g * GR + u);
+                if (i >= 0) {
+                    if ((i & 31) == 31) bits = swaps[(i >> 5) * st];
+                    const double c1 = i + 1 < n ? f1[u] : 0.0, c2 = i + 2 < n && (int)bits < 0 ? se[i + 1] : 0.0;
+                    bits <<= 1;
+                    double v = fma(-c1, xn1, fma(-c2, xn2, xv[u])) * f0[u];
+                    *px = v;
+                    px -= st;
+                    xn2 = xn1;
+                    xn1 = v;
+                    ss = fma(v, v, ss);
+                }
+            }
+        }
+        cp_async_wait<0>();
+        if (!(ss > 0.0) || !isfinite(ss)) {
+            atomicOr(&S.status[m], ST_INVIT);
+            ss = 1.0;
+        }
+    };
     if (part == 0) {
         // the shift: the level, kept apart from the cluster's earlier ones
         int q0 = q;
@@ -389,7 +625,7 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
         // LU with partial pivoting of T - lam I, the start vector eliminated along
         double ca = sd[0] - lam, cb = se[0];
         unsigned bits = 0;
-        cur = hash_uniform((unsigned)q, 0u);
+        double cur = hash_uniform((unsigned)q, 0u);
 #pragma unroll 4
         for (int i = 0; i + 1 < n; i++) {
             const double sub = se[i], a1 = sd[i + 1] - lam, b1 = se[i + 1];
@@ -414,88 +650,15 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
         }
         swaps[((n - 1) >> 5) * LD] = bits;
         u0[(n - 1) * LD] = 1.0 / (ca == 0.0 ? cl.pivmin : ca);
+        x[(n - 1) * LD] = cur;
+        backward();
+        if (alone) {
+            forward(1.0 / sqrt(ss));
+            backward();
+        }
     } else {
-        // forward: L with the row interchanges, the first solution normalised on the way
-        const double nr = stage_norms(P, m)[q];
-        auto issue = [&](int g) {
-#pragma unroll
-            for (int u = 0; u < GR; u++) {
-                const int i = g * GR + u;
-                if (i + 1 < n) {
-                    cp_async8(slot(i, 0), x + (i + 1) * LD, true);
-                    cp_async8(slot(i, 1), lm + i * LD, true);
-                }
-            }
-            cp_async_commit();
-        };
-        cur = x[0] * nr;
-        unsigned bits = 0;
-        for (int g = 0; g < NG - 1; g++) issue(g);
-        for (int g = 0; g * GR + 1 < n; g++) {
-            cp_async_wait<NG - 2>();
-            if ((g * GR & 31) == 0) bits = swaps[(g * GR >> 5) * LD];
-            double xv[GR], l[GR];
-#pragma unroll
-            for (int u = 0; u < GR; u++) xv[u] = *slot(g * GR + u, 0), l[u] = *slot(g * GR + u, 1);
-            issue(g + NG - 1);
-#pragma unroll
-            for (int u = 0; u < GR; u++) {
-                const int i = g * GR + u;
-                if (i + 1 < n) {
-                    const bool p = bits >> (i & 31) & 1;
-                    const double nxt = xv[u] * nr, top = p ? nxt : cur;
-                    x[i * LD] = top;
-                    cur = (p ? cur : nxt) - l[u] * top;
-                }
-            }
-        }
-        cp_async_wait<0>();
-    }
-    x[(n - 1) * LD] = cur;
-    // backward: U with up to two superdiagonals (e_{i+1} after an interchange)
-    double xn1 = 0.0, xn2 = 0.0, ss = 0.0;
-    auto issue = [&](int g) {
-#pragma unroll
-        for (int u = 0; u < GR; u++) {
-            const int st = g * GR + u, i = n - 1 - st;
-            if (i >= 0) {
-                cp_async8(slot(st, 0), x + i * LD, true);
-                cp_async8(slot(st, 1), u0 + i * LD, true);
-                cp_async8(slot(st, 2), u1 + i * LD, true);
-            }
-        }
-        cp_async_commit();
-    };
-    for (int g = 0; g < NG - 1; g++) issue(g);
-    unsigned bits = swaps[((n - 1) >> 5) * LD];
-    for (int g = 0; g * GR < n; g++) {
-        cp_async_wait<NG - 2>();
-        double xv[GR], f0[GR], f1[GR];
-#pragma unroll
-        for (int u = 0; u < GR; u++) {
-            xv[u] = *slot(g * GR + u, 0);
-            f0[u] = *slot(g * GR + u, 1);
-            f1[u] = *slot(g * GR + u, 2);
-        }
-        issue(g + NG - 1);
-#pragma unroll
-        for (int u = 0; u < GR; u++) {
-            const int i = n - 1 - (g * GR + u);
-            if (i >= 0) {
-                if ((i & 31) == 31) bits = swaps[(i >> 5) * LD];
-                const double c1 = i + 1 < n ? f1[u] : 0.0, c2 = i + 2 < n && (bits >> (i & 31) & 1) ? se[i + 1] : 0.0;
-                double v = fma(-c1, xn1, fma(-c2, xn2, xv[u])) * f0[u];
-                x[i * LD] = v;
-                xn2 = xn1;
-                xn1 = v;
-                ss = fma(v, v, ss);
-            }
-        }
-    }
-    cp_async_wait<0>();
-    if (!(ss > 0.0) || !isfinite(ss)) {
-        atomicOr(&S.status[m], ST_INVIT);
-        ss = 1.0;
+        forward(stage_norms(P, m)[q]);
+        backward();
     }
     stage_norms(P, m)[q] = 1.0 / sqrt(ss);  // applied by whoever reads the vector next
 }
