@@ -437,25 +437,27 @@ AxtbBatch::~AxtbBatch() {
 
 // ---- launches of the stages (stages.cuh, stages_chol.cuh, trd.cuh), shared by the batch engine and
 // the allocation-free entry point
-struct StageCounts {  // tasks; nmax: the largest matrix; full32 > 0: the products in tiles of 32
+struct StageCounts {  // tasks; nmax: the largest matrix
     int nmax;
     long long full, low, rt, vec, col, full32, low32;
 };
-// the products of a stage in tiles of 64, or of 32 where those of 64 would leave SMs without any
+// the products of a stage; in split precision X, F' and W keep the 64 x 64 tiles that have it
 template <int MODE, bool LOW>
 static void stage_tiles(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                         cudaStream_t st) {
     using namespace axg;
-    if (c.full32 > 0)
-        k_st_tiles32<MODE><<<(unsigned)(LOW ? c.low32 : c.full32), 128, GSTAGES * G32_STAGE * 8, st>>>(B, S, Q);
-    else k_st_tiles<MODE><<<(unsigned)(LOW ? c.low : c.full), TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+    if constexpr (MODE != ST_C && MODE != ST_P)
+        if (B.split) {
+            k_st_tiles<MODE><<<(unsigned)(LOW ? c.low : c.full), TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+            return;
+        }
+    k_st_tiles32<MODE><<<(unsigned)(LOW ? c.low32 : c.full32), 128, GSTAGES * G32_STAGE * 8, st>>>(B, S, Q);
 }
 static void stage_attributes() {
     using namespace axg;
-    const void* work[] = {(const void*)k_st_tiles<ST_X>, (const void*)k_st_tiles<ST_FP>, (const void*)k_st_tiles<ST_C>,
-                          (const void*)k_st_tiles<ST_P>, (const void*)k_st_tiles<ST_W>,  (const void*)k_st_tfac,
-                          (const void*)k_st_bisect,      (const void*)k_st_fermi,        (const void*)k_ch_init,
-                          (const void*)k_ch_panel,       (const void*)k_ch_trail};
+    const void* work[] = {(const void*)k_st_tiles<ST_X>, (const void*)k_st_tiles<ST_FP>, (const void*)k_st_tiles<ST_W>,
+                          (const void*)k_st_tfac,        (const void*)k_st_bisect,       (const void*)k_st_fermi,
+                          (const void*)k_ch_init,        (const void*)k_ch_panel,        (const void*)k_ch_trail};
     for (const void* f : work) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WORK_BYTES));
     const void* all[] = {(const void*)k_st_apply<8, 16>, (const void*)k_st_apply<24, 8>, (const void*)k_st_apply<24, 16>,
                          (const void*)k_st_invit};
@@ -1300,10 +1302,8 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         Q.off_low = upL(low);
         Q.off_full32 = upL(full32);
         Q.off_low32 = upL(low32);
-        if (q_low < nsm && !b.split) {
-            q_full32 = full32.back();
-            q_low32 = low32.back();
-        }
+        q_full32 = full32.back();
+        q_low32 = low32.back();
         Q.off_rt = upL(rts);
         Q.off_vec = upL(vec);
         Q.off_col = upL(col);

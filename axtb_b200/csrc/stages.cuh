@@ -1,7 +1,7 @@
 // The eigen phase of the molecules whose tridiagonal reduction runs on chip (trd.cuh), one launch
 // per stage over all of them, each stage cut into the tasks that are independent in it:
-//   k_st_tiles   64 x 64 tiles of X = L^-1 F, F' = X L^-T, C = L^-T Z, P = (C f) C^T, W (k_st_tiles32:
-//                32 x 32 when those are few)
+//   k_st_tiles32 32 x 32 tiles of X = L^-1 F, F' = X L^-T, C = L^-T Z, P = (C f) C^T, W
+//                (k_st_tiles: 64 x 64, for split precision)
 //   k_st_bisect  32 orbital energies per CTA
 //   k_st_fermi   the filling, a CTA per molecule
 //   k_st_invit   one eigenvector of the tridiagonal matrix per thread, 32 per CTA
@@ -48,16 +48,16 @@ __device__ __forceinline__ int stage_find(const long long* off, int count, long 
 // ---------------------------------------------------------------------------------- tiles
 enum { ST_X = 0, ST_FP = 1, ST_C = 2, ST_P = 3, ST_W = 4 };
 
-// One 64 x 64 tile of a stage's product per CTA (the team GEMM on a team of as many CTAs as tiles:
-// the same k-steps in the same order). The tile of C also leaves C f (C f e for W) in scr1, that of
-// P and W its mirror image above the diagonal (through shared memory, both stores coalesced).
+// One 64 x 64 tile of X, F' or W in split precision per CTA (the team GEMM on a team of as many CTAs
+// as tiles: the same k-steps in the same order); W also gets its mirror image above the diagonal
+// (through shared memory, both stores coalesced).
 template <int MODE>
 __global__ void __launch_bounds__(TEAM_THREADS, 2) k_st_tiles(Batch B, State S, StagePlan Q) {
-    constexpr bool LOW = MODE == ST_FP || MODE == ST_P || MODE == ST_W;
+    constexpr bool LOW = MODE != ST_X;
     const long long* off = LOW ? Q.off_low : Q.off_full;
     const int i = stage_find(off, Q.count, blockIdx.x), m = Q.mol[i];
     if (MODE == ST_W ? !S.conv[m] : !S.active[m]) return;
-    const int n = B.m_nao[m], rt = (n + GT - 1) / GT, ao0 = B.m_ao0[m];
+    const int n = B.m_nao[m], rt = (n + GT - 1) / GT;
     const long long mat = B.m_mat0[m];
     int tile = (int)(blockIdx.x - off[i]), bi, bj;
     if (LOW) {  // column by column from the diagonal down
@@ -68,30 +68,18 @@ __global__ void __launch_bounds__(TEAM_THREADS, 2) k_st_tiles(Batch B, State S, 
         bi = rt - 1 - tile % rt;  // the rows with the longest sums first
         bj = tile / rt;
     }
-    const int k = MODE >= ST_C ? S.kocc[m] : n;
-    if (MODE == ST_C && bj * GT >= k) return;
-    const int tn = MODE == ST_C ? (k + GT - 1) / GT : rt;
-    const Team t{bi + bj * rt, rt * tn, false};
+    const Team t{bi + bj * rt, rt * rt, false};
     const double* Li = S.Linv + mat;
-    const int sp = B.split ? GEMM_SPLIT : 0;
     if (MODE == ST_X && t.rank == 0 && threadIdx.x == 0) S.mol_cyc[m] = 0.0;  // the profiler's, summed by k_trd
-    double* out;
     if (MODE == ST_X) {
-        team_gemm(t, false, false, n, n, n, 1.0, Li, n, S.F + mat, n, 0.0, S.scr1 + mat, n, GEMM_A_LOWER | sp);
+        team_gemm(t, false, false, n, n, n, 1.0, Li, n, S.F + mat, n, 0.0, S.scr1 + mat, n, GEMM_A_LOWER | GEMM_SPLIT);
     } else if (MODE == ST_FP) {
         team_gemm(t, false, true, n, n, n, 1.0, S.scr1 + mat, n, Li, n, 0.0, S.Fp + mat, n,
-                  GEMM_B_UPPER | GEMM_LOWER_TILES | sp);
-    } else if (MODE == ST_C) {
-        out = S.C + mat;
-        team_gemm(t, true, false, n, k, n, 1.0, Li, n, S.Z + mat, n, 0.0, out, n, GEMM_A_UPPER);
-        for (int e = threadIdx.x; e < GT * GT; e += TEAM_THREADS) {
-            int r = bi * GT + e % GT, c = bj * GT + e / GT;
-            if (r < n && c < k) S.scr1[mat + r + (long long)c * n] = out[r + (long long)c * n] * S.focc[ao0 + c];
-        }
+                  GEMM_B_UPPER | GEMM_LOWER_TILES | GEMM_SPLIT);
     } else {
-        out = (MODE == ST_P ? S.P : S.W) + mat;
-        team_gemm(t, false, true, n, n, k, 1.0, S.scr1 + mat, n, S.C + mat, n, 0.0, out, n,
-                  GEMM_LOWER_TILES | (MODE == ST_W ? sp : 0));
+        double* out = S.W + mat;
+        team_gemm(t, false, true, n, n, S.kocc[m], 1.0, S.scr1 + mat, n, S.C + mat, n, 0.0, out, n,
+                  GEMM_LOWER_TILES | GEMM_SPLIT);
         for (int e = threadIdx.x; e < GT * GT; e += TEAM_THREADS) {
             int r = bi * GT + e % GT, c = bj * GT + e / GT;
             s_work[(e % GT) * (GT + 1) + e / GT] = r < n && c < n ? out[r + (long long)c * n] : 0.0;
@@ -104,9 +92,11 @@ __global__ void __launch_bounds__(TEAM_THREADS, 2) k_st_tiles(Batch B, State S, 
     }
 }
 
-// The same products in 32 x 32 tiles of four warps, for batches with fewer 64 x 64 tiles than the GPU
-// has SMs: a tile is bound by its SM's FP64 tensor rate (192 AOs: 18 us a stage in 9 tiles on 148
-// SMs, 9 in 36). Every element sums the same k-steps in the same order; FP64 only.
+// The products in FP64, 32 x 32 tiles of four warps. Tiles of 64 (eight warps, two CTAs per SM) are
+// bound by their SM's FP64 tensor rate where there are few (192 AOs: 18 us a stage in 9 tiles on 148
+// SMs, 8 in 36 of 32; 600 AOs: 48 and 26) and have fewer warps in flight where there are many (the
+// mixed batch of 1024: 7.2 ms for the four products, 6.2 in tiles of 32). The sums run over the same
+// k-steps in the same order as the team GEMM's.
 constexpr int G32 = 32, G32_STAGE = 2 * GK * (G32 + 2);
 struct Tile32 {
     const double *A, *B;
@@ -119,28 +109,31 @@ __device__ __forceinline__ void gemm_tile32(const Tile32& t, int row0, int col0,
     Stage* stg = reinterpret_cast<Stage*>(s_work);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wm = warp & 1, wn = warp >> 1, lr = lane >> 2, lc = lane & 3;
     const int nk = (t.ke - t.k0 + GK - 1) / GK;
+    // this thread's four elements of each operand's k-step: consecutive threads along the contiguous
+    // dimension, (row, k) = (am, ak) + q (ta ? (8, 0) : (0, 4)); zero outside the operands
+    const int am = t.ta ? tid >> 4 : lane, ak = t.ta ? tid & 15 : warp, bn = t.tb ? lane : tid >> 4, bk = t.tb ? warp : tid & 15;
+    const double* pa = t.A + (t.ta ? t.k0 + ak + (long long)(row0 + am) * t.lda : row0 + am + (long long)(t.k0 + ak) * t.lda);
+    const double* pb = t.B + (t.tb ? col0 + bn + (long long)(t.k0 + bk) * t.ldb : t.k0 + bk + (long long)(col0 + bn) * t.ldb);
+    const long long qa = (t.ta ? 8LL : 4LL) * t.lda, qb = (t.tb ? 4LL : 8LL) * t.ldb;
+    const long long sa = t.ta ? GK : (long long)GK * t.lda, sb = t.tb ? (long long)GK * t.ldb : GK;
     auto issue = [&](int ks) {
         if (ks < nk) {
             Stage& S = stg[ks % GSTAGES];
-            const int kb = t.k0 + ks * GK;
+            const int left = t.ke - t.k0 - ks * GK;  // k's left from this step on
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                int e = tid + q * 128;
-                int mm = t.ta ? e / GK : e % G32, kk = t.ta ? e % GK : e / G32;
-                int gr = row0 + mm, gk = kb + kk;
-                bool ok = gr < t.M && gk < t.ke;
-                long long off = t.ta ? gk + (long long)gr * t.lda : gr + (long long)gk * t.lda;
-                cp_async8(&S[0][kk][mm], ok ? t.A + off : t.A, ok);
+                const int mm = t.ta ? am + 8 * q : am, kk = t.ta ? ak : ak + 4 * q;
+                const bool ok = row0 + mm < t.M && kk < left;
+                cp_async8(&S[0][kk][mm], ok ? pa + q * qa : t.A, ok);
             }
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                int e = tid + q * 128;
-                int nn = t.tb ? e % G32 : e / GK, kk = t.tb ? e / G32 : e % GK;
-                int gc = col0 + nn, gk = kb + kk;
-                bool ok = gc < t.N && gk < t.ke;
-                long long off = t.tb ? gc + (long long)gk * t.ldb : gk + (long long)gc * t.ldb;
-                cp_async8(&S[1][kk][nn], ok ? t.B + off : t.B, ok);
+                const int nn = t.tb ? bn : bn + 8 * q, kk = t.tb ? bk + 4 * q : bk;
+                const bool ok = col0 + nn < t.N && kk < left;
+                cp_async8(&S[1][kk][nn], ok ? pb + q * qb : t.B, ok);
             }
+            pa += sa;
+            pb += sb;
         }
         cp_async_commit();
     };
