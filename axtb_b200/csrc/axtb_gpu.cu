@@ -1059,9 +1059,9 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     addD((size_t)nwk);
     addL(nmol * 5);
     addD((size_t)nsqT * 2);
-    if (o.solv >= 0) {  // solvation: 9 per-atom parameter arrays, 7 per-atom state arrays, lists
+    if (o.solv >= 0) {  // solvation: 9 per-atom parameter arrays, 8 per-atom state arrays, lists
         addD((size_t)natT * 9 + nmol);
-        addD((size_t)natT * 10 + nmol * 2);
+        addD((size_t)natT * (10 + axg::SOLV_POINTS) + nmol * 2);
         addI((size_t)natT * axg::SOLV_MAXNB + natT);
     }
     bytes += 1 << 20;
@@ -1252,7 +1252,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         b.sv_gam = upD(gam);
         b.sv_hbmag = upD(hbmag);
         b.sv_srcut = upD(srcut);
-        CK(cudaMemcpyToSymbolAsync(axg::c_lebedev, LEBEDEV_230, sizeof(LEBEDEV_230), 0, cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyToSymbolAsync(axg::d_lebedev, LEBEDEV_230, sizeof(LEBEDEV_230), 0, cudaMemcpyHostToDevice, st));
     }
     b.damping = o.damping;
     b.econv = 1e-6 * o.acc;
@@ -1462,6 +1462,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         s.sv_adet = ar.take<double>(nmol);
         s.sv_eatom = ar.take<double>(natT);
         s.sv_emol = ar.take<double>(nmol);
+        s.sv_point = ar.take<double>((size_t)natT * axg::SOLV_POINTS);
         s.sv_nb = ar.take<int>((size_t)natT * axg::SOLV_MAXNB);
         s.sv_nbn = ar.take<int>(natT);
     }
