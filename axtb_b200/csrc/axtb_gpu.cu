@@ -386,6 +386,7 @@ struct AxtbBatch {
     vector<HostMol> mols;
     int nmol = 0, natT = 0, nshT = 0, naoT = 0;
     long long nnT = 0, npairT = 0, npdT = 0, nvecT = 0, nsqT = 0, ntiles = 0, nwk = 0, nhist = 0, ngamT = 0;
+    int nsh_max = 1;  // most shells of an atom of the batch
     int hist_cap = 0, nsp = 0;
     int mixer_kind = 0;      // the mixer plan of the run: 0 auto, 1 Broyden, 2 DIIS
     bool restart = false;    // molecules start from their previous converged moments
@@ -864,6 +865,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
                 a_mol[ia] = m;
                 a_sh0[ia] = is;
                 a_nsh[ia] = NSHELL[z - 1];
+                nsh_max = std::max(nsh_max, (int)NSHELL[z - 1]);
                 a_ao0[ia] = io;
                 a_sp[ia] = sp;
                 a_rcov[ia] = cv.cn_rcov(z);
@@ -1831,7 +1833,15 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         CK(cudaMemsetAsync(d_eatm, 0, sizeof(double) * nmol, st));
     }
     // integrals
-    LAUNCH("integrals", 0, mat_bytes(all, 11.0), k_integrals<<<blocks_for(npdT, 128), 128, 0, st>>>(B, S, d_pd0, npdT));
+    // a thread per shell pair while the atom pairs are at most 256 a multiprocessor (there the two are
+    // even: 0.33 ms for 300 molecules of 1 to 20 atoms); with more the GPU is full either way and the
+    // short threads cost more (1024 molecules: 20.6 ms with a thread per atom pair, 22.8 without)
+    const bool by_shells = npdT <= 128LL * grid;
+    LAUNCH("integrals", 0, mat_bytes(all, 11.0), {
+        if (by_shells)
+            k_integrals<true><<<blocks_for(npdT, 128) * nsh_max * nsh_max, 128, 0, st>>>(B, S, d_pd0, npdT, nsh_max);
+        else k_integrals<false><<<blocks_for(npdT, 128), 128, 0, st>>>(B, S, d_pd0, npdT, nsh_max);
+    });
     if (B.solv) {  // solvation: Born radii, SASA neighbours and surfaces, ALPB shape descriptor
         unsigned wb = blocks_for((long long)natT * 32, T);
         LAUNCH("solv_born", 0, 0, k_solv_born<<<wb, T, 0, st>>>(B, S));

@@ -236,15 +236,57 @@ __device__ __forceinline__ void unpack_pair(long long p, int& i, int& j) {  // p
     i = i + 1;
 }
 
+// S, H0, D, Q of the shell pair (si on atom ia, sj on atom ja) into the matrices
+__device__ __forceinline__ void shell_pair_integrals(const Batch& B, const State& S, const Shl& ci, const Shl& cj, int si,
+                                                     int sj, int ia, int ja, const double vec[3], bool onsite, double rr,
+                                                     int n, int ao0, long long mat, long long nn) {
+    double s[25], d[75], q[150];
+    multipole_block(cj, ci, vec, B.intcut, s, d, q);
+    double hij;
+    if (onsite) hij = 0.5 * (S.se[si] + S.se[sj]);
+    else {
+        double shp = (1.0 + B.s_shpoly[si] * rr) * (1.0 + B.s_shpoly[sj] * rr);
+        hij = 0.5 * (S.se[si] + S.se[sj]) * hscale(B, sj, ja, si, ia) * shp;
+    }
+    int nsj = nsph(cj.l);
+    for (int im = 0; im < nsph(ci.l); im++)
+        for (int jm = 0; jm < nsj; jm++) {
+            int k = jm + nsj * im;
+            int mu = B.s_ao0[sj] + jm - ao0, nu = B.s_ao0[si] + im - ao0;
+            long long e1 = mat + mu + (long long)nu * n;
+            S.S[e1] = s[k];
+            S.H0[e1] = s[k] * hij;
+            for (int x = 0; x < 3; x++) S.D[x * nn + e1] = d[3 * k + x];
+            for (int x = 0; x < 6; x++) S.Q[x * nn + e1] = q[6 * k + x];
+            if (!onsite) {
+                double dj[3], qj[6];
+                shift_bra(vec, s[k], &d[3 * k], &q[6 * k], dj, qj);
+                long long e2 = mat + nu + (long long)mu * n;
+                S.S[e2] = s[k];
+                S.H0[e2] = s[k] * hij;
+                for (int x = 0; x < 3; x++) S.D[x * nn + e2] = dj[x];
+                for (int x = 0; x < 6; x++) S.Q[x * nn + e2] = qj[x];
+            }
+        }
+}
+
 // S, H0, D, Q of every atom pair (i >= j) of every molecule; m_pd0 = offsets of the pairs with
-// diagonal (sum of nat(nat+1)/2)
-__global__ void k_integrals(Batch B, State S, const long long* m_pd0, long long npd) {
-    long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// diagonal (sum of nat(nat+1)/2). SHELLS false: a thread per atom pair. SHELLS true: a thread per shell
+// pair, the blocks of the nsh_max^2 shell pairs of the same 128 atom pairs one after the other (shells
+// that an atom does not have return at once). Bound by the chain of a shell pair's primitives with
+// its tables in local memory: up to nine such chains one after the other in the first form, beside one
+// another in the second: one water 134 -> 66 us, 25 carbons 170 -> 88 us, 32 waters 160 -> 90 us
+template <bool SHELLS>
+__global__ void k_integrals(Batch B, State S, const long long* m_pd0, long long npd, int nsh_max) {
+    const int parts = SHELLS ? nsh_max * nsh_max : 1, slot = blockIdx.x % parts;
+    long long g = (long long)(blockIdx.x / parts) * blockDim.x + threadIdx.x;
     if (g >= npd) return;
     int m = find_mol(m_pd0, B.nmol, g);
     int li, lj;
     unpack_pair_diag(g - m_pd0[m], li, lj);
     int ia = B.m_at0[m] + li, ja = B.m_at0[m] + lj;
+    const int slot_i = slot / nsh_max, slot_j = slot - slot_i * nsh_max;
+    if (SHELLS && (slot_i >= B.a_nsh[ia] || slot_j >= B.a_nsh[ja])) return;
     int n = B.m_nao[m], ao0 = B.m_ao0[m];
     long long mat = B.m_mat0[m], nn = B.nnT;
     double vec[3];
@@ -254,40 +296,21 @@ __global__ void k_integrals(Batch B, State S, const long long* m_pd0, long long 
     // atom pairs beyond the conventions' distance cutoff (tblite) or screened by their exponents
     if (!onsite && (r2 > B.m_paircut2[m] || pair_screened(B.a_amin[ia], B.a_amin[ja], r2, B.intcut))) return;
     double rr = onsite ? 0.0 : sqrt(sqrt(r2) / (B.a_rad[ja] + B.a_rad[ia]));
-    double s[25], d[75], q[150];
     Shl ci, cj;
-    for (int si = B.a_sh0[ia]; si < B.a_sh0[ia] + B.a_nsh[ia]; si++) {
+    if constexpr (SHELLS) {
+        const int si = B.a_sh0[ia] + slot_i, sj = B.a_sh0[ja] + slot_j;
+        if (!onsite && pair_screened(B.s_amin[si], B.s_amin[sj], r2, B.intcut)) return;
         load_shell(B, si, ci);
-        for (int sj = B.a_sh0[ja]; sj < B.a_sh0[ja] + B.a_nsh[ja]; sj++) {
-            if (!onsite && pair_screened(B.s_amin[si], B.s_amin[sj], r2, B.intcut)) continue;
-            load_shell(B, sj, cj);
-            multipole_block(cj, ci, vec, B.intcut, s, d, q);
-            double hij;
-            if (onsite) hij = 0.5 * (S.se[si] + S.se[sj]);
-            else {
-                double shp = (1.0 + B.s_shpoly[si] * rr) * (1.0 + B.s_shpoly[sj] * rr);
-                hij = 0.5 * (S.se[si] + S.se[sj]) * hscale(B, sj, ja, si, ia) * shp;
+        load_shell(B, sj, cj);
+        shell_pair_integrals(B, S, ci, cj, si, sj, ia, ja, vec, onsite, rr, n, ao0, mat, nn);
+    } else {
+        for (int si = B.a_sh0[ia]; si < B.a_sh0[ia] + B.a_nsh[ia]; si++) {
+            load_shell(B, si, ci);
+            for (int sj = B.a_sh0[ja]; sj < B.a_sh0[ja] + B.a_nsh[ja]; sj++) {
+                if (!onsite && pair_screened(B.s_amin[si], B.s_amin[sj], r2, B.intcut)) continue;
+                load_shell(B, sj, cj);
+                shell_pair_integrals(B, S, ci, cj, si, sj, ia, ja, vec, onsite, rr, n, ao0, mat, nn);
             }
-            int nsj = nsph(cj.l);
-            for (int im = 0; im < nsph(ci.l); im++)
-                for (int jm = 0; jm < nsj; jm++) {
-                    int k = jm + nsj * im;
-                    int mu = B.s_ao0[sj] + jm - ao0, nu = B.s_ao0[si] + im - ao0;
-                    long long e1 = mat + mu + (long long)nu * n;
-                    S.S[e1] = s[k];
-                    S.H0[e1] = s[k] * hij;
-                    for (int x = 0; x < 3; x++) S.D[x * nn + e1] = d[3 * k + x];
-                    for (int x = 0; x < 6; x++) S.Q[x * nn + e1] = q[6 * k + x];
-                    if (!onsite) {
-                        double dj[3], qj[6];
-                        shift_bra(vec, s[k], &d[3 * k], &q[6 * k], dj, qj);
-                        long long e2 = mat + nu + (long long)mu * n;
-                        S.S[e2] = s[k];
-                        S.H0[e2] = s[k] * hij;
-                        for (int x = 0; x < 3; x++) S.D[x * nn + e2] = dj[x];
-                        for (int x = 0; x < 6; x++) S.Q[x * nn + e2] = qj[x];
-                    }
-                }
         }
     }
 }
