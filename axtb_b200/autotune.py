@@ -2,15 +2,13 @@
 on the whole GPU.
 
 The engine's eigen phase has two schedule choices, both exact (the results agree to
-round-off): the tridiagonal reduction of a one-CTA molecule (two-stage: band reduction on
-GEMMs, then bulge chasing; or one-stage Householder with the trailing matrix streamed per
-column), chosen by the size ``band_max_nao`` below which the two-stage one is used (from 34 AOs:
-a smaller matrix already is a band, and keeps the one-stage reduction; measured on
-B200: it wins only for small molecules, where the one-stage reduction's per-column chain is
-short of work, not for large ones, where its bulge chasing waits on one global-memory round per
-block); and the size
-``grid_min_nao`` from which a molecule's dense algebra runs on the whole cooperative grid
-instead of one CTA. The best crossovers depend on the GPU and the batch, so they are measured:
+round-off): the tridiagonal reduction (two-stage: band reduction on GEMMs, then bulge chasing,
+one CTA per molecule; or one-stage Householder with the matrix in the registers and shared memory
+of a cluster), chosen by the size ``band_max_nao`` below which the two-stage one is used (from 34
+AOs, and only when set above 64; on B200 the reduction on chip is faster at every size that it
+holds, so the default is never to use the two-stage one); and the size
+``grid_min_nao`` from which a molecule's reduction runs on the whole cooperative grid
+instead of a cluster. The best crossovers depend on the GPU and the batch, so they are measured:
 
 * ``band_max_nao``: one profiled run of a sample batch with each reduction; the engine's
   per-molecule cycle counters of the eigen phase (the on-chip bulge chasing counted in units of

@@ -973,7 +973,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
             sp_rr[a * nsp + b] = v;
             sp_r0[a * nsp + b] = 0.52 * std::sqrt(v) + 5.0;
         }
-    // one-CTA molecules of 34 AOs up to below band_max_nao reduce to tridiagonal form in two
+    // team-kernel molecules of one CTA and 34 AOs up to below band_max_nao reduce to tridiagonal form in two
     // stages, the others (and the whole-grid molecules) in one (AXTB_EIGEN_ONESTAGE=1: all in one stage)
     int band_max = o.band_max_nao >= 0 ? o.band_max_nao : DEFAULT_BAND_MAX_NAO;
     if (std::getenv("AXTB_EIGEN_ONESTAGE")) band_max = 0;

@@ -82,7 +82,7 @@ struct Batch {
     const double* sv_srcut;
     int split;                        // 1: basis-transform and W GEMMs in split precision
     int disp;                         // 0: the D4 term is left out (Options::dispersion = false)
-    int band_max;                     // one-CTA molecules below this many AOs reduce to tridiagonal form in two stages
+    int band_max;                     // team-kernel molecules of one CTA below this many AOs reduce to tridiagonal form in two stages
     const int* m_trd;                 // nonzero: the molecule's eigen phase runs in stages (stages.cuh), its reduction on chip (trd.cuh)
     int chase_max;                    // ... with stage 2 in its own launch (k_chase) up to this many AOs (0: none)
 };

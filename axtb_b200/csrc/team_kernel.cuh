@@ -1,6 +1,7 @@
-// The cooperative per-molecule dense algebra kernel. Large molecules (team = the whole grid)
-// are processed first, one after the other; then every CTA works through its own list of small
-// molecules (team = that CTA). Phases:
+// The per-molecule dense algebra kernels, for the molecules that do not run in stages (stages.cuh):
+// under 12 AOs, above what the reduction on chip holds, or asked to reduce in two stages. Large ones
+// (team = the whole grid, k_team_grid, a cooperative launch) one after the other; of the others every
+// CTA of k_team works through its own list (team = that CTA). Phases:
 //   PH_OVERLAP  Cholesky of S and L^-1 (once per geometry; crates/base/src/linalg/eigen.rs:72-113)
 //   PH_EEQ      EEQ start charges from the Cholesky factor of the EEQ matrix
 //               (crates/axtb/src/eeq.rs:43-77, bordered system solved by its Schur complement)
