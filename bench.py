@@ -435,8 +435,7 @@ def main():
                     "frac": ach / fp64, "traffic": None, "share": kd["ms"] / tot_ms,
                     "note": "FP64 dense algebra; achieved = algorithmic FLOPs n^3 (reduction to standard form) + "
                             "4/3 n^3 (tridiagonalisation) + 4 n^2 k (back-transform, L^-T, density) per molecule "
-                            "and eigen phase / CUDA-event time of the phase (k_team, then k_chase and k_team again "
-                            "when the bulge chasing of the two-stage reduction runs on chip); peak = torch "
+                            "and eigen phase / CUDA-event time of the phase (all launches of its stages); peak = torch "
                             "float64 8192^3 GEMM measured on this GPU in this run (the pool's measured peaks hold "
                             "HBM and bf16 only); traffic: ncu DRAM bytes are not measured inside the bench run"}
         else:
