@@ -376,6 +376,42 @@ size_t padded(size_t n) {
 
 }  // namespace
 
+// ------------------------------------------------------------------ plan of the back-transformation
+// Columns of the back-transformation per CTA, for staged molecules of these sizes: 24 (each block of
+// reflectors read once per 24 columns) when that fills the GPU and the molecule's rows fit, else 8
+static vector<int> apply_widths(const vector<int>& nao, int nsm) {
+    long long wide = 0;
+    for (int n : nao) wide += (n / 2 + 23) / 24;
+    vector<int> w;
+    for (int n : nao) w.push_back(wide >= nsm && n <= axg::st_apply_rows(24, axg::TRD_SMEM_MAX) ? 24 : 8);
+    return w;
+}
+// The back-transformation's launches: the molecules of one width and of lo < n <= hi AOs, each launch
+// with its own shared memory (those of which two CTAs fit a multiprocessor in one of their own). The
+// bounds are what the shared memory holds, whatever the batch's largest molecule: together they take
+// every molecule that has the width.
+struct ApplyLaunch {
+    int width, warps, lo, hi;
+    bool takes(int n, int w) const { return w == width && n > lo && n <= hi; }
+};
+static vector<ApplyLaunch> apply_launches(const vector<int>& nao, const vector<int>& width) {
+    int nmax = 0;
+    bool narrow = false, wide = false;
+    for (size_t i = 0; i < nao.size(); i++) {
+        nmax = std::max(nmax, nao[i]);
+        (width[i] == 24 ? wide : narrow) = true;
+    }
+    vector<ApplyLaunch> v;
+    if (narrow) v.push_back({8, 16, 0, nmax});
+    if (wide) {
+        const int half = std::min(nmax, axg::st_apply_rows(24, axg::TRD_SMEM_MAX / 2 - 1024));
+        const int all = std::min(nmax, axg::st_apply_rows(24, axg::TRD_SMEM_MAX));
+        v.push_back({24, 8, 0, half});
+        if (all > half) v.push_back({24, 16, half, all});
+    }
+    return v;
+}
+
 // ------------------------------------------------------------------ the batch engine
 struct Moments;  // a molecule's SCC moments (capi.cuh)
 struct StageCounts;
@@ -411,7 +447,7 @@ struct AxtbBatch {
     };
     axg::StagePlan Q{};      // the molecules whose eigen phase runs in stages (those of trd and trd_grid)
     long long q_full = 0, q_low = 0, q_rt = 0, q_vec = 0, q_col = 0, q_full32 = 0, q_low32 = 0;  // its tasks
-    bool q_wide = false, q_narrow = false;  // widths of the back-transformation's column blocks in use
+    vector<ApplyLaunch> q_apply;  // the back-transformation's launches
     int q_nmax = 0, q_natmax = 0;
     int nteam_eigen = 0;     // the other molecules (team kernels)
     vector<TrdLaunch> trd;
@@ -720,21 +756,11 @@ void AxtbBatch::launch_stages() {
     CK(cudaEventRecord(fac_ev[1], fac_st));
     stage_vectors(B, S, Q, P, cnt, st);
     CK(cudaStreamWaitEvent(st, fac_ev[1], 0));
-    auto apply = [&](auto NC, auto NW, int n_lo, int n_hi) {
-        constexpr int C_ = decltype(NC)::value, W_ = decltype(NW)::value;
-        k_st_apply<C_, W_><<<(unsigned)q_col, 32 * W_, st_apply_doubles(n_hi, C_) * 8, st>>>(B, S, Q, P, n_lo, n_hi);
+    for (const ApplyLaunch& a : q_apply) {
+        const void* fn = a.width == 8 ? (const void*)k_st_apply<8, 16> : a.warps == 8 ? (const void*)k_st_apply<24, 8> : (const void*)k_st_apply<24, 16>;
+        void* args[] = {&B, &S, &Q, &P, (void*)&a.lo, (void*)&a.hi};
+        CK(cudaLaunchKernel(fn, dim3((unsigned)q_col), dim3(32 * a.warps), args, st_apply_doubles(a.hi, a.width) * 8, st));
         launches++;
-    };
-    std::integral_constant<int, 8> c8;
-    std::integral_constant<int, 16> c16;
-    std::integral_constant<int, 24> c24;
-    if (q_narrow) apply(c8, c16, 0, q_nmax);
-    if (q_wide) {  // molecules of which two CTAs fit a multiprocessor in a launch of their own
-        int half = q_nmax, all = q_nmax;
-        while (st_apply_doubles(half, 24) * 8 > TRD_SMEM_MAX / 2 - 1024) half -= 8;
-        while (st_apply_doubles(all, 24) * 8 > TRD_SMEM_MAX) all -= 8;
-        apply(c24, c8, 0, half);
-        if (all > half) apply(c24, c16, half, all);
     }
     stage_density(B, S, Q, cnt, st);
     launches += 11;
@@ -1328,16 +1354,17 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         vector<int> list, width;
         for (int m = 0; m < nmol; m++)
             if (trd_kind[m]) list.push_back(m);
-        // columns of the back-transformation per CTA: 24 (each block of reflectors read once per 24
-        // columns) when that fills the GPU and the molecule's rows fit, else 8
-        long long wide = 0;
-        for (int m : list) wide += (m_nao[m] / 2 + 23) / 24;
+        vector<int> sizes;
+        for (int m : list) sizes.push_back(m_nao[m]);
+        width = apply_widths(sizes, nsm);
+        q_apply = apply_launches(sizes, width);
         vector<long long> full{0}, low{0}, rts{0}, vec{0}, col{0}, full32{0}, low32{0};
-        for (int m : list) {
+        for (size_t i = 0; i < list.size(); i++) {
+            const int m = list[i], w = width[i];
             long long n = m_nao[m], rt = (n + axg::GT - 1) / axg::GT;
-            int w = wide >= nsm && axg::st_apply_doubles((int)n, 24) * 8 <= axg::TRD_SMEM_MAX ? 24 : 8;
-            width.push_back(w);
-            (w == 24 ? q_wide : q_narrow) = true;
+            int takers = 0;
+            for (const ApplyLaunch& a : q_apply) takers += a.takes((int)n, w);
+            if (takers != 1) throw Fail(AXTB_ERR_DEVICE, "no launch of the back-transformation for " + std::to_string(n) + " AOs");
             q_nmax = std::max(q_nmax, (int)n);
             q_natmax = std::max(q_natmax, mols[m].nat);
             full.push_back(full.back() + rt * rt);

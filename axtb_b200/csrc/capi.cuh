@@ -476,6 +476,18 @@ int axtb_gpu_batch_set_moments(AxtbBatch* b, int32_t mol, const double* qsh, con
     });
 }
 
+int axtb_gpu_apply_plan(const int32_t* nao, int32_t count, int32_t nsm, int32_t* width, int32_t* launches) {
+    if (!nao || !width || !launches || count < 0 || nsm <= 0) return AXTB_ERR_INPUT;
+    const vector<int> sizes(nao, nao + count), w = apply_widths(sizes, nsm);
+    const vector<ApplyLaunch> plan = apply_launches(sizes, w);
+    for (int i = 0; i < count; i++) {
+        width[i] = w[i];
+        launches[i] = 0;
+        for (const ApplyLaunch& a : plan) launches[i] += a.takes(sizes[i], w[i]);
+    }
+    return AXTB_OK;
+}
+
 int axtb_gpu_batch_set_profiling(AxtbBatch* b, int32_t enable) {
     if (!b) return AXTB_ERR_INPUT;
     b->profiling = enable != 0;

@@ -762,6 +762,11 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_tfac(Batch B, State S, Stag
 // shared memory of k_st_apply (doubles): the columns, row by row, then three 64 x NC blocks. NC is 8
 // or 24: a row pitch of 8 mod 16 doubles serves the fragments without bank conflicts as it is.
 __host__ __device__ constexpr long long st_apply_doubles(int n, int nc) { return (long long)((n + 7) / 8 * 8 + 3 * ST_NB) * nc; }
+// the most AOs whose columns fit so many bytes
+__host__ __device__ constexpr int st_apply_rows(int nc, int bytes) { return (bytes / 8 / nc - 3 * ST_NB) / 8 * 8; }
+static_assert(st_apply_doubles(st_apply_rows(24, TRD_SMEM_MAX), 24) * 8 <= TRD_SMEM_MAX &&
+              st_apply_doubles(st_apply_rows(24, TRD_SMEM_MAX) + 1, 24) * 8 > TRD_SMEM_MAX,
+              "st_apply_rows is st_apply_doubles' inverse");
 
 // Z <- Q Z for NC columns, held in shared memory from the first block of reflectors to the last:
 // per block Y = V^T Z, Y <- T Y, Z -= V Y on the FP64 tensor cores, V straight from L2 into the

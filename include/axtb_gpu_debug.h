@@ -44,6 +44,11 @@ int axtb_gpu_batch_profile(const AxtbBatch* b, char* buf, size_t len);
 /* Copy quantity `what` of molecule `mol` of the last run into host memory `out`. */
 int axtb_gpu_batch_debug(AxtbBatch* b, int32_t mol, int32_t what, double* out);
 
+/* The back-transformation's plan for staged molecules of these sizes on a device of nsm
+ * multiprocessors (host arithmetic, no device needed): per molecule the columns of a CTA and the
+ * number of launches that take it. Every molecule has to be taken by exactly one. */
+int axtb_gpu_apply_plan(const int32_t* nao, int32_t count, int32_t nsm, int32_t* width, int32_t* launches);
+
 #ifdef __cplusplus
 }
 #endif
