@@ -412,6 +412,32 @@ static vector<ApplyLaunch> apply_launches(const vector<int>& nao, const vector<i
     return v;
 }
 
+// ------------------------------------------------------------------ order of the eigen phase
+// Its launches in order, each on the batch's stream or on the side stream that forks off where the first
+// side step stands and joins at the end. Whatever needs all of its CTAs resident at once (k_team_grid, and
+// k_trd_grid among the stages) stays on the batch's stream: two such kernels in flight could each hold a
+// part of the GPU and wait for the rest, and either fills it alone, so there is nothing to overlap.
+// k_team and k_chase wait for nobody outside their own CTA or cluster: beside the stages they run on
+// the side stream.
+enum EigenKernel { EK_TEAM_GRID = 0, EK_TEAM = 1, EK_CHASE = 2, EK_TEAM_TAIL = 3, EK_STAGES = 4 };
+struct EigenStep {
+    EigenKernel kernel;
+    bool side;
+};
+// grid_mols: molecules of k_team_grid; team: molecules of either team kernel; chase: bands of k_chase;
+// staged: molecules in stages
+static vector<EigenStep> eigen_steps(bool grid_mols, bool team, bool chase, bool staged) {
+    vector<EigenStep> v;
+    if (grid_mols) v.push_back({EK_TEAM_GRID, false});
+    if (team) v.push_back({EK_TEAM, staged});
+    if (team && chase) {
+        v.push_back({EK_CHASE, staged});
+        v.push_back({EK_TEAM_TAIL, staged});
+    }
+    if (staged) v.push_back({EK_STAGES, false});
+    return v;
+}
+
 // ------------------------------------------------------------------ the batch engine
 struct Moments;  // a molecule's SCC moments (capi.cuh)
 struct StageCounts;
@@ -1885,17 +1911,22 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     Psmall.nbig = 0;
     void* args_small[] = {&B, &S, &Psmall, &ph};
     // (no one-CTA molecule needs the others' CTAs: a plain launch, which shares the GPU)
-    auto team_launch = [&](int phase, cudaStream_t on = nullptr) {
-        if (!on) on = st;
+    auto team_grid_launch = [&](int phase) {
+        ph = phase;
+        CK(cudaLaunchCooperativeKernel((void*)k_team_grid, grid, TEAM_THREADS, args, SMEM_WORK_BYTES, st));
+        launches++;
+    };
+    auto team_cta_launch = [&](int phase, cudaStream_t on) {
         ph = phase;
         Psmall = P;
         Psmall.nbig = 0;
-        if (P.nbig > 0 && phase != PH_EIGEN_TAIL) {  // no whole-grid molecule has a part after k_chase
-            CK(cudaLaunchCooperativeKernel((void*)k_team_grid, grid, TEAM_THREADS, args, SMEM_WORK_BYTES, on));
-            launches++;
-        }
         CK(cudaLaunchKernel((void*)k_team, grid, TEAM_THREADS, args_small, SMEM_WORK_BYTES, on));
     };
+    auto team_launch = [&](int phase) {
+        if (P.nbig > 0) team_grid_launch(phase);
+        team_cta_launch(phase, st);
+    };
+    const vector<EigenStep> eigen = eigen_steps(P.nbig > 0, nteam_eigen > 0, nchase > 0, Q.count > 0);
     double chol_flops = 0.0;
     for (int m = 0; m < nmol; m++) chol_flops += (1.0 / 3.0 + 2.0 / 3.0) * std::pow((double)mols[m].nao, 3.0);
     LAUNCH("team_overlap", chol_flops, 0, {
@@ -1929,26 +1960,34 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
             LAUNCH("fock", 0, mat_bytes(act, 12.0), k_fock<<<(unsigned)ntiles, T, 0, st>>>(B, S, d_tile0, ntiles));
             // the eigen phase: one launch, or three when k_chase takes stage 2 of some molecules
             LAUNCH("team_eigen", eig_flops(act), 0, {
-                // the one-CTA molecules beside the staged ones
-                const bool beside = nteam_eigen > 0 && Q.count > 0;
-                cudaStream_t x = beside ? team_st : st;
-                if (beside) {
-                    CK(cudaEventRecord(team_ev[0], st));
-                    CK(cudaStreamWaitEvent(x, team_ev[0], 0));
-                }
-                if (nteam_eigen > 0) {
-                    team_launch(PH_EIGEN, x);
-                    if (nchase > 0) {
-                        CP.cycles = P.cycles;
-                        k_chase<<<chase_grid, CHASE_THREADS, CHASE_DYN_BYTES, x>>>(B, S, CP);
-                        CK(cudaGetLastError());
-                        team_launch(PH_EIGEN_TAIL, x);
-                        launches += 2;
+                bool forked = false;
+                for (const EigenStep& step : eigen) {
+                    if (step.side && !forked) {
+                        CK(cudaEventRecord(team_ev[0], st));
+                        CK(cudaStreamWaitEvent(team_st, team_ev[0], 0));
+                        forked = true;
+                    }
+                    cudaStream_t x = step.side ? team_st : st;
+                    switch (step.kernel) {
+                        case EK_TEAM_GRID: team_grid_launch(PH_EIGEN); break;
+                        case EK_TEAM: team_cta_launch(PH_EIGEN, x); break;
+                        case EK_CHASE:
+                            CP.cycles = P.cycles;
+                            k_chase<<<chase_grid, CHASE_THREADS, CHASE_DYN_BYTES, x>>>(B, S, CP);
+                            CK(cudaGetLastError());
+                            launches++;
+                            break;
+                        case EK_TEAM_TAIL:
+                            team_cta_launch(PH_EIGEN_TAIL, x);
+                            launches++;
+                            break;
+                        case EK_STAGES: launch_stages(); break;
                     }
                 }
-                if (beside) CK(cudaEventRecord(team_ev[1], x));
-                if (Q.count > 0) launch_stages();
-                if (beside) CK(cudaStreamWaitEvent(st, team_ev[1], 0));
+                if (forked) {
+                    CK(cudaEventRecord(team_ev[1], team_st));
+                    CK(cudaStreamWaitEvent(st, team_ev[1], 0));
+                }
             });
             LAUNCH("mulliken", 0, mat_bytes(act, 12.0),
                    k_mulliken<<<blocks_for((long long)naoT * 32, T), T, 0, st>>>(B, S));

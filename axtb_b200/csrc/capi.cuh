@@ -488,6 +488,16 @@ int axtb_gpu_apply_plan(const int32_t* nao, int32_t count, int32_t nsm, int32_t*
     return AXTB_OK;
 }
 
+int axtb_gpu_eigen_order(int32_t grid_mols, int32_t team, int32_t chase, int32_t staged, int32_t* kernel, int32_t* side) {
+    if (!kernel || !side) return AXTB_ERR_INPUT;
+    const vector<EigenStep> v = eigen_steps(grid_mols != 0, team != 0, chase != 0, staged != 0);
+    for (size_t i = 0; i < 5; i++) {
+        kernel[i] = i < v.size() ? (int)v[i].kernel : -1;
+        side[i] = i < v.size() && v[i].side;
+    }
+    return AXTB_OK;
+}
+
 int axtb_gpu_batch_set_profiling(AxtbBatch* b, int32_t enable) {
     if (!b) return AXTB_ERR_INPUT;
     b->profiling = enable != 0;

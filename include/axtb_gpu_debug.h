@@ -49,6 +49,12 @@ int axtb_gpu_batch_debug(AxtbBatch* b, int32_t mol, int32_t what, double* out);
  * number of launches that take it. Every molecule has to be taken by exactly one. */
 int axtb_gpu_apply_plan(const int32_t* nao, int32_t count, int32_t nsm, int32_t* width, int32_t* launches);
 
+/* The eigen phase's launches in order for a batch that has whole-grid team molecules, team molecules
+ * at all, bands of k_chase, staged molecules: five entries each of kernel (0 k_team_grid, 1 k_team,
+ * 2 k_chase, 3 k_team's second part, 4 the stages with k_trd_grid, -1 none) and side (1: on the stream
+ * beside the batch's). No device needed. */
+int axtb_gpu_eigen_order(int32_t grid_mols, int32_t team, int32_t chase, int32_t staged, int32_t* kernel, int32_t* side);
+
 #ifdef __cplusplus
 }
 #endif

@@ -28,3 +28,26 @@ def test_back_transformation_takes_every_molecule_once(engine):
     assert width.tolist() == [8] * 6 and (launches == 1).all()
     width, launches = _apply_plan([1014] * 6 + [1202])
     assert width.tolist() == [24] * 6 + [8] and (launches == 1).all()
+
+
+def test_kernels_that_need_the_whole_gpu_share_one_stream(engine):
+    """k_team_grid and k_trd_grid (in the stages) wait for all of their own CTAs: never in flight beside
+    one another. Everything asked for is launched once, the team kernel's parts in their order."""
+    from axtb_b200 import _lib
+
+    TEAM_GRID, TEAM, CHASE, TAIL, STAGES = range(5)
+    for bits in range(16):
+        grid_mols, team, chase, staged = (bits >> k & 1 for k in range(4))
+        if (grid_mols or chase) and not team:  # both are team molecules
+            continue
+        kernel, side = (C.c_int32 * 5)(), (C.c_int32 * 5)()
+        assert _lib.load().axtb_gpu_eigen_order(grid_mols, team, chase, staged, kernel, side) == 0
+        steps = [(k, s) for k, s in zip(kernel, side) if k >= 0]
+        order = [k for k, _ in steps]
+        want = [TEAM_GRID] * grid_mols + [TEAM] * team + [CHASE, TAIL] * chase + [STAGES] * staged
+        assert sorted(order) == sorted(want)
+        assert all(s == 0 for k, s in steps if k in (TEAM_GRID, STAGES)), steps
+        chain = [k for k in order if k in (TEAM, CHASE, TAIL)]
+        assert chain == sorted(chain) and len({s for k, s in steps if k in chain}) <= 1
+        if grid_mols:  # before the fork: the side stream's kernels start after it
+            assert order[0] == TEAM_GRID
