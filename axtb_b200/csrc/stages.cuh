@@ -472,6 +472,9 @@ __device__ __forceinline__ Clusters warp_clusters(const double* d, const double*
     return {1e-6 * tnrm, 10.0 * DBL_EPSILON * tnrm, DBL_EPSILON * tnrm};
 }
 
+// a pivot whose reciprocal is finite: a zero or subnormal one becomes the floor
+__device__ __forceinline__ double invit_pivot(double pv, double floor) { return fabs(pv) < DBL_MIN ? floor : pv; }
+
 __host__ __device__ constexpr int st_invit_bytes(int n) { return 8 * (2 * (n + 8) + 32 * 3 * 32); }
 __device__ __forceinline__ double* stage_norms(const TeamPlan& P, int m) { return P.wk + P.m_wk0[m] + 32; }
 
@@ -503,7 +506,7 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
     constexpr int GR = 4, NG = 8, R = GR * NG;
     double* ring = s_work + 2 * (n + 8) + threadIdx.x;
     auto slot = [&](int step, int f) { return ring + ((step & (R - 1)) * 3 + f) * 32; };  // f beyond 2: later rows
-    double ss = 1.0;
+    double nrm = 1.0;  // 1 / norm of the last solution
     // L with the row interchanges, the first solution (1 / its norm: nr) normalised on the way
     auto forward = [&](double nr) {
         const long long st = LD;
@@ -549,7 +552,7 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
         cp_async_wait<0>();
         x[(n - 1) * st] = cur;
     };
-    // U with up to two superdiagonals (e_{i+1} after an interchange); the squared norm into ss
+    // U with up to two superdiagonals (e_{i+1} after an interchange); its norm's reciprocal into nrm
     auto backward = [&]() {
         const long long st = LD;
         auto issue = [&](int g) {  // rows n - 1 - 4 g downwards
@@ -572,8 +575,7 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
             }
             cp_async_commit();
         };
-        double xn1 = 0.0, xn2 = 0.0;
-        ss = 0.0;
+        double xn1 = 0.0, xn2 = 0.0, ss = 0.0;
         for (int g = 0; g < NG - 1; g++) issue(g);
         unsigned bits = swaps[((n - 1) >> 5) * st] << (31 - ((n - 1) & 31));
         double* px = x + (n - 1) * st;
@@ -604,9 +606,19 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
             }
         }
         cp_async_wait<0>();
-        if (!(ss > 0.0) || !isfinite(ss)) {
-            atomicOr(&S.status[m], ST_INVIT);
-            ss = 1.0;
+        nrm = 1.0 / sqrt(ss);
+        if (!(ss > 1e-280 && ss < INFINITY)) {
+            // the squares left the range (a level within 1e-140 of a decoupled row's diagonal element gives
+            // elements above 1e154), not the solution: its norm from elements scaled by the largest
+            double mx = 0.0, sc = 0.0;
+            for (int i = 0; i < n; i++) mx = fmax(mx, fabs(x[i * st]));
+            const double inv = 1.0 / mx;
+            for (int i = 0; i < n; i++) sc = fma(x[i * st] * inv, x[i * st] * inv, sc);
+            nrm = inv / sqrt(sc);
+            if (isnan(ss) || !(mx > 0.0 && mx < INFINITY)) {
+                atomicOr(&S.status[m], ST_INVIT);
+                nrm = 1.0;
+            }
         }
     };
     if (part == 0) {
@@ -624,8 +636,7 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
             const double sub = se[i], a1 = sd[i + 1] - lam, b1 = se[i + 1];
             const double nxt = hash_uniform((unsigned)q, (unsigned)(i + 1));
             const bool p = fabs(ca) < fabs(sub);
-            double pv = p ? sub : ca;
-            if (pv == 0.0) pv = cl.pivmin;
+            const double pv = invit_pivot(p ? sub : ca, cl.pivmin);
             const double inv = 1.0 / pv, l = (p ? ca : sub) * inv, t1 = p ? a1 : cb;
             const long long ix = (long long)i * LD;
             u0[ix] = inv;
@@ -642,18 +653,18 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
             cb = p ? -l * b1 : b1;
         }
         swaps[((n - 1) >> 5) * LD] = bits;
-        u0[(n - 1) * LD] = 1.0 / (ca == 0.0 ? cl.pivmin : ca);
+        u0[(n - 1) * LD] = 1.0 / invit_pivot(ca, cl.pivmin);
         x[(n - 1) * LD] = cur;
         backward();
         if (alone) {
-            forward(1.0 / sqrt(ss));
+            forward(nrm);
             backward();
         }
     } else {
         forward(stage_norms(P, m)[q]);
         backward();
     }
-    stage_norms(P, m)[q] = 1.0 / sqrt(ss);  // applied by whoever reads the vector next
+    stage_norms(P, m)[q] = nrm;  // applied by whoever reads the vector next
 }
 
 // Gram-Schmidt within the clusters (ascending, each vector against all earlier ones of its cluster,
