@@ -415,7 +415,7 @@ static vector<ApplyLaunch> apply_launches(const vector<int>& nao, const vector<i
 // ------------------------------------------------------------------ order of the eigen phase
 // Its launches in order, each on the batch's stream or on the side stream that forks off where the first
 // side step stands and joins at the end. Whatever needs all of its CTAs resident at once (k_team_grid, and
-// k_trd_grid among the stages) stays on the batch's stream: two such kernels in flight could each hold a
+// k_trd_grid and k_trd_teams among the stages) stays on the batch's stream: two such kernels in flight could each hold a
 // part of the GPU and wait for the rest, and either fills it alone, so there is nothing to overlap.
 // k_team and k_chase wait for nobody outside their own CTA or cluster: beside the stages they run on
 // the side stream.
@@ -460,7 +460,7 @@ struct AxtbBatch {
     axg::ChasePlan CP{};    // molecules whose band k_chase reduces (stage 2 on chip)
     int nchase = 0, chase_grid = 0;
     // tridiagonal reductions on chip: one launch per size class and cluster size (k_trd), each on
-    // its own stream, and the whole-grid molecules one after the other (k_trd_grid)
+    // its own stream, and the whole-grid molecules one after the other or a few at a time (k_trd_grid, k_trd_teams)
     struct TrdLaunch {
         const void* fn;
         int G, count, smem;
@@ -469,7 +469,10 @@ struct AxtbBatch {
     };
     struct TrdGrid {
         const void* fn;
-        int mol, smem;
+        int teams, ctas, smem;  // ctas: of a team
+        vector<int> mols;
+        const int* list;  // the same on the device
+        long long x0;  // of its first molecule in d_xpub
     };
     axg::StagePlan Q{};      // the molecules whose eigen phase runs in stages (those of trd and trd_grid)
     long long q_full = 0, q_low = 0, q_rt = 0, q_vec = 0, q_col = 0, q_full32 = 0, q_low32 = 0;  // its tasks
@@ -478,8 +481,8 @@ struct AxtbBatch {
     int nteam_eigen = 0;     // the other molecules (team kernels)
     vector<TrdLaunch> trd;
     vector<TrdGrid> trd_grid;
-    int grid_sms = 0;          // CTAs of k_trd_grid
-    double* d_xpub = nullptr;  // what k_trd_grid's CTAs publish to one another
+    double* d_xpub = nullptr;  // what the CTAs of such a molecule publish to one another, xpub_stride doubles each
+    long long xpub_stride = 0;
     cudaStream_t fac_st = nullptr;   // the reflectors' triangular factors (stages.cuh)
     cudaEvent_t fac_ev[2] = {nullptr, nullptr};
     cudaStream_t team_st = nullptr;  // the one-CTA molecules beside the stages
@@ -644,10 +647,12 @@ static void stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::
 // TRD_MIN_NAO AOs on. Below it there is nothing to win (one water of 6 AOs: 121 us per iteration in
 // the one-CTA kernel, ~110 in stages, most of it launches), and the SCF of a water stretched to 3 A,
 // recorded as a failure in the tblite conventions, follows the one-CTA kernel's bits. A molecule sits
-// on a cluster as long as 16 CTAs hold it (768 AOs); from big_nao on, and above 768 AOs in batches of
-// at most 64 such molecules (one after the other at ~2.8 us per reflector they beat one CTA each, 296
-// at a time and ~85 ms, only while they are few), on the whole grid as long as the chip holds the
-// matrix (2400 AOs). A band_max_nao above its default asks for the two-stage reduction below it.
+// on a cluster as long as 16 CTAs hold it (768 AOs); from big_nao on, and above 768 AOs, on the grid or a
+// team of it (grid_teams) as long as the chip holds the matrix (2405 AOs). The choice is by the
+// molecule's size alone, and so are its bits. One CTA per molecule, the other way for 769 to 1023 AOs, takes
+// 167 / 201 / 224 ms per eigen phase for 65 / 148 / 296 molecules of 780 AOs and 344 / 399 / 436 at 1020; the
+// grid's teams take 55 / 117 / 228 and 104 / 227 / 454. A band_max_nao above its default asks for the two-stage
+// reduction below it.
 constexpr int TRD_MIN_NAO = 12;
 void AxtbBatch::plan_trd(int big_nao, int band_max, const vector<int>& nao, int nsm, vector<int>& kind) {
     const bool two_stage_asked = band_max > DEFAULT_BAND_MAX_NAO;
@@ -655,21 +660,34 @@ void AxtbBatch::plan_trd(int big_nao, int band_max, const vector<int>& nao, int 
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     CK(cudaDeviceGetAttribute(&clusters, cudaDevAttrClusterLaunch, device));
     if (optin < axg::TRD_SMEM_MAX || !clusters) return;
-    const int cluster_max = axg::TRD_CLUSTER_MAX_NAO;
-    int large = 0;
-    for (int n : nao) large += n > cluster_max && n < big_nao;
     for (int m = 0; m < nmol; m++) {
         int n = nao[m];
         if (n < TRD_MIN_NAO) continue;
-        bool grid_mol = n >= big_nao || (n > cluster_max && large <= 64);
-        if (!grid_mol) {
-            if (n > cluster_max || (two_stage_asked && n > axg::BW + 1 && n < band_max)) continue;
+        if (n < big_nao && two_stage_asked && n > axg::BW + 1 && n < band_max) continue;
+        if (n < big_nao && n <= axg::TRD_CLUSTER_MAX_NAO) {
             kind[m] = 1;
             continue;
         }
         const axg::TrdClass* c = axg::trd_grid_class(n);
         if (c && axg::trd_smem_doubles(n, nsm, 8, c->cr, true) * 8 <= axg::TRD_SMEM_MAX) kind[m] = 2;
     }
+}
+
+// Teams that share the grid of k_trd_grid for `count` molecules of up to n AOs, each on nsm / teams CTAs
+// as long as those hold the matrix: the fewest rounds times what a round takes. Fewer CTAs have more
+// columns each but exchange with fewer others. Measured, ms of a molecule's eigen phase on 1 / 2 / 3 / 4 /
+// 5 / 6 teams: 2.5 / 2.9 / 3.3 / 4.0 / 4.4 / 5.1 at 780 AOs, 3.5 / 4.6 / 5.6 / 6.2 at 1020, 7.2 / 10.2 at
+// 1500: 1 + 0.00026 n (teams - 1) of the whole grid's. At least 16 CTAs a team, the smallest in use there.
+static int grid_teams(int n, int count, int nsm) {
+    const axg::TrdClass* c = axg::trd_grid_class(n);
+    int best = 1;
+    double least = INFINITY;
+    for (int t = 1; t <= (c->teams ? std::max(1, nsm / 16) : 1); t++) {
+        if (axg::trd_smem_doubles(n, nsm / t, 8, c->cr, true) * 8 > axg::TRD_SMEM_MAX) break;
+        const double cost = ((count + t - 1) / t) * (1.0 + 0.00026 * n * (t - 1));
+        if (cost < least) least = cost, best = t;
+    }
+    return best;
 }
 
 // The launches of the reductions on chip: per size class, molecules grouped by the cluster size
@@ -682,13 +700,11 @@ void AxtbBatch::plan_trd(int big_nao, int band_max, const vector<int>& nao, int 
 void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int nsm,
                           const std::function<const int*(const vector<int>&)>& up) {
     std::map<std::pair<const axg::TrdClass*, int>, vector<int>> groups;  // (class, cluster size) -> molecules
+    std::map<const axg::TrdClass*, vector<int>> grids;
     vector<int> G(nmol, 0);
     for (int m = 0; m < nmol; m++) {
         int n = nao[m];
-        if (kind[m] == 2) {
-            const axg::TrdClass* c = axg::trd_grid_class(n);
-            trd_grid.push_back({c->fn, m, (int)(axg::trd_smem_doubles(n, nsm, 8, c->cr, true) * 8)});
-        }
+        if (kind[m] == 2) grids[axg::trd_grid_class(n)].push_back(m);
         if (kind[m] != 1) continue;
         G[m] = 1;
         while (axg::trd_smem_doubles(n, G[m], 1, axg::trd_class(n)->cr, false) * 8 > axg::TRD_SMEM_MAX) G[m]++;
@@ -731,8 +747,17 @@ void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int n
         trd.push_back({c.fn, g, (int)v.size(), (int)sm, up(v), (double)nao[v[0]]});
     }
     std::sort(trd.begin(), trd.end(), [](const TrdLaunch& a, const TrdLaunch& b) { return a.cost > b.cost; });
-    for (auto& t : trd_grid) CK(cudaFuncSetAttribute(t.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
-    grid_sms = nsm;
+    long long x0 = 0;
+    for (auto& kv : grids) {
+        vector<int>& v = kv.second;
+        std::sort(v.begin(), v.end(), [&](int a, int b) { return nao[a] > nao[b]; });
+        const axg::TrdClass& c = *kv.first;
+        const int teams = grid_teams(nao[v[0]], (int)v.size(), nsm), ctas = nsm / teams;
+        const void* fn = teams > 1 ? c.teams : c.fn;
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, axg::TRD_SMEM_MAX));
+        trd_grid.push_back({fn, teams, ctas, (int)(axg::trd_smem_doubles(nao[v[0]], ctas, 8, c.cr, true) * 8), v, up(v), x0});
+        x0 += xpub_stride * (long long)v.size();
+    }
     // side streams: every launch after the first runs beside it
     for (size_t i = 1; i < trd.size(); i++) {
         cudaStream_t x;
@@ -748,10 +773,16 @@ void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int n
 
 void AxtbBatch::launch_trd() {
     for (auto& t : trd_grid) {
-        void* args[] = {&B, &S, &t.mol, &d_xpub, &P.cycles};
-        CK(cudaMemsetAsync(d_xpub, 0, sizeof(double) * (4 * (size_t)mols[t.mol].nao + 1), st));  // no pair is there yet
-        CK(cudaLaunchCooperativeKernel(t.fn, grid_sms, axg::TRD_THREADS, args, t.smem, st));
-        launches++;
+        double* x = d_xpub + t.x0;
+        CK(cudaMemsetAsync(x, 0, sizeof(double) * xpub_stride * t.mols.size(), st));  // no pair is there yet
+        for (size_t i = 0; i < t.mols.size(); i += t.teams, x += xpub_stride * t.teams) {  // a team per molecule
+            const int* list = t.list + i;
+            void* one[] = {&B, &S, &t.mols[i], &x, &P.cycles};
+            void* many[] = {&B, &S, &list, &x, &xpub_stride, &P.cycles};
+            const unsigned teams = (unsigned)std::min<size_t>(t.teams, t.mols.size() - i);
+            CK(cudaLaunchCooperativeKernel(t.fn, dim3(t.ctas, teams), axg::TRD_THREADS, t.teams > 1 ? many : one, t.smem, st));
+            launches++;
+        }
     }
     if (trd.size() > 1) CK(cudaEventRecord(side_ev[0], st));
     for (size_t i = 0; i < trd.size(); i++) {
@@ -1137,7 +1168,10 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     for (int c = 0; c < 7; c++) addL((size_t)nmol + 1);
     for (int c = 0; c < 128; c++) addI(1);                   // k_trd lists: at most one per class and cluster size
     addI(nmol);
-    addD(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()) + 1);
+    for (int m = 0; m < nmol; m++)
+        if (trd_kind[m] == 2) xpub_stride = std::max(xpub_stride, 4LL * m_nao[m] + 2);
+    const size_t nxpub = std::max<size_t>(1, (size_t)xpub_stride * std::count(trd_kind.begin(), trd_kind.end(), 2));
+    addD(nxpub);
     {  // the chase plan (k_chase): offsets per cluster and per CTA, molecule lists
         size_t ncl = (size_t)std::max(1, nsm / 2);
         addI(ncl + 1);
@@ -1580,7 +1614,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         s.sv_nbn = ar.take<int>(natT);
     }
     s.red = ar.take<double>((size_t)axg::team_red_doubles(grid));  // grid-team partials
-    d_xpub = ar.take<double>(4 * (size_t)*std::max_element(m_nao.begin(), m_nao.end()) + 1);
+    d_xpub = ar.take<double>(nxpub);
     s.eeq_A = ar.take<double>((size_t)nsqT * 3);
     s.gam = ar.take<double>((size_t)std::max(ngamT, 1LL));
     // team plan

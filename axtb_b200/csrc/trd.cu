@@ -8,7 +8,7 @@ namespace axg {
 // ~90 of 255 registers to the pass. For clusters of G CTAs whose warps have few columns (clusters that
 // grew) a class with all of them in registers and nothing unrolled for columns that are not there.
 const TrdClass* trd_class(int n, int G) {
-#define TRD_C(RT, CR) {RT, CR, (const void*)k_trd<RT, CR>}
+#define TRD_C(RT, CR) {RT, CR, (const void*)k_trd<RT, CR>, nullptr}
     static const TrdClass c[] = {TRD_C(1, 4),  TRD_C(2, 8),  TRD_C(3, 12), TRD_C(4, 16), TRD_C(5, 13), TRD_C(6, 12), TRD_C(7, 10), TRD_C(8, 9),  TRD_C(9, 8),
                                  TRD_C(10, 7), TRD_C(11, 7), TRD_C(12, 6), TRD_C(13, 6), TRD_C(14, 5), TRD_C(15, 5),
                                  TRD_C(16, 5), TRD_C(17, 4), TRD_C(18, 4), TRD_C(19, 4), TRD_C(20, 4), TRD_C(21, 3),
@@ -23,8 +23,10 @@ const TrdClass* trd_class(int n, int G) {
 }
 // whole grid: n <= 256 rt
 const TrdClass* trd_grid_class(int n) {
-#define TRD_C(RT, CR) {RT, CR, (const void*)k_trd_grid<RT, CR>}
-    static const TrdClass c[] = {TRD_C(4, 8), TRD_C(5, 9), TRD_C(6, 11), TRD_C(7, 11), TRD_C(8, 9), TRD_C(10, 9)};
+#define TRD_C(RT, CR) {RT, CR, (const void*)k_trd_grid<RT, CR>, nullptr}
+#define TRD_T(RT, CR) {RT, CR, (const void*)k_trd_grid<RT, CR>, (const void*)k_trd_teams<RT, CR>}
+    static const TrdClass c[] = {TRD_T(4, 8), TRD_T(5, 9), TRD_T(6, 11), TRD_T(7, 11), TRD_C(8, 9), TRD_C(10, 9)};
+#undef TRD_T
 #undef TRD_C
     for (const TrdClass& x : c)
         if (n <= 256 * x.rt) return &x;

@@ -25,6 +25,7 @@ __host__ __device__ constexpr long long trd_smem_doubles(int n, int G, int AW, i
 struct TrdClass {
     int rt, cr;
     const void* fn;
+    const void* teams;  // whole grid: the kernel for several molecules at once (nullptr: sizes that need every CTA)
 };
 // The class of an n x n matrix on clusters of G CTAs (0: the class that says how many it takes), and on
 // the whole grid; nullptr: none.

@@ -81,8 +81,9 @@ typedef struct AxtbOptions {
                           AOs and more keep the reduction on chip (axtb_b200.autotune measures the
                           crossover on a device) */
     int32_t grid_min_nao; /* molecules from this many AOs run their tridiagonal reduction (above 2405
-                          AOs all of their dense algebra) on the whole GPU, one after the other, the rest
-                          beside one another; -1 the default (1024) */
+                          AOs all of their dense algebra) on the whole GPU, one after the other or a few at
+                          a time, the rest beside one another; -1 the default (1024). Molecules above 768
+                          AOs do so in any case (more than a cluster holds) */
 } AxtbOptions;
 
 /* Results of one single point (crates/base/src/method/results.rs:39-57). Array members are
