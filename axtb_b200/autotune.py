@@ -5,8 +5,8 @@ The engine's eigen phase has two schedule choices, both exact (the results agree
 round-off): the tridiagonal reduction (two-stage: band reduction on GEMMs, then bulge chasing,
 one CTA per molecule; or one-stage Householder with the matrix in the registers and shared memory
 of a cluster), chosen by the size ``band_max_nao`` below which the two-stage one is used (from 34
-AOs, and only when set above 64; on B200 the reduction on chip is faster at every size that it
-holds, so the default is never to use the two-stage one); and the size
+AOs; the default, 64, stands for never: on B200 the reduction on chip is faster at every size that it
+holds); and the size
 ``grid_min_nao`` from which a molecule's reduction runs on the whole cooperative grid
 instead of a cluster. The best crossovers depend on the GPU and the batch, so they are measured:
 

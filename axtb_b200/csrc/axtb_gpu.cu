@@ -309,10 +309,9 @@ struct Opt {
     int grid_min_nao = -1;  // schedule: whole-grid teams from this many AOs (-1: default)
 };
 
-// default schedule of the dense algebra (axtb_b200.autotune measures both crossovers on a device):
-// the two-stage reduction below 64 AOs (measured on B200: per molecule it is also cheaper between
-// 224 and 416 AOs with the bulge chasing on chip, but whole batches run no faster, the eigen phase
-// then being three launches with three tails)
+// default schedule of the dense algebra (axtb_b200.autotune measures both crossovers on a device). A
+// band_max_nao of 64, as -1, is the default: no two-stage reduction where the one on chip holds the
+// molecule. Any other asks for the two-stage reduction of molecules of 34 AOs up to below it.
 constexpr int DEFAULT_BAND_MAX_NAO = 64;
 constexpr int STATIC_BAND_MAX_NAO = 64;
 constexpr int DEFAULT_GRID_MIN_NAO = 1024;
@@ -651,11 +650,11 @@ static void stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::
 // team of it (grid_teams) as long as the chip holds the matrix (2405 AOs). The choice is by the
 // molecule's size alone, and so are its bits. One CTA per molecule, the other way for 769 to 1023 AOs, takes
 // 167 / 201 / 224 ms per eigen phase for 65 / 148 / 296 molecules of 780 AOs and 344 / 399 / 436 at 1020; the
-// grid's teams take 55 / 117 / 228 and 104 / 227 / 454. A band_max_nao above its default asks for the two-stage
-// reduction below it.
+// grid's teams take 55 / 117 / 228 and 104 / 227 / 454. A band_max_nao other than the default asks for the
+// two-stage reduction below it (DEFAULT_BAND_MAX_NAO).
 constexpr int TRD_MIN_NAO = 12;
 void AxtbBatch::plan_trd(int big_nao, int band_max, const vector<int>& nao, int nsm, vector<int>& kind) {
-    const bool two_stage_asked = band_max > DEFAULT_BAND_MAX_NAO;
+    const bool two_stage_asked = band_max != DEFAULT_BAND_MAX_NAO;
     int optin = 0, clusters = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     CK(cudaDeviceGetAttribute(&clusters, cudaDevAttrClusterLaunch, device));

@@ -76,10 +76,10 @@ typedef struct AxtbOptions {
     int32_t dispersion;  /* 1 (default): with the D4 dispersion term; 0: without it (Options::dispersion,
                           crates/axtb/src/lib.rs:106-107, 185-187: for validation only) */
     int32_t band_max_nao; /* schedule of the dense algebra (no reference counterpart; results agree to
-                          round-off either way): above 64, molecules of 34 AOs up to below this many use
-                          the two-stage tridiagonal reduction; up to 64, and -1 the default, molecules of 12
-                          AOs and more keep the reduction on chip (axtb_b200.autotune measures the
-                          crossover on a device) */
+                          round-off either way): molecules of 34 AOs up to below this many use the
+                          two-stage tridiagonal reduction, the others of 12 AOs and more the one
+                          on chip; -1 and 64 are the default, the one on chip for all of them
+                          (axtb_b200.autotune measures the crossover on a device) */
     int32_t grid_min_nao; /* molecules from this many AOs run their tridiagonal reduction (above 2405
                           AOs all of their dense algebra) on the whole GPU, one after the other or a few at
                           a time, the rest beside one another; -1 the default (1024). Molecules above 768

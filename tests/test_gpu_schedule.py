@@ -1,0 +1,24 @@
+"""The schedule options choose the reduction they name (GPU; the profiler's cycle shares tell)."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _two_stage(engine, waters, **options):
+    from axtb_b200 import structures as S
+
+    b = engine.Batch([S.water_cluster(waters, seed=2)], accuracy=1.0, **options)
+    b.set_profiling(True)
+    r = b.run(gradient=False)[0]
+    parts = b.profile()["two_stage_parts"]
+    b.close()
+    assert r.status == 0
+    return parts["band_reduction"] > 0.0
+
+
+# 36, 42, 60 and 96 AOs around thresholds below, at and above the default; 780 AOs: above what a cluster holds
+@pytest.mark.parametrize("waters, threshold, expected", [
+    (6, 40, True), (7, 40, False), (7, 48, True), (10, 48, False), (10, 63, True), (10, 65, True), (16, 65, False),
+    (16, 97, True), (130, 1 << 20, True), (6, 33, False), (7, 0, False), (6, 64, False), (10, -1, False)])
+def test_band_max_nao(engine, waters, threshold, expected):
+    assert _two_stage(engine, waters, band_max_nao=threshold) is expected
