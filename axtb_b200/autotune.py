@@ -11,10 +11,10 @@ holds); and the size
 instead of a cluster. The best crossovers depend on the GPU and the batch, so they are measured:
 
 * ``band_max_nao``: one profiled run of a sample batch with each reduction; the engine's
-  per-molecule cycle counters of the eigen phase (the on-chip bulge chasing counted in units of
-  the team kernel's half-SM CTAs) are binned by AO count, and the bin edge that minimises the
-  sample's total with the two-stage reduction below it is the candidate; it, the default and 0
-  (one-stage only) are then timed as whole runs of the sample, and the fastest is kept;
+  per-molecule cycle counters of the eigen phase (all of its stages, in units of the team kernel's
+  half-SM CTAs) are binned by AO count, and the bin edge that minimises the sample's total with the
+  two-stage reduction below it is the candidate; it (when it covers any size) and the default are then
+  timed as whole runs of the sample, and the faster is kept;
 * ``grid_min_nao``: whole runs of the sample with each candidate threshold below its largest
   molecule, timed with CUDA events; the fastest wins (no candidate applies to a sample without
   molecules that large, and the default stays).
@@ -75,6 +75,13 @@ def crossover(nao: np.ndarray, cyc_two: np.ndarray, cyc_one: np.ndarray, width: 
     return int(cut), bins
 
 
+def band_candidates(cut: int) -> list[int]:
+    """The distinct schedules to time: the default (no two-stage reduction) and the two-stage one below
+    `cut`, when that covers any size (from 34 AOs). A cut at the default's own value is named by the next."""
+    default = DEFAULT["band_max_nao"]
+    return [default] + ([cut + (cut == default)] if cut > 34 else [])
+
+
 def _eigen_cycles(mols, options, device):
     from .calculator import Batch
 
@@ -132,10 +139,8 @@ def tune(molecules=None, device: int = 0, accuracy: float = 0.1, save: bool = Tr
         two = _eigen_cycles(small, dict(opts, band_max_nao=1 << 30), device)
         one = _eigen_cycles(small, dict(opts, band_max_nao=0), device)
         cut, bins = crossover(nsmall, two, one)
-        # the per-molecule cycles do not see the launches' tails (the two-stage eigen phase is
-        # three launches, each balanced on its own): the cut, the default and none are timed as
-        # whole runs of the sample, and the fastest wins
-        for bm in sorted({0, DEFAULT["band_max_nao"], cut}):
+        # the per-molecule cycles do not see the launches' tails: whole runs of the sample decide
+        for bm in band_candidates(cut):
             band_times[bm] = _timed_run(mols, {"accuracy": accuracy, "band_max_nao": bm, "grid_min_nao": grid}, device)
         band = min(band_times, key=band_times.get)
     grid_times = {}

@@ -382,7 +382,7 @@ static vector<int> apply_widths(const vector<int>& nao, int nsm) {
     long long wide = 0;
     for (int n : nao) wide += (n / 2 + 23) / 24;
     vector<int> w;
-    for (int n : nao) w.push_back(wide >= nsm && n <= axg::st_apply_rows(24, axg::TRD_SMEM_MAX) ? 24 : 8);
+    for (int n : nao) w.push_back(wide >= nsm && n <= axg::st_apply_rows(24, axg::ST_SMEM_MAX) ? 24 : 8);
     return w;
 }
 // The back-transformation's launches: the molecules of one width and of lo < n <= hi AOs, each launch
@@ -404,7 +404,7 @@ static vector<ApplyLaunch> apply_launches(const vector<int>& nao, const vector<i
     if (narrow) v.push_back({8, 16, 0, nmax});
     if (wide) {
         const int half = std::min(nmax, axg::st_apply_rows(24, axg::TRD_SMEM_MAX / 2 - 1024));
-        const int all = std::min(nmax, axg::st_apply_rows(24, axg::TRD_SMEM_MAX));
+        const int all = std::min(nmax, axg::st_apply_rows(24, axg::ST_SMEM_MAX));
         v.push_back({24, 8, 0, half});
         if (all > half) v.push_back({24, 16, half, all});
     }
@@ -489,6 +489,7 @@ struct AxtbBatch {
     vector<cudaStream_t> side;
     vector<cudaEvent_t> side_ev;  // fork, then one join per side stream
     void launch_trd();
+    template <bool PROF>
     void launch_stages();
     StageCounts stage_counts() const;
     void launch_cholesky(int eeq);
@@ -565,37 +566,45 @@ struct StageCounts {  // tasks; nmax: the largest matrix
     long long full, low, rt, vec, col, full32, low32;
 };
 // the products of a stage; in split precision X, F' and W keep the 64 x 64 tiles that have it
-template <int MODE, bool LOW>
+template <int MODE, bool LOW, bool PROF>
 static void stage_tiles(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                         cudaStream_t st) {
     using namespace axg;
     if constexpr (MODE != ST_C && MODE != ST_P)
         if (B.split) {
-            k_st_tiles<MODE><<<(unsigned)(LOW ? c.low : c.full), TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
+            k_st_tiles<MODE, PROF><<<(unsigned)(LOW ? c.low : c.full), TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
             return;
         }
-    k_st_tiles32<MODE><<<(unsigned)(LOW ? c.low32 : c.full32), 128, GSTAGES * G32_STAGE * 8, st>>>(B, S, Q);
+    k_st_tiles32<MODE, PROF><<<(unsigned)(LOW ? c.low32 : c.full32), 128, GSTAGES * G32_STAGE * 8, st>>>(B, S, Q);
 }
-static void stage_attributes() {
+template <bool PROF>
+static void stage_attributes_of() {
     using namespace axg;
-    const void* work[] = {(const void*)k_st_tiles<ST_X>, (const void*)k_st_tiles<ST_FP>, (const void*)k_st_tiles<ST_W>,
-                          (const void*)k_st_tfac,        (const void*)k_st_bisect,       (const void*)k_st_fermi,
-                          (const void*)k_ch_init,        (const void*)k_ch_panel,        (const void*)k_ch_trail};
+    const void* work[] = {(const void*)k_st_tiles<ST_X, PROF>, (const void*)k_st_tiles<ST_FP, PROF>, (const void*)k_st_tfac<PROF>,
+                          (const void*)k_st_bisect<PROF>, (const void*)k_st_fermi<PROF>};
     for (const void* f : work) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WORK_BYTES));
-    const void* all[] = {(const void*)k_st_apply<8, 16>, (const void*)k_st_apply<24, 8>, (const void*)k_st_apply<24, 16>,
-                         (const void*)k_st_invit};
-    for (const void* f : all) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, TRD_SMEM_MAX));
+    const void* all[] = {(const void*)k_st_apply<8, 16, PROF>, (const void*)k_st_apply<24, 8, PROF>,
+                         (const void*)k_st_apply<24, 16, PROF>, (const void*)k_st_invit<PROF>};
+    for (const void* f : all) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM_MAX));
+}
+static void stage_attributes(bool profiling) {
+    using namespace axg;
+    if (profiling) return stage_attributes_of<true>();
+    stage_attributes_of<false>();
+    const void* work[] = {(const void*)k_st_tiles<ST_W, false>, (const void*)k_ch_init, (const void*)k_ch_panel, (const void*)k_ch_trail};
+    for (const void* f : work) CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WORK_BYTES));
 }
 // F' = L^-1 F L^-T
+template <bool PROF>
 static void stage_transform(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                             cudaStream_t st) {
     using namespace axg;
-    stage_tiles<ST_X, false>(B, S, Q, c, st);
-    stage_tiles<ST_FP, true>(B, S, Q, c, st);
+    stage_tiles<ST_X, false, PROF>(B, S, Q, c, st);
+    stage_tiles<ST_FP, true, PROF>(B, S, Q, c, st);
 }
 // count reductions of one class on clusters of G CTAs
 static void stage_reduce(const void* fn, int G, int count, int smem, const axg::Batch& B, const axg::State& S, const int* list,
-                         int cycles, cudaStream_t st) {
+                         unsigned long long* cycles, cudaStream_t st) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = G;
@@ -611,22 +620,24 @@ static void stage_reduce(const void* fn, int G, int count, int smem, const axg::
     CK(cudaLaunchKernelExC(&cfg, fn, args));
 }
 // levels, filling and vectors of the tridiagonal matrices
+template <bool PROF>
 static void stage_vectors(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P,
                           const StageCounts& c, cudaStream_t st) {
     using namespace axg;
-    k_st_bisect<<<(unsigned)c.vec, ST_POINTS, 16 * (c.nmax + 32), st>>>(B, S, Q, 0);
-    k_st_fermi<<<(unsigned)Q.count, TEAM_THREADS, 24 * (c.nmax + 32), st>>>(B, S, Q);
+    k_st_bisect<PROF><<<(unsigned)c.vec, ST_POINTS, 16 * (c.nmax + 32), st>>>(B, S, Q, 0);
+    k_st_fermi<PROF><<<(unsigned)Q.count, TEAM_THREADS, 24 * (c.nmax + 32), st>>>(B, S, Q);
     for (int part = 0; part < 2; part++) {
-        k_st_invit<<<(unsigned)c.vec, 32, st_invit_bytes(c.nmax), st>>>(B, S, Q, P, part);
-        k_st_gs<<<(unsigned)c.vec, 32, 0, st>>>(B, S, Q, P);
+        k_st_invit<PROF><<<(unsigned)c.vec, 32, st_invit_bytes(c.nmax), st>>>(B, S, Q, P, part);
+        k_st_gs<PROF><<<(unsigned)c.vec, 32, 0, st>>>(B, S, Q, P);
     }
 }
 // C = L^-T Z and P = (C f) C^T
+template <bool PROF>
 static void stage_density(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                           cudaStream_t st) {
     using namespace axg;
-    stage_tiles<ST_C, false>(B, S, Q, c, st);
-    stage_tiles<ST_P, true>(B, S, Q, c, st);
+    stage_tiles<ST_C, false, PROF>(B, S, Q, c, st);
+    stage_tiles<ST_P, true, PROF>(B, S, Q, c, st);
 }
 // factor and inverse factor of the overlap matrices, or of the EEQ matrices; nmax: the largest
 static void stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P, int nmax,
@@ -771,13 +782,18 @@ void AxtbBatch::place_trd(const vector<int>& kind, const vector<int>& nao, int n
 }
 
 void AxtbBatch::launch_trd() {
+    unsigned long long* cycles = nullptr;  // the profiler's slot of the reduction
+    if (P.cycles) {
+        CK(cudaGetSymbolAddress((void**)&cycles, axg::g_team_cycles));
+        cycles++;
+    }
     for (auto& t : trd_grid) {
         double* x = d_xpub + t.x0;
         CK(cudaMemsetAsync(x, 0, sizeof(double) * xpub_stride * t.mols.size(), st));  // no pair is there yet
         for (size_t i = 0; i < t.mols.size(); i += t.teams, x += xpub_stride * t.teams) {  // a team per molecule
             const int* list = t.list + i;
-            void* one[] = {&B, &S, &t.mols[i], &x, &P.cycles};
-            void* many[] = {&B, &S, &list, &x, &xpub_stride, &P.cycles};
+            void* one[] = {&B, &S, &t.mols[i], &x, &cycles};
+            void* many[] = {&B, &S, &list, &x, &xpub_stride, &cycles};
             const unsigned teams = (unsigned)std::min<size_t>(t.teams, t.mols.size() - i);
             CK(cudaLaunchCooperativeKernel(t.fn, dim3(t.ctas, teams), axg::TRD_THREADS, t.teams > 1 ? many : one, t.smem, st));
             launches++;
@@ -788,7 +804,7 @@ void AxtbBatch::launch_trd() {
         TrdLaunch& t = trd[i];
         cudaStream_t x = i == 0 ? st : side[i - 1];
         if (i > 0) CK(cudaStreamWaitEvent(x, side_ev[0], 0));
-        stage_reduce(t.fn, t.G, t.count, t.smem, B, S, t.list, P.cycles, x);
+        stage_reduce(t.fn, t.G, t.count, t.smem, B, S, t.list, cycles, x);
         launches++;
         if (i > 0) {
             CK(cudaEventRecord(side_ev[i], x));
@@ -800,25 +816,30 @@ void AxtbBatch::launch_trd() {
 StageCounts AxtbBatch::stage_counts() const { return {q_nmax, q_full, q_low, q_rt, q_vec, q_col, q_full32, q_low32}; }
 
 // The staged molecules' eigen phase (stages.cuh), between its tridiagonal reductions
+template <bool PROF>
 void AxtbBatch::launch_stages() {
     using namespace axg;
     const StageCounts cnt = stage_counts();
-    stage_transform(B, S, Q, cnt, st);
+    if constexpr (PROF) {
+        k_st_clear_cycles<<<(Q.count + 255) / 256, 256, 0, st>>>(S, Q);
+        launches++;
+    }
+    stage_transform<PROF>(B, S, Q, cnt, st);
     launch_trd();
     // the reflectors' triangular factors beside the levels and vectors of the tridiagonal matrices
     CK(cudaEventRecord(fac_ev[0], st));
     CK(cudaStreamWaitEvent(fac_st, fac_ev[0], 0));
-    k_st_tfac<<<(unsigned)q_rt, TEAM_THREADS, SMEM_WORK_BYTES, fac_st>>>(B, S, Q, P);
+    k_st_tfac<PROF><<<(unsigned)q_rt, TEAM_THREADS, SMEM_WORK_BYTES, fac_st>>>(B, S, Q, P);
     CK(cudaEventRecord(fac_ev[1], fac_st));
-    stage_vectors(B, S, Q, P, cnt, st);
+    stage_vectors<PROF>(B, S, Q, P, cnt, st);
     CK(cudaStreamWaitEvent(st, fac_ev[1], 0));
     for (const ApplyLaunch& a : q_apply) {
-        const void* fn = a.width == 8 ? (const void*)k_st_apply<8, 16> : a.warps == 8 ? (const void*)k_st_apply<24, 8> : (const void*)k_st_apply<24, 16>;
+        const void* fn = a.width == 8 ? (const void*)k_st_apply<8, 16, PROF> : a.warps == 8 ? (const void*)k_st_apply<24, 8, PROF> : (const void*)k_st_apply<24, 16, PROF>;
         void* args[] = {&B, &S, &Q, &P, (void*)&a.lo, (void*)&a.hi};
         CK(cudaLaunchKernel(fn, dim3((unsigned)q_col), dim3(32 * a.warps), args, st_apply_doubles(a.hi, a.width) * 8, st));
         launches++;
     }
-    stage_density(B, S, Q, cnt, st);
+    stage_density<PROF>(B, S, Q, cnt, st);
     launches += 11;
     CK(cudaGetLastError());
 }
@@ -1458,7 +1479,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
             CK(cudaStreamCreateWithFlags(&team_st, cudaStreamNonBlocking));
             for (auto& e : fac_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             for (auto& e : team_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            stage_attributes();
+            stage_attributes(false);
         }
     }
     vector<int> pair_off, pair_list, solo_off, solo_list;
@@ -1852,6 +1873,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     if (profiling) {
         unsigned long long z[TEAM_CYCLE_SLOTS] = {0};
         CK(cudaMemcpyToSymbolAsync(g_team_cycles, z, sizeof z, 0, cudaMemcpyHostToDevice, st));
+        if (Q.count > 0) stage_attributes(true);
     }
     const int T = 256;
     long long nn = nnT;
@@ -2014,7 +2036,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
                             team_cta_launch(PH_EIGEN_TAIL, x);
                             launches++;
                             break;
-                        case EK_STAGES: launch_stages(); break;
+                        case EK_STAGES: P.cycles ? launch_stages<true>() : launch_stages<false>(); break;
                     }
                 }
                 if (forked) {
@@ -2078,7 +2100,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     if (want_levels) {
         LAUNCH("team_levels", 0, 0, {
             if (nteam_eigen > 0) team_launch(PH_LEVELS);
-            if (Q.count > 0) k_st_bisect<<<(unsigned)q_vec, ST_POINTS, 16 * (q_nmax + 32), st>>>(B, S, Q, 1);
+            if (Q.count > 0) k_st_bisect<false><<<(unsigned)q_vec, ST_POINTS, 16 * (q_nmax + 32), st>>>(B, S, Q, 1);
         });
     }
     CK(cudaEventRecord(phase_ev[2], st));
@@ -2087,7 +2109,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
             if (nteam_eigen > 0) team_launch(PH_WDENS);
             if (Q.count > 0) {
                 k_st_scale<<<(unsigned)q_full, TEAM_THREADS, 0, st>>>(B, S, Q);
-                stage_tiles<ST_W, true>(B, S, Q, stage_counts(), st);
+                stage_tiles<ST_W, true, false>(B, S, Q, stage_counts(), st);
                 launches++;
             }
         });
@@ -2205,7 +2227,7 @@ extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_ove
                 e = cudaFuncSetAttribute((const void*)axg::k_density_static, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          axg::SMEM_WORK_BYTES);
             try {
-                stage_attributes();
+                stage_attributes(false);
                 for (int n = TRD_MIN_NAO; n <= STATIC_MAX_NAO; n++)
                     for (int g = 1; g <= 8; g *= 2)
                         CK(cudaFuncSetAttribute(axg::trd_class(n, g)->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2290,16 +2312,15 @@ extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_ove
         while (trd_smem_doubles(nao, G, 1, trd_class(nao, G)->cr, false) * 8 > TRD_SMEM_MAX) G *= 2;
         while (G < 8 && 16 * G <= nao) G *= 2;
         const TrdClass* cls = trd_class(nao, G);
-        const int cycles = 0;
         try {
             stage_cholesky(B, S, Q, P, nao, 0, on);
-            stage_transform(B, S, Q, c, on);
-            stage_reduce(cls->fn, G, 1, (int)(trd_smem_doubles(nao, G, 1, cls->cr, false) * 8), B, S, Q.mol, cycles, on);
-            k_st_tfac<<<(unsigned)c.rt, TEAM_THREADS, SMEM_WORK_BYTES, on>>>(B, S, Q, P);
-            stage_vectors(B, S, Q, P, c, on);
-            k_st_apply<8, 16><<<(unsigned)c.col, 512, st_apply_doubles(nao, 8) * 8, on>>>(B, S, Q, P, 0, nao);
-            stage_density(B, S, Q, c, on);
-            k_st_bisect<<<(unsigned)c.vec, ST_POINTS, 16 * (nao + 32), on>>>(B, S, Q, 1);
+            stage_transform<false>(B, S, Q, c, on);
+            stage_reduce(cls->fn, G, 1, (int)(trd_smem_doubles(nao, G, 1, cls->cr, false) * 8), B, S, Q.mol, nullptr, on);
+            k_st_tfac<false><<<(unsigned)c.rt, TEAM_THREADS, SMEM_WORK_BYTES, on>>>(B, S, Q, P);
+            stage_vectors<false>(B, S, Q, P, c, on);
+            k_st_apply<8, 16, false><<<(unsigned)c.col, 512, st_apply_doubles(nao, 8) * 8, on>>>(B, S, Q, P, 0, nao);
+            stage_density<false>(B, S, Q, c, on);
+            k_st_bisect<false><<<(unsigned)c.vec, ST_POINTS, 16 * (nao + 32), on>>>(B, S, Q, 1);
         } catch (const Fail& f) {
             g_last_error = std::string("axtb_gpu_density_static: launch: ") + f.what();
             return AXTB_ERR_DEVICE;

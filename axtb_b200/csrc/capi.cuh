@@ -519,7 +519,7 @@ int axtb_gpu_batch_profile(const AxtbBatch* b, char* buf, size_t len) {
         s += tmp;
         first = false;
     }
-    // SM-cycle shares of the eigen phase's parts (one-CTA teams)
+    // SM-cycle shares of the eigen phase's parts
     static const char* PH[8] = {"transform", "tridiagonal", "bisection", "fermi", "inverse_iteration",
                                 "back_transform", "c_matrix", "density"};
     // slots 8..13: parts of the tridiagonal reduction (counted instead of slot 1)

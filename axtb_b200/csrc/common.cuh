@@ -129,7 +129,7 @@ struct State {
     double *grad, *dedcn, *dedcn_d4;  // natT*3, natT, natT
     double* pair_buf;  // npairT*8: per atom-pair gradient partials
     double* e_atom;    // natT
-    double* mol_cyc;   // nmol: SM cycles of each molecule's last eigen phase (profiling runs)
+    double* mol_cyc;   // nmol: cycles of each molecule's last eigen phase, of half an SM (profiling runs)
     double* e_terms;   // natT*5: ES2, ES3, AES, D4 two-body, band per atom
     // implicit solvation: Born radii and dbrad/dpsi, surface areas, H-bond weights and their
     // surface derivative factors, self surface derivatives (natT*3), dE/dpsi, A_det per molecule,

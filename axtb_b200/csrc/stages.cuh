@@ -32,6 +32,33 @@ struct StagePlan {
     const int* width;            // ... and their width (8 or 24), per molecule
 };
 
+// Profiling runs (instances of the kernels with PROF): SM cycles of a stage's CTA into its molecule's counter
+// and the profiler's slot of the part (mol_eigen's slots), in units of the team kernel's half-SM CTAs (by
+// threads).
+template <bool PROF>
+__device__ __forceinline__ long long& stage_t0() {
+    __shared__ long long t0;
+    return t0;
+}
+template <bool PROF>
+__device__ __forceinline__ void stage_start() {
+    if constexpr (PROF)
+        if (threadIdx.x == 0) stage_t0<PROF>() = clock64();
+}
+template <bool PROF>
+__device__ __forceinline__ void stage_stop(const State& S, int m, int slot, int thread = 0) {
+    if constexpr (PROF)
+        if ((int)threadIdx.x == thread) {
+            const double c = (double)(clock64() - stage_t0<PROF>()) * blockDim.x / TEAM_THREADS;
+            atomicAdd(&S.mol_cyc[m], c);
+            atomicAdd(&g_team_cycles[slot], (unsigned long long)c);
+        }
+}
+__global__ void k_st_clear_cycles(State S, StagePlan Q) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < Q.count && S.active[Q.mol[i]]) S.mol_cyc[Q.mol[i]] = 0.0;
+}
+
 // triangular factors of the reflector blocks in the molecule's workspace (after the filling's part)
 __host__ __device__ constexpr long long stage_t_offset(int n) { return 32 + ((n + 31) & ~31); }
 
@@ -51,7 +78,7 @@ enum { ST_X = 0, ST_FP = 1, ST_C = 2, ST_P = 3, ST_W = 4 };
 // One 64 x 64 tile of X, F' or W in split precision per CTA (the team GEMM on a team of as many CTAs
 // as tiles: the same k-steps in the same order); W also gets its mirror image above the diagonal
 // (through shared memory, both stores coalesced).
-template <int MODE>
+template <int MODE, bool PROF>
 __global__ void __launch_bounds__(TEAM_THREADS, 2) k_st_tiles(Batch B, State S, StagePlan Q) {
     constexpr bool LOW = MODE != ST_X;
     const long long* off = LOW ? Q.off_low : Q.off_full;
@@ -70,7 +97,7 @@ __global__ void __launch_bounds__(TEAM_THREADS, 2) k_st_tiles(Batch B, State S, 
     }
     const Team t{bi + bj * rt, rt * rt, false};
     const double* Li = S.Linv + mat;
-    if (MODE == ST_X && t.rank == 0 && threadIdx.x == 0) S.mol_cyc[m] = 0.0;  // the profiler's, summed by k_trd
+    if (MODE != ST_W) stage_start<PROF>();
     if (MODE == ST_X) {
         team_gemm(t, false, false, n, n, n, 1.0, Li, n, S.F + mat, n, 0.0, S.scr1 + mat, n, GEMM_A_LOWER | GEMM_SPLIT);
     } else if (MODE == ST_FP) {
@@ -90,6 +117,7 @@ __global__ void __launch_bounds__(TEAM_THREADS, 2) k_st_tiles(Batch B, State S, 
             if (r < n && r > c) out[c + (long long)r * n] = s_work[(e / GT) * (GT + 1) + e % GT];
         }
     }
+    if (MODE != ST_W) stage_stop<PROF>(S, m, 0);
 }
 
 // The products in FP64, 32 x 32 tiles of four warps. Tiles of 64 (eight warps, two CTAs per SM) are
@@ -164,7 +192,7 @@ __device__ __forceinline__ void gemm_tile32(const Tile32& t, int row0, int col0,
     __syncthreads();
 }
 
-template <int MODE>
+template <int MODE, bool PROF>
 __global__ void __launch_bounds__(128) k_st_tiles32(Batch B, State S, StagePlan Q) {
     constexpr bool LOW = MODE == ST_FP || MODE == ST_P || MODE == ST_W;
     const long long* off = LOW ? Q.off_low32 : Q.off_full32;
@@ -183,7 +211,7 @@ __global__ void __launch_bounds__(128) k_st_tiles32(Batch B, State S, StagePlan 
     }
     const int k = MODE >= ST_C ? S.kocc[m] : n, row0 = bi * G32, col0 = bj * G32;
     if (MODE == ST_C && col0 >= k) return;
-    if (MODE == ST_X && tile == 0 && threadIdx.x == 0) S.mol_cyc[m] = 0.0;
+    if (MODE != ST_W) stage_start<PROF>();
     const double* Li = S.Linv + mat;
     double* out;
     Tile32 t;
@@ -219,6 +247,7 @@ __global__ void __launch_bounds__(128) k_st_tiles32(Batch B, State S, StagePlan 
                 out[r + (long long)c * n] = v;
                 if (MODE == ST_C) S.scr1[mat + r + (long long)c * n] = v * S.focc[ao0 + c];
             }
+    if (MODE != ST_W) stage_stop<PROF>(S, m, MODE == ST_C ? 6 : MODE == ST_P ? 7 : 0);
 }
 
 // scr1 = C (f e), the left factor of W
@@ -363,6 +392,7 @@ __device__ __forceinline__ int first_levels(const Batch& B, int m, int n) {
 // issue slots set the time of a single molecule). The SCF takes the lowest ceil(n_occ) + max(16,
 // n/16) and gives the others the Gershgorin bound; rest: those others (every orbital energy of the
 // result).
+template <bool PROF>
 __global__ void __launch_bounds__(ST_POINTS) k_st_bisect(Batch B, State S, StagePlan Q, int rest) {
     const int i = stage_find(Q.off_vec, Q.count, blockIdx.x), m = Q.mol[i];
     if (!rest && !S.active[m]) return;
@@ -370,21 +400,25 @@ __global__ void __launch_bounds__(ST_POINTS) k_st_bisect(Batch B, State S, Stage
     const int k0 = 32 * (int)(blockIdx.x - Q.off_vec[i]), k1 = min(n, k0 + 32);
     const int lo = rest ? max(k0, kc) : k0, hi = rest ? k1 : min(k1, kc);
     if (rest && lo >= hi) return;
+    if (!rest) stage_start<PROF>();
     double2* de = reinterpret_cast<double2*>(s_work);
     double g[3];
     int nb = cta_tridiagonal(S.dtri + ao0, S.etri + ao0, n, de, g);
     if (lo < hi) cta_levels(de, nb, g, lo, hi, S.emo + ao0);
     if (!rest)
         for (int k = max(k0, kc) + threadIdx.x; k < k1; k += blockDim.x) S.emo[ao0 + k] = g[1];
+    if (!rest) stage_stop<PROF>(S, m, 2);
 }
 
 // ---------------------------------------------------------------------------------- filling
 // tblite's Fermi filling (mol_fermi: the same sums in the same order; with equal spins the second
 // filling is the first, and a level with 0 or 1 electrons has no entropy). When the last computed
 // level still holds electrons, the CTA computes the others and fills again.
+template <bool PROF>
 __global__ void __launch_bounds__(TEAM_THREADS) k_st_fermi(Batch B, State S, StagePlan Q) {
     const int m = Q.mol[blockIdx.x];
     if (!S.active[m]) return;
+    stage_start<PROF>();
     const int n = B.m_nao[m], ao0 = B.m_ao0[m], lane = threadIdx.x & 31;
     const double na = B.m_nalpha[m], nbeta = B.m_nbeta[m];
     double* focc = S.focc + ao0;
@@ -447,6 +481,7 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_fermi(Batch B, State S, Sta
         for (int k0 = kc; k0 < n; k0 += 64) cta_levels(de, nb, g, k0, min(n, k0 + 64), S.emo + ao0);
         kc = n;
     }
+    stage_stop<PROF>(S, m, 3);
 }
 
 // ---------------------------------------------------------------------------------- vectors
@@ -478,12 +513,14 @@ __device__ __forceinline__ double invit_pivot(double pv, double floor) { return 
 __host__ __device__ constexpr int st_invit_bytes(int n) { return 8 * (2 * (n + 8) + 32 * 3 * 32); }
 __device__ __forceinline__ double* stage_norms(const TeamPlan& P, int m) { return P.wk + P.m_wk0[m] + 32; }
 
+template <bool PROF>
 __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, TeamPlan P, int part) {
     const int ti = stage_find(Q.off_vec, Q.count, blockIdx.x), m = Q.mol[ti];
     if (!S.active[m]) return;
     const int n = B.m_nao[m], ao0 = B.m_ao0[m], k = S.kocc[m];
     const int q = 32 * (int)(blockIdx.x - Q.off_vec[ti]) + threadIdx.x;
     if (q - (int)threadIdx.x >= k) return;
+    stage_start<PROF>();
     const long long mat = B.m_mat0[m], LD = n;
     const double* w = S.emo + ao0;
     double *sd = s_work, *se = s_work + n + 8;  // the tridiagonal matrix (e: two rows of zeros beyond)
@@ -493,10 +530,12 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
     }
     __syncwarp();
     const Clusters cl = warp_clusters(sd, se, n);
-    if (q >= k) return;
     // alone: no level close by, so nothing to be made orthogonal to, and part 0 takes both solves
-    const bool alone = !(q > 0 && w[q] - w[q - 1] <= cl.ctol) && !(q + 1 < k && w[q + 1] - w[q] <= cl.ctol);
-    if (part == 1 && alone) return;
+    const bool alone = q < k && !(q > 0 && w[q] - w[q - 1] <= cl.ctol) && !(q + 1 < k && w[q + 1] - w[q] <= cl.ctol);
+    const bool works = q < k && !(part == 1 && alone);
+    int first = 0;  // keeps the time
+    if constexpr (PROF) first = __ffs(__ballot_sync(0xffffffffu, works)) - 1;
+    if (!works) return;
     double* u0 = S.scr1 + mat + q;  // reciprocal pivots
     double* u1 = S.scr2 + mat + q;
     double* lm = S.scr3 + mat + q;
@@ -665,17 +704,20 @@ __global__ void __launch_bounds__(32) k_st_invit(Batch B, State S, StagePlan Q, 
         backward();
     }
     stage_norms(P, m)[q] = nrm;  // applied by whoever reads the vector next
+    stage_stop<PROF>(S, m, 4, first);
 }
 
 // Gram-Schmidt within the clusters (ascending, each vector against all earlier ones of its cluster,
 // then normalised), a warp per cluster: the warp of block q's 32 levels takes the clusters whose
 // first level lies there.
+template <bool PROF>
 __global__ void __launch_bounds__(32) k_st_gs(Batch B, State S, StagePlan Q, TeamPlan P) {
     const int ti = stage_find(Q.off_vec, Q.count, blockIdx.x), m = Q.mol[ti];
     if (!S.active[m]) return;
     const int n = B.m_nao[m], ao0 = B.m_ao0[m], k = S.kocc[m], lane = threadIdx.x;
     const int qb = 32 * (int)(blockIdx.x - Q.off_vec[ti]);
     if (qb >= k) return;
+    stage_start<PROF>();
     const double* w = S.emo + ao0;
     const Clusters cl = warp_clusters(S.dtri + ao0, S.etri + ao0, n);
     // heads: not close to the level below, close to the level above
@@ -731,6 +773,7 @@ __global__ void __launch_bounds__(32) k_st_gs(Batch B, State S, StagePlan Q, Tea
             }
         }
     }
+    stage_stop<PROF>(S, m, 4);
 }
 
 // ---------------------------------------------------------------------------------- back-transformation
@@ -738,11 +781,13 @@ constexpr int ST_NB = 64;  // reflectors per block
 
 // T of block b: H_{64 b} H_{64 b + 1} .. = I - V T V^T (T upper triangular; column c is
 // -tau_c T[0:c, 0:c] (V^T V)[0:c, c]), four threads per row
+template <bool PROF>
 __global__ void __launch_bounds__(TEAM_THREADS) k_st_tfac(Batch B, State S, StagePlan Q, TeamPlan P) {
     const int i = stage_find(Q.off_rt, Q.count, blockIdx.x), m = Q.mol[i];
     if (!S.active[m]) return;
     const int n = B.m_nao[m], b0 = ST_NB * (int)(blockIdx.x - Q.off_rt[i]), jb = min(ST_NB, n - 2 - b0);
     if (jb <= 0) return;
+    stage_start<PROF>();
     const double* V = S.Fp + B.m_mat0[m];
     double* T = P.wk + P.m_wk0[m] + stage_t_offset(n) + (long long)(b0 / ST_NB) * ST_NB * ST_NB;
     const Team t{0, 1, false};
@@ -768,6 +813,7 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_tfac(Batch B, State S, Stag
         __syncthreads();
     }
     for (int e = threadIdx.x; e < ST_NB * ST_NB; e += blockDim.x) T[e] = st[(e / ST_NB) * LT + e % ST_NB];
+    stage_stop<PROF>(S, m, 5);
 }
 
 // shared memory of k_st_apply (doubles): the columns, row by row, then three 64 x NC blocks. NC is 8
@@ -775,15 +821,16 @@ __global__ void __launch_bounds__(TEAM_THREADS) k_st_tfac(Batch B, State S, Stag
 __host__ __device__ constexpr long long st_apply_doubles(int n, int nc) { return (long long)((n + 7) / 8 * 8 + 3 * ST_NB) * nc; }
 // the most AOs whose columns fit so many bytes
 __host__ __device__ constexpr int st_apply_rows(int nc, int bytes) { return (bytes / 8 / nc - 3 * ST_NB) / 8 * 8; }
-static_assert(st_apply_doubles(st_apply_rows(24, TRD_SMEM_MAX), 24) * 8 <= TRD_SMEM_MAX &&
-              st_apply_doubles(st_apply_rows(24, TRD_SMEM_MAX) + 1, 24) * 8 > TRD_SMEM_MAX,
+constexpr int ST_SMEM_MAX = TRD_SMEM_MAX - 512;  // dynamic, of the stages' kernels (they have some of their own)
+static_assert(st_apply_doubles(st_apply_rows(24, ST_SMEM_MAX), 24) * 8 <= ST_SMEM_MAX &&
+              st_apply_doubles(st_apply_rows(24, ST_SMEM_MAX) + 1, 24) * 8 > ST_SMEM_MAX,
               "st_apply_rows is st_apply_doubles' inverse");
 
 // Z <- Q Z for NC columns, held in shared memory from the first block of reflectors to the last:
 // per block Y = V^T Z, Y <- T Y, Z -= V Y on the FP64 tensor cores, V straight from L2 into the
 // fragments. Y's sum over the rows runs in halves (row / 64 mod 2) of four interleaved chains (row / 4
 // mod 4), added in order: by 16 warps at once, or by 8 one half after the other (two CTAs per SM).
-template <int NC, int NW>
+template <int NC, int NW, bool PROF>
 __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1) k_st_apply(Batch B, State S, StagePlan Q, TeamPlan P, int n_lo, int n_hi) {
     constexpr int NT = NC / 8, LP = NC;
     static_assert(NC % 16 == 8, "row pitch");
@@ -791,6 +838,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1) k_st_apply(Batch B, 
     if (!S.active[m] || Q.width[ti] != NC) return;
     const int n = B.m_nao[m], k = S.kocc[m], c0 = NC * (int)(blockIdx.x - Q.off_col[ti]);
     if (c0 >= k || n <= n_lo || n > n_hi) return;  // another launch's molecules: each asks for its own shared memory
+    stage_start<PROF>();
     const long long mat = B.m_mat0[m];
     const int n8 = (n + 7) / 8 * 8, nrefl = n - 2;
     double* z = s_work;
@@ -899,6 +947,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 1) k_st_apply(Batch B, 
         int r = e % n, c = e / n;
         if (c0 + c < k) S.Z[mat + r + (long long)(c0 + c) * n] = z[r * LP + c];
     }
+    stage_stop<PROF>(S, m, 5);
 }
 
 }  // namespace axg

@@ -553,15 +553,20 @@ __device__ __forceinline__ bool trd_mol(int rank, int G, int n, double* __restri
     return ok;
 }
 
-// SM cycles of the reduction into the molecule's counter (in units of the team kernel's half-SM CTAs)
-__device__ __forceinline__ void trd_cycles(const State& S, int m, int rank, int G, long long t0) {
-    if (rank == 0 && threadIdx.x == 0) S.mol_cyc[m] += 2.0 * G * (double)(clock64() - t0);
+// SM cycles of the reduction into the molecule's counter and the profiler's slot (nullptr: not profiling), in
+// units of the team kernel's half-SM CTAs
+__device__ __forceinline__ void trd_cycles(const State& S, int m, int rank, int G, long long t0, unsigned long long* slot) {
+    if (rank == 0 && threadIdx.x == 0) {
+        const double c = 2.0 * G * (double)(clock64() - t0);
+        S.mol_cyc[m] += c;
+        atomicAdd(slot, (unsigned long long)c);
+    }
 }
 
 // One cluster per molecule of `list` (one-CTA-team molecules of the batch), CTAs of a cluster by
 // their rank. Launched per size class with the class's row slots and cluster size.
 template <int RT, int CR>
-__global__ void __launch_bounds__(TRD_THREADS, 1) k_trd(Batch B, State S, const int* list, int cycles) {
+__global__ void __launch_bounds__(TRD_THREADS, 1) k_trd(Batch B, State S, const int* list, unsigned long long* cycles) {
     const long long t0 = clock64();
     unsigned rank, G;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -572,19 +577,19 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_trd(Batch B, State S, const 
     if (!trd_mol<RT, CR, 1, false>((int)rank, (int)G, n, S.Fp + B.m_mat0[m], S.dtri + ao0, S.etri + ao0, S.tau + ao0,
                                    nullptr, &S.status[m]))
         atomicOr(&S.status[m], ST_TIMEOUT);
-    if (cycles) trd_cycles(S, m, (int)rank, (int)G, t0);
+    if (cycles) trd_cycles(S, m, (int)rank, (int)G, t0, cycles);
 }
 
 // One molecule on the whole cooperative grid (every CTA resident, as its waits need); xpub: 4 n doubles and a count, zero
 template <int RT, int CR>
-__global__ void __launch_bounds__(TRD_THREADS, 1) k_trd_grid(Batch B, State S, int m, double* xpub, int cycles) {
+__global__ void __launch_bounds__(TRD_THREADS, 1) k_trd_grid(Batch B, State S, int m, double* xpub, unsigned long long* cycles) {
     const long long t0 = clock64();
     if (!S.active[m]) return;  // uniform over the grid
     const int n = B.m_nao[m], ao0 = B.m_ao0[m];
     if (!trd_mol<RT, CR, 8, true>((int)blockIdx.x, (int)gridDim.x, n, S.Fp + B.m_mat0[m], S.dtri + ao0, S.etri + ao0,
                                   S.tau + ao0, xpub, &S.status[m]))
         atomicOr(&S.status[m], ST_TIMEOUT);
-    if (cycles) trd_cycles(S, m, (int)blockIdx.x, (int)gridDim.x, t0);
+    if (cycles) trd_cycles(S, m, (int)blockIdx.x, (int)gridDim.x, t0, cycles);
 }
 
 // One molecule of `list` per team, gridDim.y teams of gridDim.x CTAs; xpub: `stride` doubles per entry of the
@@ -592,7 +597,7 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_trd_grid(Batch B, State S, i
 // parameters the one above took 16.4 ms instead of 16.0 at 2400 AOs.
 template <int RT, int CR>
 __global__ void __launch_bounds__(TRD_THREADS, 1)
-    k_trd_teams(Batch B, State S, const int* list, double* xpub, long long stride, int cycles) {
+    k_trd_teams(Batch B, State S, const int* list, double* xpub, long long stride, unsigned long long* cycles) {
     const long long t0 = clock64();
     const int m = list[blockIdx.y];
     if (!S.active[m]) {  // uniform over the team; the other teams' grid barrier counts these CTAs too
@@ -603,7 +608,7 @@ __global__ void __launch_bounds__(TRD_THREADS, 1)
     if (!trd_mol<RT, CR, 8, true>((int)blockIdx.x, (int)gridDim.x, n, S.Fp + B.m_mat0[m], S.dtri + ao0, S.etri + ao0,
                                   S.tau + ao0, xpub + blockIdx.y * stride, &S.status[m]))
         atomicOr(&S.status[m], ST_TIMEOUT);
-    if (cycles) trd_cycles(S, m, (int)blockIdx.x, (int)gridDim.x, t0);
+    if (cycles) trd_cycles(S, m, (int)blockIdx.x, (int)gridDim.x, t0, cycles);
 }
 
 }  // namespace axg

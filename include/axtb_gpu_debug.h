@@ -25,7 +25,8 @@ enum AxtbDebugQuantity {
     AXTB_DBG_WDENSITY = 9,    /* nao*nao energy-weighted density (after a gradient run) */
     AXTB_DBG_EEQ = 10,        /* nat EEQ start charges */
     AXTB_DBG_LINV = 11,       /* nao*nao inverse Cholesky factor of the overlap */
-    AXTB_DBG_EIGEN_CYCLES = 12, /* 1 value: SM clock cycles of the molecule's last eigen phase
+    AXTB_DBG_EIGEN_CYCLES = 12, /* 1 value: clock cycles of the molecule's last eigen phase, in units of
+                                   half a multiprocessor, all of its stages' CTAs together
                                    (runs with profiling on; 0 otherwise) */
     AXTB_DBG_STATUS_BITS = 13,  /* 1 value: the molecule's raw status bits of its last attempt
                                    (1 overlap/EEQ not positive definite, 2 non-finite energy,

@@ -22,3 +22,24 @@ def _two_stage(engine, waters, **options):
     (16, 97, True), (130, 1 << 20, True), (6, 33, False), (7, 0, False), (6, 64, False), (10, -1, False)])
 def test_band_max_nao(engine, waters, threshold, expected):
     assert _two_stage(engine, waters, band_max_nao=threshold) is expected
+
+
+def test_cycles_cover_the_whole_eigen_phase(engine):
+    """The profiler's shares have every part of a staged molecule's eigen phase, and the molecules' own
+    counters (the last iteration) add up to no more than all iterations' parts, the reduction being one of
+    them."""
+    from axtb_b200 import structures as S
+
+    mols = [S.water_cluster(k, seed=k) for k in (2, 10, 40, 140)]  # 12 to 840 AOs: clusters and the grid
+    b = engine.Batch(mols, accuracy=1.0)
+    b.run(gradient=False)
+    assert all(b.debug(i, "eigen_cycles")[0] == 0.0 for i in range(4))
+    b.set_profiling(True)
+    assert all(r.status == 0 for r in b.run(gradient=True, levels=True))
+    p = b.profile()
+    shares = p["team_eigen_phases"]
+    assert abs(sum(shares.values()) - 1.0) < 1e-3
+    for part in ("transform", "tridiagonal", "bisection", "inverse_iteration", "back_transform", "c_matrix", "density"):
+        assert shares[part] > 0.0, shares
+    cycles = [float(b.debug(i, "eigen_cycles")[0]) for i in range(4)]
+    assert all(x < y for x, y in zip(cycles, cycles[1:])) and cycles[0] > 0.0

@@ -51,3 +51,11 @@ def test_kernels_that_need_the_whole_gpu_share_one_stream(engine):
         assert chain == sorted(chain) and len({s for k, s in steps if k in chain}) <= 1
         if grid_mols:  # before the fork: the side stream's kernels start after it
             assert order[0] == TEAM_GRID
+
+
+def test_autotune_times_distinct_schedules():
+    from axtb_b200.autotune import band_candidates
+
+    assert band_candidates(0) == band_candidates(32) == [64]  # no molecule of 34 AOs or more below 32
+    assert band_candidates(64) == [64, 65]
+    assert band_candidates(160) == [64, 160]
