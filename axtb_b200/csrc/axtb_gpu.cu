@@ -560,22 +560,23 @@ AxtbBatch::~AxtbBatch() {
 }
 
 // ---- launches of the stages (stages.cuh, stages_chol.cuh, trd.cuh), shared by the batch engine and
-// the allocation-free entry point
+// the allocation-free entry point; each returns how many kernels it launched
 struct StageCounts {  // tasks; nmax: the largest matrix
     int nmax;
     long long full, low, rt, vec, col, full32, low32;
 };
 // the products of a stage; in split precision X, F' and W keep the 64 x 64 tiles that have it
 template <int MODE, bool LOW, bool PROF>
-static void stage_tiles(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
+static int stage_tiles(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                         cudaStream_t st) {
     using namespace axg;
     if constexpr (MODE != ST_C && MODE != ST_P)
         if (B.split) {
             k_st_tiles<MODE, PROF><<<(unsigned)(LOW ? c.low : c.full), TEAM_THREADS, SMEM_WORK_BYTES, st>>>(B, S, Q);
-            return;
+            return 1;
         }
     k_st_tiles32<MODE, PROF><<<(unsigned)(LOW ? c.low32 : c.full32), 128, GSTAGES * G32_STAGE * 8, st>>>(B, S, Q);
+    return 1;
 }
 template <bool PROF>
 static void stage_attributes_of() {
@@ -596,11 +597,10 @@ static void stage_attributes(bool profiling) {
 }
 // F' = L^-1 F L^-T
 template <bool PROF>
-static void stage_transform(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
+static int stage_transform(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                             cudaStream_t st) {
     using namespace axg;
-    stage_tiles<ST_X, false, PROF>(B, S, Q, c, st);
-    stage_tiles<ST_FP, true, PROF>(B, S, Q, c, st);
+    return stage_tiles<ST_X, false, PROF>(B, S, Q, c, st) + stage_tiles<ST_FP, true, PROF>(B, S, Q, c, st);
 }
 // count reductions of one class on clusters of G CTAs
 static void stage_reduce(const void* fn, int G, int count, int smem, const axg::Batch& B, const axg::State& S, const int* list,
@@ -621,7 +621,7 @@ static void stage_reduce(const void* fn, int G, int count, int smem, const axg::
 }
 // levels, filling and vectors of the tridiagonal matrices
 template <bool PROF>
-static void stage_vectors(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P,
+static int stage_vectors(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P,
                           const StageCounts& c, cudaStream_t st) {
     using namespace axg;
     k_st_bisect<PROF><<<(unsigned)c.vec, ST_POINTS, 16 * (c.nmax + 32), st>>>(B, S, Q, 0);
@@ -630,27 +630,33 @@ static void stage_vectors(const axg::Batch& B, const axg::State& S, const axg::S
         k_st_invit<PROF><<<(unsigned)c.vec, 32, st_invit_bytes(c.nmax), st>>>(B, S, Q, P, part);
         k_st_gs<PROF><<<(unsigned)c.vec, 32, 0, st>>>(B, S, Q, P);
     }
+    return 6;
 }
 // C = L^-T Z and P = (C f) C^T
 template <bool PROF>
-static void stage_density(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
+static int stage_density(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const StageCounts& c,
                           cudaStream_t st) {
     using namespace axg;
-    stage_tiles<ST_C, false, PROF>(B, S, Q, c, st);
-    stage_tiles<ST_P, true, PROF>(B, S, Q, c, st);
+    return stage_tiles<ST_C, false, PROF>(B, S, Q, c, st) + stage_tiles<ST_P, true, PROF>(B, S, Q, c, st);
 }
 // factor and inverse factor of the overlap matrices, or of the EEQ matrices; nmax: the largest
-static void stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P, int nmax,
+static int stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P, int nmax,
                            int eeq, cudaStream_t st) {
     using namespace axg;
     const int W = SMEM_WORK_BYTES, T = TEAM_THREADS, rt = (nmax + CB - 1) / CB;
     const unsigned cnt = (unsigned)Q.count;
+    int launched = 1;
     k_ch_init<<<dim3(rt * rt, cnt), T, W, st>>>(B, S, Q, P, eeq);
     for (int p = 0; p < rt && rt > 1; p++) {
         k_ch_panel<<<dim3(rt - 1, cnt), T, W, st>>>(B, S, Q, P, p, eeq);
+        launched++;
         const int left = rt - 1 - p;
-        if (left > 0) k_ch_trail<<<dim3(left * (left + 1) / 2, cnt), T, W, st>>>(B, S, Q, P, p, eeq);
+        if (left > 0) {
+            k_ch_trail<<<dim3(left * (left + 1) / 2, cnt), T, W, st>>>(B, S, Q, P, p, eeq);
+            launched++;
+        }
     }
+    return launched;
 }
 
 // Which molecules' eigen phase runs in stages with the reduction on chip (stages.cuh, trd.cuh): from
@@ -824,14 +830,14 @@ void AxtbBatch::launch_stages() {
         k_st_clear_cycles<<<(Q.count + 255) / 256, 256, 0, st>>>(S, Q);
         launches++;
     }
-    stage_transform<PROF>(B, S, Q, cnt, st);
+    launches += stage_transform<PROF>(B, S, Q, cnt, st);
     launch_trd();
     // the reflectors' triangular factors beside the levels and vectors of the tridiagonal matrices
     CK(cudaEventRecord(fac_ev[0], st));
     CK(cudaStreamWaitEvent(fac_st, fac_ev[0], 0));
     k_st_tfac<PROF><<<(unsigned)q_rt, TEAM_THREADS, SMEM_WORK_BYTES, fac_st>>>(B, S, Q, P);
     CK(cudaEventRecord(fac_ev[1], fac_st));
-    stage_vectors<PROF>(B, S, Q, P, cnt, st);
+    launches += stage_vectors<PROF>(B, S, Q, P, cnt, st);
     CK(cudaStreamWaitEvent(st, fac_ev[1], 0));
     for (const ApplyLaunch& a : q_apply) {
         const void* fn = a.width == 8 ? (const void*)k_st_apply<8, 16, PROF> : a.warps == 8 ? (const void*)k_st_apply<24, 8, PROF> : (const void*)k_st_apply<24, 16, PROF>;
@@ -839,8 +845,7 @@ void AxtbBatch::launch_stages() {
         CK(cudaLaunchKernel(fn, dim3((unsigned)q_col), dim3(32 * a.warps), args, st_apply_doubles(a.hi, a.width) * 8, st));
         launches++;
     }
-    stage_density<PROF>(B, S, Q, cnt, st);
-    launches += 11;
+    launches += stage_density<PROF>(B, S, Q, cnt, st) + 1;  // and k_st_tfac
     CK(cudaGetLastError());
 }
 
@@ -849,14 +854,12 @@ void AxtbBatch::launch_stages() {
 void AxtbBatch::launch_cholesky(int eeq) {
     using namespace axg;
     const int T = TEAM_THREADS;
-    const int rt = ((eeq ? q_natmax : q_nmax) + CB - 1) / CB;
     for (int c0 = 0; c0 < Q.count; c0 += 65535) {  // molecules along the grid's y
         StagePlan q = Q;
         q.mol = Q.mol + c0;
         const unsigned cnt = (unsigned)std::min(65535, Q.count - c0);
         q.count = (int)cnt;
-        stage_cholesky(B, S, q, P, eeq ? q_natmax : q_nmax, eeq, st);
-        launches += 2 * rt;
+        launches += stage_cholesky(B, S, q, P, eeq ? q_natmax : q_nmax, eeq, st);
         if (eeq) {
             k_ch_eeq<<<dim3((q_natmax + 31) / 32, cnt), T, 0, st>>>(B, S, q, P, 0);
             k_ch_eeq<<<dim3((q_natmax + 7) / 8, cnt), T, 0, st>>>(B, S, q, P, 1);
@@ -1825,7 +1828,6 @@ void AxtbBatch::upload_positions(const double* x, bool device_ptr) {
 // resolved after the run; with the algorithmic work of each launch (FLOPs of the dense algebra,
 // bytes of the matrix passes) for the roofline report.
 void AxtbBatch::begin_launch(const char* name, double flops, double bytes) {
-    launches++;
     if (!profiling) return;
     Rec r;
     r.name = name;
@@ -1877,11 +1879,16 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     }
     const int T = 256;
     long long nn = nnT;
-#define LAUNCH(name, flops, bytes, ...)  \
+#define PHASE(name, flops, bytes, ...)   /* kernels that count themselves */ \
     do {                                 \
         begin_launch(name, flops, bytes); \
         __VA_ARGS__;                     \
         end_launch();                    \
+    } while (0)
+#define LAUNCH(name, flops, bytes, ...)  /* one kernel */ \
+    do {                                 \
+        PHASE(name, flops, bytes, __VA_ARGS__); \
+        launches++;                      \
     } while (0)
     // algorithmic work of the matrix passes over the molecules in `act` (1 = included)
     auto mat_bytes = [&](const vector<int>& act, double per_n2) {
@@ -1976,6 +1983,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         Psmall = P;
         Psmall.nbig = 0;
         CK(cudaLaunchKernel((void*)k_team, grid, TEAM_THREADS, args_small, SMEM_WORK_BYTES, on));
+        launches++;
     };
     auto team_launch = [&](int phase) {
         if (P.nbig > 0) team_grid_launch(phase);
@@ -1984,7 +1992,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     const vector<EigenStep> eigen = eigen_steps(P.nbig > 0, nteam_eigen > 0, nchase > 0, Q.count > 0);
     double chol_flops = 0.0;
     for (int m = 0; m < nmol; m++) chol_flops += (1.0 / 3.0 + 2.0 / 3.0) * std::pow((double)mols[m].nao, 3.0);
-    LAUNCH("team_overlap", chol_flops, 0, {
+    PHASE("team_overlap", chol_flops, 0, {
         if (nteam_eigen > 0) team_launch(PH_OVERLAP);
         if (Q.count > 0) launch_cholesky(0);
     });
@@ -1995,7 +2003,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         LAUNCH("eeq_matrix", 0, 0, k_eeq_matrix<<<blocks_for(nsqT, T), T, 0, st>>>(B, S, d_sq0, P.eeq_rhs, nsqT));
         double f = 0.0;
         for (int m = 0; m < nmol; m++) f += 3.0 * std::pow((double)mols[m].nat, 3.0);
-        LAUNCH("team_eeq", f, 0, {
+        PHASE("team_eeq", f, 0, {
             if (nteam_eigen > 0) team_launch(PH_EEQ);
             if (Q.count > 0) launch_cholesky(1);
         });
@@ -2014,7 +2022,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
                 LAUNCH("solv_potential", 0, 0, k_solv_potential<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));
             LAUNCH("fock", 0, mat_bytes(act, 12.0), k_fock<<<(unsigned)ntiles, T, 0, st>>>(B, S, d_tile0, ntiles));
             // the eigen phase: one launch, or three when k_chase takes stage 2 of some molecules
-            LAUNCH("team_eigen", eig_flops(act), 0, {
+            PHASE("team_eigen", eig_flops(act), 0, {
                 bool forked = false;
                 for (const EigenStep& step : eigen) {
                     if (step.side && !forked) {
@@ -2032,10 +2040,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
                             CK(cudaGetLastError());
                             launches++;
                             break;
-                        case EK_TEAM_TAIL:
-                            team_cta_launch(PH_EIGEN_TAIL, x);
-                            launches++;
-                            break;
+                        case EK_TEAM_TAIL: team_cta_launch(PH_EIGEN_TAIL, x); break;
                         case EK_STAGES: P.cycles ? launch_stages<true>() : launch_stages<false>(); break;
                     }
                 }
@@ -2098,19 +2103,21 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         CK(cudaMemcpyAsync(S.have_guess, S.conv, sizeof(int) * nmol, cudaMemcpyDeviceToDevice, st));
     }
     if (want_levels) {
-        LAUNCH("team_levels", 0, 0, {
+        PHASE("team_levels", 0, 0, {
             if (nteam_eigen > 0) team_launch(PH_LEVELS);
-            if (Q.count > 0) k_st_bisect<false><<<(unsigned)q_vec, ST_POINTS, 16 * (q_nmax + 32), st>>>(B, S, Q, 1);
+            if (Q.count > 0) {
+                k_st_bisect<false><<<(unsigned)q_vec, ST_POINTS, 16 * (q_nmax + 32), st>>>(B, S, Q, 1);
+                launches++;
+            }
         });
     }
     CK(cudaEventRecord(phase_ev[2], st));
     if (want_grad) {
-        LAUNCH("team_wdens", w_flops(all), 0, {
+        PHASE("team_wdens", w_flops(all), 0, {
             if (nteam_eigen > 0) team_launch(PH_WDENS);
             if (Q.count > 0) {
                 k_st_scale<<<(unsigned)q_full, TEAM_THREADS, 0, st>>>(B, S, Q);
-                stage_tiles<ST_W, true, false>(B, S, Q, stage_counts(), st);
-                launches++;
+                launches += 1 + stage_tiles<ST_W, true, false>(B, S, Q, stage_counts(), st);
             }
         });
         if (B.output_aes)
@@ -2132,6 +2139,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
         LAUNCH("cn_chain", 0, 0, k_cn_chain<<<blocks_for((long long)natT * 32, T), T, 0, st>>>(B, S));
     }
 #undef LAUNCH
+#undef PHASE
     CK(cudaEventRecord(phase_ev[3], st));
     CK(cudaGetLastError());
     resolve_profile();

@@ -43,3 +43,26 @@ def test_cycles_cover_the_whole_eigen_phase(engine):
         assert shares[part] > 0.0, shares
     cycles = [float(b.debug(i, "eigen_cycles")[0]) for i in range(4)]
     assert all(x < y for x, y in zip(cycles, cycles[1:])) and cycles[0] > 0.0
+
+
+@pytest.mark.parametrize("waters, options", [
+    ([1], {}), ([2, 10, 40], {}), ([1, 11, 60, 130, 140], {}), ([6, 10, 20], {"band_max_nao": 80}),
+    ([3, 5], {"solvation": ("alpb", "water")}), ([12, 30], {"precision": "split", "guess": "sad"}), ([20], {"mixer": "diis"})])
+def test_launches_are_those_of_the_run(engine, waters, options):
+    """The number of launches of a run is that of its kernels in the profiler's trace (CUPTI)."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    from axtb_b200 import structures as S
+
+    b = engine.Batch([S.water_cluster(k, seed=k) for k in waters], accuracy=1.0, **options)
+    for gradient, levels in ((True, True), (False, False)):
+        b.run(gradient=gradient, levels=levels)
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            b.run(gradient=gradient, levels=levels)
+            torch.cuda.synchronize()
+        kernels = [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA and "axg::" in e.name]
+        if not kernels:
+            pytest.skip("no kernel in the profiler's trace on this machine")
+        assert b.launches == len(kernels)
+    b.close()
