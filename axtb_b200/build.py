@@ -5,6 +5,7 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
@@ -30,19 +31,20 @@ def sources():
 def build(force: bool = False) -> Path:
     if not force and OUT.exists() and OUT.stat().st_mtime >= max(p.stat().st_mtime for p in sources()):
         return OUT
-    tmp = OUT.with_suffix(".so.tmp")
-    objs = [OUT.parent / (p.stem + ".o") for p in (SRC, TRD)]
-    flags = [f for f in FLAGS if f != "-shared"]
-    jobs = [subprocess.Popen([nvcc(), *flags, "-c", "-o", str(o), str(p)]) for p, o in zip((SRC, TRD), objs)]
-    for job in jobs:
-        job.wait()
-    for job in jobs:
-        if job.returncode:
-            raise subprocess.CalledProcessError(job.returncode, job.args)
-    subprocess.run([nvcc(), *FLAGS, "-o", str(tmp), *map(str, objs)], check=True)
-    for o in objs:
-        o.unlink()
-    tmp.replace(OUT)
+    # objects and library in a folder of this call's own: several processes may build at once, each its own
+    # whole library, the last of which stays
+    with tempfile.TemporaryDirectory(prefix=".build", dir=OUT.parent) as work:
+        objs = [Path(work) / (p.stem + ".o") for p in (SRC, TRD)]
+        flags = [f for f in FLAGS if f != "-shared"]
+        jobs = [subprocess.Popen([nvcc(), *flags, "-c", "-o", str(o), str(p)]) for p, o in zip((SRC, TRD), objs)]
+        for job in jobs:
+            job.wait()
+        for job in jobs:
+            if job.returncode:
+                raise subprocess.CalledProcessError(job.returncode, job.args)
+        tmp = Path(work) / OUT.name
+        subprocess.run([nvcc(), *FLAGS, "-o", str(tmp), *map(str, objs)], check=True)
+        tmp.replace(OUT)
     return OUT
 
 
