@@ -51,3 +51,14 @@ def test_builds_at_once_do_not_share_objects(tmp_path, monkeypatch):
     assert set(seen) <= {"first first ", "second second "} and len(seen) == 2
     assert sorted(os.listdir(tmp_path)) == ["first", "libaxtb_gpu.so", "second"]
     assert isinstance(B.OUT, Path)
+
+
+def test_documented_command_is_the_build(engine):
+    """The nvcc command that the integration guide gives has the build's flags and sources."""
+    from axtb_b200 import build as B
+
+    root = Path(B.__file__).resolve().parent.parent
+    words = next(line for line in (root / "INTEGRATION.md").read_text().splitlines() if line.startswith("`nvcc ")).strip("`)").split()
+    assert words[0] == "nvcc" and set(B.FLAGS) <= set(words)
+    assert [w for w in words if w.endswith(".cu")] == [str(p.relative_to(root)) for p in (B.SRC, B.TRD)]
+    assert words[words.index("-o") + 1] == str(B.OUT.relative_to(root))
