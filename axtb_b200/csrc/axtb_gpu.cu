@@ -313,7 +313,6 @@ struct Opt {
 // band_max_nao of 64, as -1, is the default: no two-stage reduction where the one on chip holds the
 // molecule. Any other asks for the two-stage reduction of molecules of 34 AOs up to below it.
 constexpr int DEFAULT_BAND_MAX_NAO = 64;
-constexpr int STATIC_BAND_MAX_NAO = 64;
 constexpr int DEFAULT_GRID_MIN_NAO = 1024;
 
 // ------------------------------------------------------------------ solvation parameters
@@ -2147,8 +2146,8 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
 
 // ------------------------------------------------------------------ allocation-free density
 // Eigenvalues, Fermi occupations and density of one molecule from its Fock and overlap
-// matrices (the team kernel's overlap and eigen phases on one CTA) with every scratch buffer in
-// one file-scope device array instead of memory from cudaMalloc: for callers that cannot
+// matrices (the batch engine's stages; below TRD_MIN_NAO basis functions the team kernel's phases on one
+// CTA) with every scratch buffer in one file-scope device array instead of memory from cudaMalloc: for callers that cannot
 // allocate device memory themselves (code running inside another framework's stream-ordered
 // memory pool or under a fixed device-memory budget, where a cudaMalloc would fail or would
 // synchronise the device and stall unrelated work). The array exists once per device for as
@@ -2156,21 +2155,20 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
 namespace {
 constexpr int STATIC_MAX_NAO = 256;
 constexpr long long STATIC_PLANE = (long long)STATIC_MAX_NAO * STATIC_MAX_NAO;  // doubles per matrix
-constexpr long long STATIC_WK = axg::team_workspace(STATIC_MAX_NAO);             // team workspace
-static_assert(STATIC_WK >= axg::band_workspace(STATIC_MAX_NAO) && STATIC_WK >= axg::onestage_workspace(STATIC_MAX_NAO),
-              "the static workspace holds the eigen phase's layout at the largest molecule");
+constexpr long long STATIC_WK =                                                  // workspace of either
+    std::max(axg::stage_workspace(STATIC_MAX_NAO), axg::onestage_workspace(TRD_MIN_NAO - 1));
 constexpr long long STATIC_VEC = 8LL * STATIC_MAX_NAO;                           // d, e, tau + spare
 constexpr long long STATIC_PIV = STATIC_PLANE / 8;                               // pivot bytes, as doubles
 constexpr long long STATIC_PAR = 128;                                            // small parameters
-constexpr long long STATIC_DOUBLES = 8 * STATIC_PLANE + STATIC_WK + STATIC_VEC + STATIC_PIV + STATIC_PAR;
-static __device__ __align__(256) double g_density_scratch[STATIC_DOUBLES];  // 4.89 MiB
+constexpr long long STATIC_DOUBLES = 7 * STATIC_PLANE + STATIC_WK + STATIC_VEC + STATIC_PIV + STATIC_PAR;
+static __device__ __align__(256) double g_density_scratch[STATIC_DOUBLES];  // 3.77 MiB
 
 std::mutex g_static_mu;
 double* g_static_addr[256] = {nullptr};
 }  // namespace
 
 namespace axg {
-// parameters into the static area (one thread); off: the stages' task offsets, {0, count} each
+// parameters into the static area (one thread)
 __device__ void density_static_setup(const Batch& B, State& S, const TeamPlan& P, int nao, double nalpha, double nbeta) {
     *const_cast<int*>(B.m_nao) = nao;
     *const_cast<int*>(B.m_ao0) = 0;
@@ -2267,7 +2265,6 @@ extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_ove
     S.C = take(STATIC_PLANE);
     S.scr2 = take(STATIC_PLANE);
     S.scr3 = take(STATIC_PLANE);
-    S.W = take(STATIC_PLANE);  // the band reduction's second-stage reflectors
     P.wk = take(STATIC_WK);
     double* vec = take(STATIC_VEC);
     S.dtri = vec;
@@ -2292,8 +2289,7 @@ extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_ove
     S.P = d_density;
     B.nmol = 1;
     B.kt = kt;
-    B.band_max = STATIC_BAND_MAX_NAO;
-    B.chase_max = 0;  // stage 2 in this kernel
+    B.band_max = B.chase_max = 0;  // no molecule of the one CTA's is large enough for two stages
     cudaStream_t on = (cudaStream_t)stream;
     if (nao < TRD_MIN_NAO) {
         axg::k_density_static<<<1, axg::TEAM_THREADS, axg::SMEM_WORK_BYTES, on>>>(B, S, P, nao, nalpha, nbeta, d_status);

@@ -61,6 +61,11 @@ __global__ void k_st_clear_cycles(State S, StagePlan Q) {
 
 // triangular factors of the reflector blocks in the molecule's workspace (after the filling's part)
 __host__ __device__ constexpr long long stage_t_offset(int n) { return 32 + ((n + 31) & ~31); }
+// workspace of a molecule's stages (doubles): the filling's part and the factors (64 x 64 per block of 64)
+__host__ __device__ constexpr long long stage_workspace(int n) { return stage_t_offset(n) + (n + 63) / 64 * 4096LL; }
+static_assert(stage_workspace(12) <= team_workspace(12) && stage_workspace(256) <= team_workspace(256) &&
+                  stage_workspace(2405) <= team_workspace(2405),
+              "a molecule's workspace has the team kernel's size");
 
 __device__ __forceinline__ int stage_find(const long long* off, int count, long long task) {
     int lo = 0, hi = count - 1;
