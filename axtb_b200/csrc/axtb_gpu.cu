@@ -1968,9 +1968,6 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     int ph = PH_OVERLAP;
     args[3] = &ph;
     // a team phase: the whole-grid molecules in their own launch (k_team_grid), then the rest
-    TeamPlan Psmall = P;
-    Psmall.nbig = 0;
-    void* args_small[] = {&B, &S, &Psmall, &ph};
     // (no one-CTA molecule needs the others' CTAs: a plain launch, which shares the GPU)
     auto team_grid_launch = [&](int phase) {
         ph = phase;
@@ -1979,9 +1976,7 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     };
     auto team_cta_launch = [&](int phase, cudaStream_t on) {
         ph = phase;
-        Psmall = P;
-        Psmall.nbig = 0;
-        CK(cudaLaunchKernel((void*)k_team, grid, TEAM_THREADS, args_small, SMEM_WORK_BYTES, on));
+        CK(cudaLaunchKernel((void*)k_team, grid, TEAM_THREADS, args, SMEM_WORK_BYTES, on));
         launches++;
     };
     auto team_launch = [&](int phase) {

@@ -320,11 +320,6 @@ __device__ void run_mol(const Team& t, const Batch& B, State& S, const TeamPlan&
 __global__ void __launch_bounds__(TEAM_THREADS, 2) k_team(Batch B, State S, TeamPlan P, int phase) {
     if (threadIdx.x == 0) s_team_gen = 0;
     __syncthreads();
-    Team g{(int)blockIdx.x, (int)gridDim.x, true};
-    for (int i = 0; i < P.nbig; i++) {
-        int m = P.big[i];
-        if (phase_wants(B, S, phase, m)) run_mol<false>(g, B, S, P, phase, m);  // uniform across the grid
-    }
     Team one{0, 1, false};
     const int* off = phase == PH_EIGEN ? P.head_off : phase == PH_EIGEN_TAIL ? P.tail_off : P.small_off;
     const int* list = phase == PH_EIGEN ? P.head_list : phase == PH_EIGEN_TAIL ? P.tail_list : P.small_list;
@@ -335,8 +330,8 @@ __global__ void __launch_bounds__(TEAM_THREADS, 2) k_team(Batch B, State S, Team
 }
 
 // The whole-grid molecules (P.big) of a phase, one after the other on the whole cooperative grid.
-// A batch that holds such molecules runs this launch first and then k_team for the rest (with
-// nbig = 0): the grid path gets its own instance of the dense algebra, and the one-CTA path's
+// A batch that holds such molecules runs this launch first and then k_team for the rest: the grid
+// path gets its own instance of the dense algebra, and the one-CTA path's
 // kernel is compiled without the grid-only code.
 __global__ void __launch_bounds__(TEAM_THREADS, 2) k_team_grid(Batch B, State S, TeamPlan P, int phase) {
     if (threadIdx.x == 0) s_team_gen = 0;
