@@ -667,14 +667,15 @@ static int stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::S
 // molecule's size alone, and so are its bits. One CTA per molecule, the other way for 769 to 1023 AOs, takes
 // 167 / 201 / 224 ms per eigen phase for 65 / 148 / 296 molecules of 780 AOs and 344 / 399 / 436 at 1020; the
 // grid's teams take 55 / 117 / 228 and 104 / 227 / 454. A band_max_nao other than the default asks for the
-// two-stage reduction below it (DEFAULT_BAND_MAX_NAO).
+// two-stage reduction below it (DEFAULT_BAND_MAX_NAO). AXTB_EIGEN_TEAM=1 leaves all molecules to the team
+// kernels, for their tests.
 constexpr int TRD_MIN_NAO = 12;
 void AxtbBatch::plan_trd(int big_nao, int band_max, const vector<int>& nao, int nsm, vector<int>& kind) {
     const bool two_stage_asked = band_max != DEFAULT_BAND_MAX_NAO;
     int optin = 0, clusters = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     CK(cudaDeviceGetAttribute(&clusters, cudaDevAttrClusterLaunch, device));
-    if (optin < axg::TRD_SMEM_MAX || !clusters) return;
+    if (optin < axg::TRD_SMEM_MAX || !clusters || std::getenv("AXTB_EIGEN_TEAM")) return;
     for (int m = 0; m < nmol; m++) {
         int n = nao[m];
         if (n < TRD_MIN_NAO) continue;

@@ -51,3 +51,12 @@ def test_grid(engine, size, threshold, count):
         _check(b, i, r)
     alone = engine.Batch(mols[-1:], accuracy=1.0, grid_min_nao=threshold).run(gradient=True)[0]
     assert alone.energy == rs[-1].energy and np.array_equal(alone.gradient, rs[-1].gradient)
+
+
+def test_small_molecules_on_teams(engine):
+    """14 to 42 AOs with the threshold lowered to 12: teams of more CTAs than a molecule has columns."""
+    mols = [ammonia(k, k) for k in (2, 2, 3, 3, 4, 5, 6, 6, 6, 2)]
+    b = engine.Batch(mols, accuracy=1.0, grid_min_nao=12)
+    for i, r in enumerate(b.run(gradient=True, levels=True)):
+        assert r.status == 0
+        _check(b, i, r)
