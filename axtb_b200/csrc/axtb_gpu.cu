@@ -70,8 +70,8 @@ struct Fail : std::runtime_error {
 
 // Page-locked blocks of closed batches, kept for the next ones of the process: cudaMallocHost and
 // cudaFreeHost take 1 to 4 ms a call here, as much as the whole run of a small batch, and drivers such
-// as the numerical Hessian open and close two batches a call (3 waters: 16.3 ms without
-// the pool, 11.5 to 12.2 ms with it).
+// as the numerical Hessian open and close two batches a call (3 waters, medians of 80 calls in three turns of
+// each: 16.6, 18.6 and 21.4 ms without the pool, 11.2, 11.7 and 13.1 with it).
 // At most 8 blocks of at most 1 MiB each stay; larger ones go back at once, all of them when an
 // allocation fails. Blocks are portable (usable on every device) and come back only when the owner's
 // stream is idle, so that no copy still uses them.
@@ -1949,8 +1949,9 @@ void AxtbBatch::run(bool want_grad, bool warm, bool want_levels) {
     }
     // integrals
     // a thread per shell pair while the atom pairs are at most 256 a multiprocessor (there the two are
-    // even: 0.33 ms for 300 molecules of 1 to 20 atoms); with more the GPU is full either way and the
-    // short threads cost more (1024 molecules: 20.6 ms with a thread per atom pair, 22.8 without)
+    // even: 0.32 ms by shell pairs and 0.33 by atom pairs for 300 molecules of 3 to 32 atoms); with more the
+    // GPU is full either way and the short threads cost more (1024 molecules of 15 to 300 atoms: 20.6 ms with a
+    // thread per atom pair, 22.7 without)
     const bool by_shells = npdT <= 128LL * grid;
     LAUNCH("integrals", 0, mat_bytes(all, 11.0), {
         if (by_shells)

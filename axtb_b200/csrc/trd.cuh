@@ -72,7 +72,8 @@ __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned phase) {
     return false;
 }
 // The grid's pairs (row element, y entry) travel through global memory as single 128-bit words that
-// carry their own flag: the values are scaled by 2^-500 (exactly: |x| < 2^500), which leaves the
+// carry their own flag: the values are scaled by 2^-500 (|x| < 2^500; exact from 2^-522 up, and what is
+// below loses bits that no sum with the matrix's other elements holds), which leaves the
 // top exponent bit of the row element zero and free for the phase of the buffer's use. A reader
 // checks the very words it needs, so no fence has to order them: a count of the CTAs that have
 // published tells one thread per CTA when to look (all threads polling their words from the start
