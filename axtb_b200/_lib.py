@@ -74,6 +74,7 @@ SIGNATURES = {
     "axtb_gpu_batch_profile": (C.c_int, [C.c_void_p, C.c_char_p, C.c_size_t]),
     "axtb_gpu_apply_plan": (C.c_int, [PI32, C.c_int32, C.c_int32, PI32, PI32]),
     "axtb_gpu_eigen_order": (C.c_int, [C.c_int32] * 4 + [PI32, PI32]),
+    "axtb_gpu_cholesky_plan": (C.c_int, [PI32, C.c_int32, C.c_int32, PI32, C.c_int32]),
     "axtb_gpu_get_moments": (C.c_int, [C.c_void_p, PD, PD, PD]),
     "axtb_gpu_set_moments": (C.c_int, [C.c_void_p, PD, PD, PD, C.c_int32]),
     "axtb_gpu_batch_get_moments": (C.c_int, [C.c_void_p, C.c_int32, PD, PD, PD]),

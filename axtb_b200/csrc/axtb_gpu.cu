@@ -410,6 +410,54 @@ static vector<ApplyLaunch> apply_launches(const vector<int>& nao, const vector<i
     return v;
 }
 
+// ------------------------------------------------------------------ plan of the Cholesky steps
+// The launches of the factorisation (stages_chol.cuh) over matrices of these sizes, the largest first:
+// kernel 0 k_ch_init, then per step p of 64 columns 1 k_ch_panel and 2 k_ch_trail, for the EEQ matrices
+// 3 to 5 the parts of k_ch_eeq. A launch is a rectangle, x CTAs for each of its molecules, of which the
+// smaller ones need fewer; where the empty ones add up to more than CH_EMPTY (20 us at 1.25 ns each, several
+// launches' worth) the molecules from there on get a launch of their own. 20000 molecules of 12 to 24 AOs with one
+// of 2400 among them: 313 ms in one rectangle over everything, 6 in launches by size.
+constexpr long long CH_EMPTY = 16384;
+struct ChLaunch {
+    int kernel, p, x, first, count;
+};
+static int cholesky_ctas(int kernel, int p, int n) {
+    const int rt = (n + axg::CB - 1) / axg::CB, left = rt - 1 - p;
+    switch (kernel) {
+        case 0: return rt * rt;
+        case 1: return rt > 1 && p < rt ? rt - 1 : 0;
+        case 2: return left > 0 ? left * (left + 1) / 2 : 0;
+        case 3: return (n + 31) / 32;
+        case 4: return (n + 7) / 8;
+        default: return 1;
+    }
+}
+static vector<ChLaunch> cholesky_plan(const vector<int>& sizes, bool eeq) {
+    vector<ChLaunch> v;
+    const int count = (int)sizes.size();
+    auto add = [&](int kernel, int p) {
+        for (int i = 0, j; i < count; i = j) {
+            const int x = cholesky_ctas(kernel, p, sizes[i]);
+            if (x == 0) break;  // and for all smaller ones
+            long long empty = 0;
+            for (j = i; j < count && j - i < 65535; j++) {  // molecules along the grid's y
+                const int t = cholesky_ctas(kernel, p, sizes[j]);
+                empty += x - t;
+                if (t == 0 || empty > CH_EMPTY) break;
+            }
+            v.push_back({kernel, p, x, i, j - i});
+        }
+    };
+    add(0, 0);
+    const int rt = count > 0 ? (sizes[0] + axg::CB - 1) / axg::CB : 0;
+    for (int p = 0; p < rt; p++) {
+        add(1, p);
+        add(2, p);
+    }
+    for (int k = 3; eeq && k < 6; k++) add(k, 0);
+    return v;
+}
+
 // ------------------------------------------------------------------ order of the eigen phase
 // Its launches in order, each on the batch's stream or on the side stream that forks off where the first
 // side step stands and joins at the end. Whatever needs all of its CTAs resident at once (k_team_grid, and
@@ -475,7 +523,9 @@ struct AxtbBatch {
     axg::StagePlan Q{};      // the molecules whose eigen phase runs in stages (those of trd and trd_grid)
     long long q_full = 0, q_low = 0, q_rt = 0, q_vec = 0, q_col = 0, q_full32 = 0, q_low32 = 0;  // its tasks
     vector<ApplyLaunch> q_apply;  // the back-transformation's launches
-    int q_nmax = 0, q_natmax = 0;
+    int q_nmax = 0;
+    vector<ChLaunch> q_chol[2];  // the Cholesky steps of the overlap and the EEQ matrices
+    const int* q_chol_mol[2] = {nullptr, nullptr};  // ... and their molecules, the largest matrix first
     int nteam_eigen = 0;     // the other molecules (team kernels)
     vector<TrdLaunch> trd;
     vector<TrdGrid> trd_grid;
@@ -638,24 +688,22 @@ static int stage_density(const axg::Batch& B, const axg::State& S, const axg::St
     using namespace axg;
     return stage_tiles<ST_C, false, PROF>(B, S, Q, c, st) + stage_tiles<ST_P, true, PROF>(B, S, Q, c, st);
 }
-// factor and inverse factor of the overlap matrices, or of the EEQ matrices; nmax: the largest
-static int stage_cholesky(const axg::Batch& B, const axg::State& S, const axg::StagePlan& Q, const axg::TeamPlan& P, int nmax,
-                           int eeq, cudaStream_t st) {
+// factor and inverse factor of the overlap matrices, or the EEQ charges from those of the EEQ matrices;
+// mol: the molecules in the plan's order
+static int stage_cholesky(const axg::Batch& B, const axg::State& S, axg::StagePlan Q, const axg::TeamPlan& P,
+                          const vector<ChLaunch>& plan, const int* mol, int eeq, cudaStream_t st) {
     using namespace axg;
-    const int W = SMEM_WORK_BYTES, T = TEAM_THREADS, rt = (nmax + CB - 1) / CB;
-    const unsigned cnt = (unsigned)Q.count;
-    int launched = 1;
-    k_ch_init<<<dim3(rt * rt, cnt), T, W, st>>>(B, S, Q, P, eeq);
-    for (int p = 0; p < rt && rt > 1; p++) {
-        k_ch_panel<<<dim3(rt - 1, cnt), T, W, st>>>(B, S, Q, P, p, eeq);
-        launched++;
-        const int left = rt - 1 - p;
-        if (left > 0) {
-            k_ch_trail<<<dim3(left * (left + 1) / 2, cnt), T, W, st>>>(B, S, Q, P, p, eeq);
-            launched++;
-        }
+    const int W = SMEM_WORK_BYTES, T = TEAM_THREADS;
+    for (const ChLaunch& l : plan) {
+        const dim3 g((unsigned)l.x, (unsigned)l.count);
+        Q.mol = mol + l.first;
+        Q.count = l.count;
+        if (l.kernel == 0) k_ch_init<<<g, T, W, st>>>(B, S, Q, P, eeq);
+        else if (l.kernel == 1) k_ch_panel<<<g, T, W, st>>>(B, S, Q, P, l.p, eeq);
+        else if (l.kernel == 2) k_ch_trail<<<g, T, W, st>>>(B, S, Q, P, l.p, eeq);
+        else k_ch_eeq<<<g, T, 0, st>>>(B, S, Q, P, l.kernel - 3);
     }
-    return launched;
+    return (int)plan.size();
 }
 
 // Which molecules' eigen phase runs in stages with the reduction on chip (stages.cuh, trd.cuh): from
@@ -852,21 +900,7 @@ void AxtbBatch::launch_stages() {
 // Factor and inverse factor of the staged molecules' overlap matrices, or the EEQ charges from those
 // of their EEQ matrices
 void AxtbBatch::launch_cholesky(int eeq) {
-    using namespace axg;
-    const int T = TEAM_THREADS;
-    for (int c0 = 0; c0 < Q.count; c0 += 65535) {  // molecules along the grid's y
-        StagePlan q = Q;
-        q.mol = Q.mol + c0;
-        const unsigned cnt = (unsigned)std::min(65535, Q.count - c0);
-        q.count = (int)cnt;
-        launches += stage_cholesky(B, S, q, P, eeq ? q_natmax : q_nmax, eeq, st);
-        if (eeq) {
-            k_ch_eeq<<<dim3((q_natmax + 31) / 32, cnt), T, 0, st>>>(B, S, q, P, 0);
-            k_ch_eeq<<<dim3((q_natmax + 7) / 8, cnt), T, 0, st>>>(B, S, q, P, 1);
-            k_ch_eeq<<<dim3(1, cnt), T, 0, st>>>(B, S, q, P, 2);
-            launches += 3;
-        }
-    }
+    launches += stage_cholesky(B, S, Q, P, q_chol[eeq], q_chol_mol[eeq], eeq, st);
     CK(cudaGetLastError());
 }
 
@@ -1186,8 +1220,7 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
     addI(tail_off.size());
     addI(tail_list.size() + 1);
     addI(nmol);                                              // trd_kind
-    addI(nmol);                                              // the stages' molecules, widths and tasks
-    addI(nmol);
+    for (int c = 0; c < 4; c++) addI(nmol);                  // the stages' molecules (three orders), widths and tasks
     for (int c = 0; c < 7; c++) addL((size_t)nmol + 1);
     for (int c = 0; c < 128; c++) addI(1);                   // k_trd lists: at most one per class and cluster size
     addI(nmol);
@@ -1449,7 +1482,6 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
             for (const ApplyLaunch& a : q_apply) takers += a.takes((int)n, w);
             if (takers != 1) throw Fail(AXTB_ERR_DEVICE, "no launch of the back-transformation for " + std::to_string(n) + " AOs");
             q_nmax = std::max(q_nmax, (int)n);
-            q_natmax = std::max(q_natmax, mols[m].nat);
             full.push_back(full.back() + rt * rt);
             low.push_back(low.back() + rt * (rt + 1) / 2);
             const long long r32 = (n + axg::G32 - 1) / axg::G32;
@@ -1466,6 +1498,14 @@ void AxtbBatch::build(const vector<HostMol>& in, const Opt& o) {
         q_rt = rts.back();
         q_vec = vec.back();
         q_col = col.back();
+        for (int eeq = 0; eeq < 2; eeq++) {
+            vector<int> by_size = list, size;
+            auto n_of = [&](int m) { return eeq ? mols[m].nat : m_nao[m]; };
+            std::stable_sort(by_size.begin(), by_size.end(), [&](int a, int b) { return n_of(a) > n_of(b); });
+            for (int m : by_size) size.push_back(n_of(m));
+            q_chol[eeq] = cholesky_plan(size, eeq != 0);
+            q_chol_mol[eeq] = upI(by_size);
+        }
         Q.mol = upI(list);
         Q.width = upI(width);
         Q.off_full = upL(full);
@@ -2314,7 +2354,7 @@ extern "C" int axtb_gpu_density_static(const double* d_fock, const double* d_ove
         while (G < 8 && 16 * G <= nao) G *= 2;
         const TrdClass* cls = trd_class(nao, G);
         try {
-            stage_cholesky(B, S, Q, P, nao, 0, on);
+            stage_cholesky(B, S, Q, P, cholesky_plan({nao}, false), Q.mol, 0, on);
             stage_transform<false>(B, S, Q, c, on);
             stage_reduce(cls->fn, G, 1, (int)(trd_smem_doubles(nao, G, 1, cls->cr, false) * 8), B, S, Q.mol, nullptr, on);
             k_st_tfac<false><<<(unsigned)c.rt, TEAM_THREADS, SMEM_WORK_BYTES, on>>>(B, S, Q, P);

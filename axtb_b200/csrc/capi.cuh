@@ -498,6 +498,16 @@ int axtb_gpu_eigen_order(int32_t grid_mols, int32_t team, int32_t chase, int32_t
     return AXTB_OK;
 }
 
+int axtb_gpu_cholesky_plan(const int32_t* sizes, int32_t count, int32_t eeq, int32_t* out, int32_t capacity) {
+    if (!sizes || count < 0 || (capacity > 0 && !out)) return AXTB_ERR_INPUT;
+    const vector<ChLaunch> v = cholesky_plan(vector<int>(sizes, sizes + count), eeq != 0);
+    for (size_t i = 0; i < v.size() && i < (size_t)std::max(capacity, 0); i++) {
+        const int row[5] = {v[i].kernel, v[i].p, v[i].x, v[i].first, v[i].count};
+        std::copy(row, row + 5, out + 5 * i);
+    }
+    return (int)v.size();
+}
+
 int axtb_gpu_batch_set_profiling(AxtbBatch* b, int32_t enable) {
     if (!b) return AXTB_ERR_INPUT;
     b->profiling = enable != 0;

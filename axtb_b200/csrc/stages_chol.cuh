@@ -1,5 +1,6 @@
 // Cholesky factor and triangular inverse of the staged molecules' overlap matrices (and EEQ matrices),
-// the same blocks of 64 as team_cholesky and team_trinv, one launch per step over all molecules:
+// the same blocks of 64 as team_cholesky and team_trinv, a launch per step over molecules of like size
+// (cholesky_plan):
 //   k_ch_init    the matrix into place; the first diagonal block factored and inverted
 //   k_ch_panel   step p: L[i, p] = A[i, p] L[p, p]^-T below, and row block p of the inverse,
 //                X[p, j] = -L[p, p]^-1 (L[p, j:p] X[j:p, j]), a 64 x 64 tile per CTA

@@ -56,6 +56,11 @@ int axtb_gpu_apply_plan(const int32_t* nao, int32_t count, int32_t nsm, int32_t*
  * beside the batch's). No device needed. */
 int axtb_gpu_eigen_order(int32_t grid_mols, int32_t team, int32_t chase, int32_t staged, int32_t* kernel, int32_t* side);
 
+/* The launches of the factorisation over matrices of these sizes, the largest first: five numbers each
+ * (0 set-up, 1 panel, 2 trailing update, 3 to 5 the EEQ parts; step; CTAs per molecule; first molecule;
+ * molecules). Returns how many there are, writes at most `capacity`. No device needed. */
+int axtb_gpu_cholesky_plan(const int32_t* sizes, int32_t count, int32_t eeq, int32_t* out, int32_t capacity);
+
 #ifdef __cplusplus
 }
 #endif

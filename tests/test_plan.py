@@ -2,6 +2,7 @@
 import ctypes as C
 
 import numpy as np
+import pytest
 
 
 def _apply_plan(nao, nsm=148):
@@ -59,3 +60,45 @@ def test_autotune_times_distinct_schedules():
     assert band_candidates(0) == band_candidates(32) == [64]  # no molecule of 34 AOs or more below 32
     assert band_candidates(64) == [64, 65]
     assert band_candidates(160) == [64, 160]
+
+
+def _cholesky_plan(sizes, eeq):
+    from axtb_b200 import _lib
+
+    a = np.ascontiguousarray(sizes, dtype=np.int32)
+    out = np.zeros((4096, 5), dtype=np.int32)
+    ptr = lambda x: x.ctypes.data_as(C.POINTER(C.c_int32))
+    n = _lib.load().axtb_gpu_cholesky_plan(ptr(a), len(a), eeq, ptr(out), len(out))
+    assert 0 <= n <= len(out)
+    return out[:n]
+
+
+def _tiles(kernel, p, n):
+    rt = (n + 63) // 64
+    left = np.maximum(rt - 1 - p, 0)
+    return [rt * rt, np.where((rt > 1) & (p < rt), rt - 1, 0), left * (left + 1) // 2, (n + 31) // 32, (n + 7) // 8,
+            np.ones_like(n)][kernel]
+
+
+@pytest.mark.parametrize("eeq", [0, 1])
+@pytest.mark.parametrize("case", ["one", "small", "edges", "mixed", "small and one large", "many", "none"])
+def test_cholesky_steps_cover_every_tile_with_few_empty_ctas(engine, case, eeq):
+    rng = np.random.default_rng(1)
+    sizes = {"one": [1202], "small": [12] * 300, "edges": [129, 128, 127, 65, 64, 63, 1], "mixed": rng.integers(12, 603, 1024),
+             "small and one large": [2400] + [18] * 20000, "many": rng.integers(12, 130, 140000), "none": []}[case]
+    n = np.sort(np.asarray(sizes, dtype=np.int64))[::-1]
+    plan = _cholesky_plan(n, eeq)
+    steps = int((n.max() + 63) // 64) if len(n) else 0
+    order = [(0, 0)] + [(k, p) for p in range(steps) for k in (1, 2)] + [(k, 0) for k in (3, 4, 5)] * eeq
+    at = 0
+    for kernel, p in order:  # in this order, each molecule with tiles in exactly one launch that has them all
+        need, got = _tiles(kernel, p, n), np.zeros(len(n), dtype=int)
+        while at < len(plan) and tuple(plan[at][:2]) == (kernel, p):
+            x, first, count = plan[at][2:]
+            assert count <= 65535 and (need[first:first + count] <= x).all()
+            assert (x - need[first:first + count]).sum() <= 16384
+            got[first:first + count] += 1
+            at += 1
+        assert ((got == 1) == (need > 0)).all()
+    assert at == len(plan)
+    assert len(plan) <= 3 * len(order) + 16  # no launch for each size
